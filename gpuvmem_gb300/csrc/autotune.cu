@@ -93,7 +93,7 @@ gv_status autotune(Problem& P, gv_tune_report* rep) {
   GV_TRY(chi2());  // residuals of the tuned launch
   // ---- tensor-core DChi2 --------------------------------------------------
   rep->tc_pair = -1;
-  if (P.engine == 2) {
+  if (P.engine == 2 && !P.nu) {
     auto dchi2 = [&]() {
       GV_CUDA(cudaMemsetAsync(xi, 0, sizeof(float) * 2 * MN, P.stream));
       return dchi2_launch(P, img, 0, xi);

@@ -843,8 +843,14 @@ gv_status launch_tc(const Problem& P, const TcParams& p, int nitems) {
 
 }  // namespace tc
 
+// sides and w-term the GEMM covers (the w-term has to be separable:
+// |w * rho| below 1e-7 cycles)
+bool dchi2_tc_geometry(const Problem& P) {
+  return P.N >= 128 && P.N == P.M && P.max_wrho < 1e-7;
+}
+
 bool dchi2_tc_supported(const Problem& P) {
-  return P.N >= 128 && P.N == P.M && P.max_wrho < 1e-7 && P.tc_partial != nullptr;
+  return dchi2_tc_geometry(P) && P.tc_partial != nullptr;
 }
 
 int tc_tile_n(const Problem& P) { return P.N >= 256 ? 256 : 128; }

@@ -104,8 +104,7 @@ gv_status error_images(Problem& P, float* d_img, float* d_err) {
       s = cuda_fail(ce, "error_images");
       break;
     }
-    s = P.engine == 2 ? dchi2_tc(P, nullptr, 0, P.d_tmp, c, 4)
-                      : dchi2_direct(P, nullptr, 0, P.d_tmp, c, 4);
+    s = dchi2_run(P, nullptr, 0, P.d_tmp, c, 4);
     if (s != GV_OK) break;
     e.freq = P.chans[c].freq;
     dim3 blk(32, 8), grd((P.M + 31) / 32, (P.N + 7) / 8);

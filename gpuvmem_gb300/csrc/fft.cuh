@@ -1,0 +1,140 @@
+// Inverse FFT of lines held in shared memory, for the image passes of the
+// objective (objective.cu) and of the gradient (dchi2_nu.cu): radix-8
+// Stockham passes with the butterflies in registers.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace gv {
+
+// The arithmetic that more than one kernel performs on the same values (the
+// FFT butterflies and twiddles, the phase rotation, the degridding's model
+// and chi2 terms, the prior stencils) spells out every multiply-add with
+// rounding intrinsics: the compiler never contracts those, so the separate
+// kernels and the fused ones round each operation alike wherever the code
+// is inlined (the compiler's choice of which product to fuse into an FMA
+// can otherwise differ between inlining contexts).
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)),
+                     __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+
+// R-point inverse DFT (exp(+2 pi i r s / R), R = 2^LR <= 8) of v in
+// registers, radix-2 decimation in frequency: the result is in bit-reversed
+// order (X[r] = v[brev(r)]).  The twiddles are 1, i and (+-1 + i)/sqrt(2):
+// multiplications by 1 and i are exact.
+__device__ __forceinline__ float2 rot_turn(float2 d, int s, int m) {
+  // d * e^{2 pi i s / m}, m in {2, 4, 8}, s < m / 2 (compile-time after
+  // unrolling)
+  const float c = 0.70710678118654752440f;
+  if (s == 0) return d;
+  if (m == 4 || s == 2) return make_float2(-d.y, d.x);                 // * i
+  if (s == 1) return make_float2(__fmul_rn(c, d.x - d.y), __fmul_rn(c, d.x + d.y));  // * (1 + i)/sqrt 2
+  return make_float2(__fmul_rn(c, -d.x - d.y), __fmul_rn(c, d.x - d.y));           // * (-1 + i)/sqrt 2
+}
+
+template <int LR>
+__device__ __forceinline__ void dft_inv(float2 (&v)[1 << LR]) {
+  constexpr int R = 1 << LR;
+#pragma unroll
+  for (int half = R / 2; half >= 1; half >>= 1) {
+#pragma unroll
+    for (int g = 0; g < R; g += 2 * half) {
+#pragma unroll
+      for (int s = 0; s < half; s++) {
+        const float2 a = v[g + s], b = v[g + s + half];
+        v[g + s] = make_float2(a.x + b.x, a.y + b.y);
+        v[g + s + half] = rot_turn(make_float2(a.x - b.x, a.y - b.y), s, 2 * half);
+      }
+    }
+  }
+}
+
+template <int LR>
+__device__ __forceinline__ constexpr int brev_c(int r) {
+  int o = 0;
+  for (int b = 0; b < LR; b++) o |= ((r >> b) & 1) << (LR - 1 - b);
+  return o;
+}
+
+// Shared-memory position of element e of an FFT line: one float2 of padding
+// after every eight, so the first Stockham pass's writes (eight elements
+// apart across the lanes) and the second's (runs of eight, 64 apart) fall in
+// distinct banks.  A line of n elements takes fft_span(n) positions; the
+// lines of a multi-column buffer are fft_stride(n) apart (four more, so four
+// columns read row by row do not share banks either).
+__device__ __forceinline__ int fpad(int e) { return e + (e >> 3); }
+__host__ __device__ __forceinline__ int fft_span(int n) { return n + (n >> 3); }
+__host__ __device__ __forceinline__ int fft_stride(int n) { return fft_span(n) + 4; }
+
+// One Stockham autosort pass of radix R = 2^LR over `ncol` columns of length
+// n = 2^log2n in shared memory (element e of column c at
+// buf[c * fft_stride(n) + fpad(e)], natural order).
+// Work item (c, j), j < n / R, reads x[j + r n/R] (r < R), multiplies by the
+// twiddles e^{2 pi i r k / (Ns R)} with k = j mod Ns (table tw[m] =
+// e^{2 pi i m / n}, read through L1), takes the R-point inverse DFT and
+// writes y[(j / Ns) Ns R + k + r Ns] (Govindaraju et al., "High Performance
+// Discrete Fourier Transforms on Graphics Processors", SC 2008).  In place:
+// all items are read before a block barrier and written after it, so each
+// thread holds its items' values in registers: max(VPT, R) of them, VPT the
+// values per thread (ncol * n <= VPT * blockDim.x).
+template <int LR, int VPT>
+__device__ __forceinline__ void stockham_pass(float2* buf, int log2n, int ncol, int lNs,
+                                              const float2* __restrict__ tw) {
+  constexpr int R = 1 << LR;
+  constexpr int kMaxItems = VPT / R > 1 ? VPT / R : 1;
+  const int lq = log2n - LR;  // log2 of the items per column
+  const int items = ncol << lq;
+  float2 v[kMaxItems][R];
+#pragma unroll
+  for (int t = 0; t < kMaxItems; t++) {
+    const int it = threadIdx.x + t * blockDim.x;
+    if (it < items) {
+      const int c = it >> lq, j = it & ((1 << lq) - 1);
+      const float2* x = buf + c * fft_stride(1 << log2n);
+#pragma unroll
+      for (int r = 0; r < R; r++) v[t][r] = x[fpad(j + (r << lq))];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kMaxItems; t++) {
+    const int it = threadIdx.x + t * blockDim.x;
+    if (it < items) {
+      const int c = it >> lq, j = it & ((1 << lq) - 1);
+      const int k = j & ((1 << lNs) - 1);
+      if (lNs > 0) {
+        const int step = k << (log2n - lNs - LR);  // r k n / (Ns R) = r * step
+#pragma unroll
+        for (int r = 1; r < R; r++) v[t][r] = cmul(v[t][r], __ldg(tw + r * step));
+      }
+      dft_inv<LR>(v[t]);
+      float2* y = buf + c * fft_stride(1 << log2n);
+      const int base = ((j >> lNs) << (lNs + LR)) + k;
+#pragma unroll
+      for (int r = 0; r < R; r++) y[fpad(base + (r << lNs))] = v[t][brev_c<LR>(r)];
+    }
+  }
+  __syncthreads();
+}
+
+// In-place inverse FFT (cuFFT's CUFFT_INVERSE convention: exp(+i),
+// unnormalised) of `ncol` independent columns of length n = 2^log2n held in
+// shared memory (element e of column c at buf[c * fft_stride(n) + fpad(e)]),
+// natural order in and out: radix-8
+// Stockham passes, then one of radix 4 or 2.  The caller has synchronised
+// the block after filling buf; needs ncol * n <= VPT * blockDim.x and
+// n <= 2 * blockDim.x * max(1, VPT / 2).
+template <int VPT>
+__device__ void smem_fft(float2* buf, int log2n, int ncol, const float2* __restrict__ tw) {
+  int lNs = 0;
+  while (log2n - lNs >= 3) {
+    stockham_pass<3, VPT>(buf, log2n, ncol, lNs, tw);
+    lNs += 3;
+  }
+  if (log2n - lNs == 2) stockham_pass<2, VPT>(buf, log2n, ncol, lNs, tw);
+  else if (log2n - lNs == 1) stockham_pass<1, VPT>(buf, log2n, ncol, lNs, tw);
+}
+
+}  // namespace gv

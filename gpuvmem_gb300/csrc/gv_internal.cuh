@@ -153,6 +153,7 @@ struct Problem {
                                  // (GV_FUSED=1 at creation turns it on)
   int fused_off = 0;             // > 0 while callers that run problems concurrently launch
   int fused_blocks[3] = {0, 0, 0};  // cooperative blocks of k_objective_fused (per image kind)
+  struct NuPlan* nu = nullptr;   // non-uniform FFT of DChi2 (dchi2_nu.cu), or null: direct sums
   void* graphs = nullptr;        // graph cache (graph.cu)
   void* ls_graphs = nullptr;     // device line-search graphs (optim.cu)
   struct LsState* d_ls = nullptr;  // device line-search state
@@ -397,6 +398,17 @@ gv_status dchi2_direct(Problem& P, const float* d_img, int flag_opt, float* d_re
                        int only_channel, int mode);
 gv_status dchi2_tc(Problem& P, const float* d_img, int flag_opt, float* d_result,
                    int only_channel, int mode);
+// non-uniform FFT (dchi2_nu.cu), where P.nu is set
+gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result,
+                   int only_channel, int mode);
+gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw);
+gv_status nu_finish(Problem& P);
+void nu_free(Problem& P);
+uint32_t nu_tiles_x(int N);  // tiles per row of the doubled grid's half plane
+// the engine P runs DChi2 with
+gv_status dchi2_run(Problem& P, const float* d_img, int flag_opt, float* d_result,
+                    int only_channel, int mode);
+bool dchi2_tc_geometry(const Problem& P);
 bool dchi2_tc_supported(const Problem& P);
 int tc_tile_n(const Problem& P);
 bool tc_pair(const Problem& P);

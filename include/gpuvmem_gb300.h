@@ -122,7 +122,10 @@ typedef struct gv_problem_desc {
   const gv_channel_desc* channels;
   int32_t nterms;
   const gv_fi_desc* terms;
-  int32_t dchi2_engine;     /* 0 auto, 1 direct SIMT, 2 tensor-core GEMM */
+  /* 0 auto: DChi2 as a non-uniform FFT where it covers the w-term (nearer
+   * the 64-bit sum than the direct sums, and much faster), else the direct
+   * sum; 1 direct SIMT sum, 2 direct sum as a tensor-core GEMM */
+  int32_t dchi2_engine;
   /* gridding correction function (host, M*N floats) of gridded data, or
    * NULL: with it chi2() multiplies the beam-weighted image by it before the
    * FFT (apply_GCF, src/functions.cu:2468) and DChi2 takes the GCF variant
@@ -142,7 +145,9 @@ typedef struct gv_problem_info {
   int64_t nvis_total;
   int64_t nvis_in_grid;  /* visibilities whose weight vis_mod keeps */
   int64_t mask_pixels;   /* pixels with noise < noise_cut */
-  int32_t dchi2_engine;  /* engine actually used */
+  int32_t dchi2_engine;  /* direct-sum engine of the problem (1 SIMT, 2 GEMM);
+                            created with 0, it runs where the non-uniform
+                            FFT does not */
   int32_t nterms;        /* terms kept (lambda != 0) */
 } gv_problem_info;
 
