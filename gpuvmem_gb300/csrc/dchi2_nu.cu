@@ -10,10 +10,9 @@
 //                  Klinteberg, "A parallel non-uniform fast Fourier transform
 //                  library based on an exponential of semicircle kernel",
 //                  SIAM J. Sci. Comput. 41, 2019);
-//  2. k_nu_merge   the tiles' sums are added into the rows and columns of the
-//                  grid that the data cover;
-//  3. k_nu_rows    row FFTs of the covered rows, the image's N of 2N outputs;
-//  4. k_nu_cols    column FFTs, the kernel's correction, the w-term, beam,
+//  2. k_nu_rows    the tiles' sums added up along the rows of the grid that
+//                  the data cover, and their FFTs, the image's N of 2N outputs;
+//  3. k_nu_cols    column FFTs, the kernel's correction, the w-term, beam,
 //                  mask and chain rule, summed over the channels.
 //
 // The w-term is a Chebyshev series (the Jacobi-Anger expansion): with
@@ -39,31 +38,33 @@
 
 namespace gv {
 
-// Work of one warp of k_nu_spread: `count` consecutive visibilities, all
+// Work of one block of k_nu_spread: `count` consecutive visibilities, all
 // with their first cell in one 8 x 8 tile of the doubled grid.
 struct NuTask {
   uint32_t begin;
   int count;
+  int first, pieces;  // first task of the tile, tasks of the tile
 };
 
 struct NuPlan {
   int pairs = 0;           // complex FFTs per channel
+  int warps = 4;           // of a block of k_nu_spread
   float wmax = 0.0f;
-  int cmin = 0, ncol = 0;  // covered columns (signed), ncol even
+  int cmin = 0, ncol = 0;  // covered columns (signed)
   int rmin = 0, nrow = 0;  // covered rows (signed)
   int wrap = 0;            // cells beyond +-N: the grid's period matters
   int tx0 = 0, ntx = 0, ty0 = 0, nty = 0;  // tiles in use
   std::vector<int> task_off;   // [C + 1]
   std::vector<int> groups;     // channel group boundaries
   NuTask* d_tasks = nullptr;
-  int* d_slot_off = nullptr;   // [C nty ntx + 1] tasks of each tile
+  int* d_slot = nullptr;       // [C nty ntx] first task of each tile, or -1
+  uint32_t* d_done = nullptr;  // [tasks] tasks of a tile done (at its first task)
   float2* d_slots = nullptr;   // per task: [pair][plane][225] sums
-  float2* d_F = nullptr;       // [channel of the group][pair][nrow][ncol]
   float2* d_H = nullptr;       // [channel of the group][pair][nrow][N]
-  float2* d_turn = nullptr;    // [N] e^{2 pi i (j - N/2) / 2N}
+  float2* d_twiddle = nullptr; // fft16_twiddles(log2 2N)
   float* d_corr = nullptr;     // [N] 1 / kernel transform
   float2* d_coef = nullptr;    // [pair][MN] w-term coefficients (k_nu_coefficients)
-  float* d_fac = nullptr;      // [channel of the group][MN] k_nu_factors
+  float* d_fac = nullptr;      // [C][MN] image-independent factors (k_nu_factors)
   float coef[4][12];           // the taps' polynomials (tap_polynomials)
 };
 
@@ -72,7 +73,7 @@ namespace {
 constexpr int kTaps = 8;
 constexpr int kTileSide = 15;  // 8 first cells + 7
 constexpr int kTilePts = kTileSide * kTileSide;
-constexpr int kSpreadWarps = 4;
+constexpr int kMinShare = 16;  // visibilities a warp takes at least
 constexpr int kMaxPairs = 4;
 constexpr double kBeta = 2.30 * kTaps;
 constexpr int kPolyHalf = 6;  // even and odd coefficients of a tap's polynomial
@@ -86,9 +87,10 @@ struct SpreadArgs {
   const float2* __restrict__ cvr;
   const float4* __restrict__ deg;
   const float2* __restrict__ vo;
-  const NuTask* __restrict__ tasks;
-  int ntasks;
-  float2* __restrict__ slots;
+  const NuTask* __restrict__ tasks;  // of the group
+  int ntasks, t0;                    // t0: the group's first task
+  uint32_t* __restrict__ done;
+  float2* slots;
   int mode;        // of the DChi2 engines: 0/1 residuals, 2 Vo, 3 weights, 4 conjugated residuals
   int sh;          // fraction bits of a fixed-point position on the doubled grid
   float frac;      // 2^-sh
@@ -133,38 +135,42 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
   }
 }
 
-// One warp per task.  Each lane prepares one of 32 visibilities at a time
-// (position, taps, the pairs' values) in shared memory; then the warp takes
-// them one by one, lane l summing taps (l & 7, l >> 3) and (l & 7, 4 + l >> 3)
-// of every plane in registers as long as the first cell stays the same (the
-// visibilities are sorted by cell), and adds them to the task's 15 x 15 tile
-// in shared memory when it changes.  The tile goes out once, to the task's
-// own slot, so no two warps write the same place.
-template <int NP>
+// One block per task, its visibilities shared out among the warps in order.
+// Each lane prepares one of 32 visibilities at a time (position, taps, the
+// pairs' values) in shared memory; then the warp takes them one by one.  Lane
+// l owns the cells whose column is l mod 8 and whose row is l / 8 or l / 8 + 4
+// mod 8: of any 8 x 8 footprint exactly two, whose sums it keeps in registers
+// while the footprint moves along a row of cells (the visibilities are sorted
+// by cell), so a step to the next cell writes back only the column that is
+// left.  The warps' 15 x 15 tiles are added in order and go out once, to the
+// task's own slot; where a tile has several tasks, the last of their blocks
+// to finish adds the slots up, in order, into the first.
+template <int NP, int kSpreadWarps>
 __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   extern __shared__ float4 smem_f4[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kPerWarp = NP * kTilePts + NP * 32 + 32 * 5;  // float4
-  float4* tile = smem_f4 + warp * kPerWarp;
-  float4* val = tile + NP * kTilePts;           // [NP][32]
+  constexpr int kStage = NP * 32 + 32 * 5;  // float4 of a warp's staging
+  float4* tile = smem_f4 + warp * (NP * kTilePts);
+  float4* val = smem_f4 + kSpreadWarps * (NP * kTilePts) + warp * kStage;  // [NP][32]
   float* wts = reinterpret_cast<float*>(val + NP * 32);  // [32][20]: x taps, y taps, padding
-  const int id = blockIdx.x * kSpreadWarps + warp;
-  if (id >= a.ntasks) return;
-  const NuTask task = a.tasks[id];
-  for (int k = lane; k < NP * kTilePts; k += 32) tile[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const NuTask task = a.tasks[blockIdx.x];
+  // whole batches of 32, unless one would do for all the warps
+  const int even = (task.count + kSpreadWarps - 1) / kSpreadWarps;
+  const int share = kSpreadWarps == 1 ? task.count
+                    : task.count <= 32 ? max(kMinShare, even) : (even + 31) & ~31;
+  const int first = min(task.count, warp * share), last = min(task.count, first + share);
   const int tx = lane & 7, ty = lane >> 3;
   f32x2 acc[2][NP][2];
-  auto clear = [&]() {
 #pragma unroll
-    for (int h = 0; h < 2; h++)
+  for (int h = 0; h < 2; h++)
 #pragma unroll
-      for (int q = 0; q < NP; q++) acc[h][q][0] = acc[h][q][1] = 0ull;
-  };
-  auto flush = [&](int base) {
-    __syncwarp();
+    for (int q = 0; q < NP; q++) acc[h][q][0] = acc[h][q][1] = 0ull;
+  // this lane's place in the footprint at (bx, by): its x tap and two y taps
+  int bx = 0, by = 0, ox = tx, oy0 = ty, oy1 = ty + 4;
+  auto flush = [&]() {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int idx = base + (ty + 4 * h) * kTileSide + tx;
+      const int idx = (by + (h ? oy1 : oy0)) * kTileSide + bx + ox;
 #pragma unroll
       for (int q = 0; q < NP; q++) {
         float4 t = tile[q * kTilePts + idx];
@@ -174,15 +180,17 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
         t.z += m.x;
         t.w += m.y;
         tile[q * kTilePts + idx] = t;
+        acc[h][q][0] = acc[h][q][1] = 0ull;
       }
     }
   };
-  clear();
+  if (first < last)
+    for (int k = lane; k < NP * kTilePts; k += 32) tile[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   int cur = -1;
-  for (int k0 = 0; k0 < task.count; k0 += 32) {
-    const int cnt = min(32, task.count - k0);
+  for (int k0 = first; k0 < last; k0 += 32) {
+    const int cnt = min(32, last - k0);
     __syncwarp();  // the last 32 are done with the staging
-    int base = 0;
+    int base = -1;
     if (lane < cnt) {
       const uint32_t g = task.begin + k0 + lane;
       const uint4 p = __ldcs(a.ph + g);
@@ -213,7 +221,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
       }
       const uint32_t below = (1u << a.sh) - 1u;
       const int ix = (int)(fu >> a.sh), iy = (int)((int32_t)fv >> a.sh) + a.N;
-      base = (iy & 7) * kTileSide + (ix & 7);
+      base = ((iy & 7) << 3) | (ix & 7);
       float w[kTaps];
       float4* wl = reinterpret_cast<float4*>(wts + lane * 20);
       taps(a, (float)(fu & below) * a.frac, w);
@@ -235,17 +243,23 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
     if (lane == 0) prev = cur;
     const uint32_t heads = __ballot_sync(0xffffffffu, base != prev);
     __syncwarp();
-#pragma unroll 2
     for (int i = 0; i < cnt; i++) {
       if ((heads >> i) & 1u) {
-        if (cur >= 0) {
-          flush(cur);
-          clear();
-        }
-        cur = __shfl_sync(0xffffffffu, base, i);
+        const int next = __shfl_sync(0xffffffffu, base, i);
+        const int nx = next & 7, ny = next >> 3;
+        // every cell is one lane's, so the lanes that write back need not
+        // wait for one another; the barrier orders one step after the last
+        if (cur >= 0 && (ny != by || nx < bx || ox < nx - bx)) flush();
+        __syncwarp();
+        cur = next;
+        bx = nx;
+        by = ny;
+        ox = (tx - bx) & 7;
+        oy0 = (ty - by) & 7;
+        oy1 = oy0 ^ 4;
       }
-      const float kx = wts[i * 20 + tx];
-      const float w0 = kx * wts[i * 20 + 8 + ty], w1 = kx * wts[i * 20 + 12 + ty];
+      const float kx = wts[i * 20 + ox];
+      const float w0 = kx * wts[i * 20 + 8 + oy0], w1 = kx * wts[i * 20 + 8 + oy1];
       const f32x2 p0 = pack2(w0, w0), p1 = pack2(w1, w1);
 #pragma unroll
       for (int q = 0; q < NP; q++) {
@@ -258,156 +272,214 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
       }
     }
   }
-  if (cur >= 0) flush(cur);
-  __syncwarp();
-  float2* out = a.slots + (size_t)id * (NP * 2 * kTilePts);
-  for (int k = lane; k < kTilePts; k += 32) {
-#pragma unroll
-    for (int q = 0; q < NP; q++) {
-      const float4 t = tile[q * kTilePts + k];
-      out[(2 * q) * kTilePts + k] = make_float2(t.x, t.y);
-      out[(2 * q + 1) * kTilePts + k] = make_float2(t.z, t.w);
+  if (cur >= 0) flush();
+  __syncthreads();
+  const int nw = (task.count + share - 1) / share;
+  float2* out = a.slots + (size_t)blockIdx.x * (NP * 2 * kTilePts);
+  for (int k = threadIdx.x; k < NP * kTilePts; k += 32 * kSpreadWarps) {
+    float4 t = smem_f4[k];
+    for (int w = 1; w < nw; w++) {
+      const float4 u = smem_f4[w * (NP * kTilePts) + k];
+      t.x += u.x;
+      t.y += u.y;
+      t.z += u.z;
+      t.w += u.w;
     }
+    const int q = k / kTilePts, o = k - q * kTilePts;
+    out[(2 * q) * kTilePts + o] = make_float2(t.x, t.y);
+    out[(2 * q + 1) * kTilePts + o] = make_float2(t.z, t.w);
+  }
+  if (task.pieces == 1) return;
+  __shared__ int last_block;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last_block = atomicAdd(a.done + task.first, 1u) == (uint32_t)task.pieces - 1u;
+    if (last_block) a.done[task.first] = 0u;
+  }
+  __syncthreads();
+  if (!last_block) return;
+  __threadfence();
+  constexpr size_t kSlot = NP * 2 * kTilePts;
+  float2* sum = a.slots + (size_t)(task.first - a.t0) * kSlot;
+  for (int k = threadIdx.x; k < (int)kSlot; k += 32 * kSpreadWarps) {
+    float2 t = __ldcg(sum + k);
+#pragma unroll 8
+    for (int w = 1; w < task.pieces; w++) {
+      const float2 u = __ldcg(sum + w * kSlot + k);
+      t.x += u.x;
+      t.y += u.y;
+    }
+    sum[k] = t;
   }
 }
 
-struct MergeArgs {
+struct RowArgs {
   const float2* __restrict__ slots;
-  const int* __restrict__ slot_off;
-  float2* __restrict__ F;
+  const int* __restrict__ slot;
+  const float2* __restrict__ tw;
+  float2* __restrict__ H;
   int N, pairs, c0, t0;  // first channel and first task of the group
+  int lines;
   int cmin, ncol, rmin, nrow, wrap;
   int tx0, ntx, ty0, nty;
 };
 
-// Sum of a plane at (column c, row r) over the tiles whose footprint holds
-// it (two per axis at most) and their tasks, in order.
-__device__ __forceinline__ float2 plane_at(const MergeArgs& a, int ch, int plane, int c, int r) {
+// The tiles over a row of the grid (two at most) and the row's place in them.
+struct RowTiles {
+  const int* slot[2];
+  int at[2];  // first cell of the row in the tile's plane, or -1
+};
+
+__device__ __forceinline__ RowTiles row_tiles(const RowArgs& a, int ch, int r) {
+  RowTiles t;
+  const int rr = r + a.N + 3;
+#pragma unroll
+  for (int d = 0; d < 2; d++) {
+    const int ty = (rr >> 3) - d - a.ty0, ly = (rr & 7) + 8 * d;
+    const bool in = rr >= 0 && ly < kTileSide && (unsigned)ty < (unsigned)a.nty;
+    t.slot[d] = a.slot + ((size_t)ch * a.nty + (in ? ty : 0)) * a.ntx;
+    t.at[d] = in ? ly * kTileSide : -1;
+  }
+  return t;
+}
+
+// Sum of a plane at column c of a row over the tiles that hold it, in order.
+__device__ __forceinline__ float2 plane_at(const RowArgs& a, const RowTiles& t, int plane, int c) {
   float2 s = make_float2(0.0f, 0.0f);
-  const int cc = c + 3, rr = r + a.N + 3;
-  if (cc < 0 || rr < 0) return s;
+  const int cc = c + 3;
+  const float2* p[4];
 #pragma unroll
-  for (int dy = 0; dy < 2; dy++) {
-    const int ty = (rr >> 3) - dy - a.ty0, ly = (rr & 7) + 8 * dy;
-    if (ly >= kTileSide || (unsigned)ty >= (unsigned)a.nty) continue;
+  for (int k = 0; k < 4; k++) {
+    const int tx = (cc >> 3) - (k & 1) - a.tx0, lx = (cc & 7) + 8 * (k & 1);
+    int id = -1;
+    if (cc >= 0 && lx < kTileSide && t.at[k >> 1] >= 0 && (unsigned)tx < (unsigned)a.ntx)
+      id = __ldg(t.slot[k >> 1] + tx);
+    p[k] = id >= 0 ? a.slots + ((size_t)(id - a.t0) * a.pairs * 2 + plane) * kTilePts +
+                         t.at[k >> 1] + lx
+                   : nullptr;
+  }
 #pragma unroll
-    for (int dx = 0; dx < 2; dx++) {
-      const int tx = (cc >> 3) - dx - a.tx0, lx = (cc & 7) + 8 * dx;
-      if (lx >= kTileSide || (unsigned)tx >= (unsigned)a.ntx) continue;
-      const int* so = a.slot_off + ((size_t)ch * a.nty + ty) * a.ntx + tx;
-      const int s0 = __ldg(so) - a.t0, s1 = __ldg(so + 1) - a.t0;
-      const float2* p = a.slots + ((size_t)s0 * a.pairs * 2 + plane) * kTilePts +
-                        ly * kTileSide + lx;
-      for (int k = s0; k < s1; k++, p += (size_t)a.pairs * 2 * kTilePts) {
-        const float2 v = *p;
-        s.x += v.x;
-        s.y += v.y;
-      }
+  for (int k = 0; k < 4; k++) {
+    if (p[k]) {
+      const float2 v = __ldg(p[k]);
+      s.x += v.x;
+      s.y += v.y;
     }
   }
   return s;
 }
 
-// F = (h+ (c, r) + conj(h- (-c, -r))) / 2 with h+- the sums of the even plus /
-// minus the odd term: the Hermitian part of the even term's grid plus the
-// anti-Hermitian part of the odd one's.
-__global__ void __launch_bounds__(128) k_nu_merge(MergeArgs a) {
-  const int ci = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ci >= a.ncol) return;
-  const int c = a.cmin + ci, r = a.rmin + blockIdx.y;
-  const int ch = a.c0 + blockIdx.z / a.pairs, q = blockIdx.z % a.pairs;
-  float2 hp = make_float2(0.0f, 0.0f), hm = hp;
-  const int G = 2 * a.N;
-  const int w = a.wrap ? 1 : 0;
-  for (int wy = -w; wy <= w; wy++)
-    for (int wx = -w; wx <= w; wx++) {
-      const int cc = c + wx * G, rr = r + wy * G;
-      const float2 p = plane_at(a, ch, 2 * q, cc, rr);
-      const float2 m = plane_at(a, ch, 2 * q + 1, -cc, -rr);
-      hp.x += p.x;
-      hp.y += p.y;
-      hm.x += m.x;
-      hm.y += m.y;
+// The grid's value at (c, r): (h+ (c, r) + conj(h- (-c, -r))) / 2 with h+- the
+// sums of the even plus / minus the odd term, which is the Hermitian part of
+// the even term's grid plus the anti-Hermitian part of the odd one's.  The
+// sums lie in u >= 0, so away from u = 0 only one of the two is there.
+__device__ __forceinline__ float2 grid_at(const RowArgs& a, const RowTiles& up,
+                                          const RowTiles& down, int q, int c) {
+  float2 g = make_float2(0.0f, 0.0f);
+  if (c >= -3) {
+    const float2 p = plane_at(a, up, 2 * q, c);
+    g = make_float2(0.5f * p.x, 0.5f * p.y);
+  }
+  if (c <= 3) {
+    const float2 m = plane_at(a, down, 2 * q + 1, -c);
+    g.x = fmaf(0.5f, m.x, g.x);
+    g.y = fmaf(-0.5f, m.y, g.y);
+  }
+  return g;
+}
+
+// Rows of the doubled grid put together from the tiles and transformed over
+// its 2N cells, of which the N outputs about the
+// middle are kept: output x = j + r N / 8 of thread j is pixel x + N/2 for
+// r < 4 and x - 2N + N/2 for r >= 12, so pixel j + s N / 8 is r = s - 4 or
+// s + 12.  kLines rows per block.
+template <int LG>
+struct RowShape {
+  static constexpr int kThreads = (1 << LG) / 16;  // per line
+  static constexpr int kLines = kThreads >= 128 ? 1 : 128 / kThreads;
+};
+
+__device__ __forceinline__ constexpr int kept_output(int s) {
+  return brev_c<4>(s < 4 ? s + 12 : s - 4);
+}
+
+template <int LG>
+__global__ void __launch_bounds__(RowShape<LG>::kThreads * RowShape<LG>::kLines)
+    k_nu_rows(RowArgs a) {
+  constexpr int n = 1 << LG, N = n / 2, T = RowShape<LG>::kThreads, L = RowShape<LG>::kLines;
+  extern __shared__ float2 smem_f2[];
+  const int j = threadIdx.x % T, l = threadIdx.x / T;
+  const int line = blockIdx.x * L + l;
+  const bool in = line < a.lines;
+  const int plane = in ? line / a.nrow : 0, r = a.rmin + (in ? line - plane * a.nrow : 0);
+  const int ch = a.c0 + plane / a.pairs, q = plane % a.pairs;
+  float2 v[16];
+  if (!a.wrap) {
+    const RowTiles up = row_tiles(a, ch, r), down = row_tiles(a, ch, -r);
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      const int c = e < 8 ? j + e * T : j + e * T - n;
+      v[e] = in && (unsigned)(c - a.cmin) < (unsigned)a.ncol ? grid_at(a, up, down, q, c)
+                                                            : make_float2(0.0f, 0.0f);
     }
-  a.F[((size_t)blockIdx.z * a.nrow + blockIdx.y) * a.ncol + ci] =
-      make_float2(0.5f * (hp.x + hm.x), 0.5f * (hp.y - hm.y));
+  } else {
+    // footprints that reach over the grid's edge come back at the other side
+#pragma unroll
+    for (int e = 0; e < 16; e++) v[e] = make_float2(0.0f, 0.0f);
+    if (in) {
+      for (int wy = -1; wy <= 1; wy++) {
+        const RowTiles up = row_tiles(a, ch, r + wy * n), down = row_tiles(a, ch, -r - wy * n);
+        for (int wx = -1; wx <= 1; wx++) {
+#pragma unroll
+          for (int e = 0; e < 16; e++) {
+            const int c = (e < 8 ? j + e * T : j + e * T - n) + wx * n;
+            const float2 g = grid_at(a, up, down, q, c);
+            v[e].x += g.x;
+            v[e].y += g.y;
+          }
+        }
+      }
+    }
+  }
+  fft16<LG>(v, smem_f2 + l * span16(n), j, a.tw);
+  if (!in) return;
+  float2* h = a.H + (size_t)line * N;
+#pragma unroll
+  for (int s = 0; s < 8; s++) h[j + s * T] = v[kept_output(s)];
 }
 
-// An inverse FFT over the 2N cells of a line, of which the N outputs about
-// the middle are kept: X[x] = E[x mod N] + e^{2 pi i x / 2N} O[x mod N] with
-// the N-point transforms E, O of the even and odd cells.
-template <int VPT>
-__global__ void __launch_bounds__(VPT == 16 ? 512 : 256) k_nu_rows(
-    int N, int log2n, int cmin, int ncol, int nrow, const float2* __restrict__ F,
-    const float2* __restrict__ tw, const float2* __restrict__ turn, float2* __restrict__ H) {
-  extern __shared__ float2 buf[];
-  const float2* f = F + ((size_t)blockIdx.y * nrow + blockIdx.x) * ncol;
-  const int stride = fft_stride(N);
-  float2 v[VPT];
-#pragma unroll
-  for (int k = 0; k < VPT; k++) {
-    const int p = threadIdx.x + k * blockDim.x;
-    const int c = (p < N ? p : p - 2 * N) - cmin;
-    v[k] = (p < 2 * N && (unsigned)c < (unsigned)ncol) ? f[c] : make_float2(0.0f, 0.0f);
-  }
-#pragma unroll
-  for (int k = 0; k < VPT; k++) {
-    const int p = threadIdx.x + k * blockDim.x;
-    if (p < 2 * N) buf[(p & 1) * stride + fpad(p >> 1)] = v[k];
-  }
-  __syncthreads();
-  smem_fft<VPT>(buf, log2n, 2, tw);
-  float2* h = H + ((size_t)blockIdx.y * nrow + blockIdx.x) * N;
-  for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    const int m = (j + N / 2) & (N - 1);
-    const float2 e = buf[fpad(m)], o = cmul(buf[stride + fpad(m)], __ldg(turn + j));
-    h[j] = make_float2(e.x + o.x, e.y + o.y);
-  }
-}
-
-// The factor of every pixel's sum for one channel (blockIdx.y): beam,
-// fg_scale, GCF and the chain rule as the direct engines apply them, 0
-// outside the mask.
+// Per pixel and channel (blockIdx.y) the factor of the sum that does not
+// depend on the image: - fg_scale, beam, GCF and 1/V as the direct engines
+// apply them, 0 outside the mask.  Like the coefficients below it is fixed by
+// the problem, made once and laid out column by column ([j][i]), as the
+// column pass reads it.
 struct FactorArgs {
-  int N, c0;
-  int64_t MN;
-  int mode, flag_opt, normalize, pb;
-  float nu_0, D, pbf, pbcut, fg_scale, threshold;
+  int N, normalize, pb;
+  float D, pbf, pbcut, fg_scale;
   const float* __restrict__ beam_x;
   const float* __restrict__ beam_y;
   const float* __restrict__ chfreq;
   const int64_t* __restrict__ chnvis;
   const uint8_t* __restrict__ mask;
-  const float* __restrict__ img;
   const float* __restrict__ gcf;
   float* __restrict__ fac;
 };
 
 __global__ void __launch_bounds__(256) k_nu_factors(FactorArgs a) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= a.MN) return;
-  const int c = a.c0 + blockIdx.y;
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, MN = (int64_t)a.N * a.N;
+  if (q >= MN) return;
+  const int c = blockIdx.y;
+  const int j = (int)(q / a.N), i = (int)(q - (int64_t)j * a.N);
+  const int64_t px = (int64_t)a.N * i + j;
   float f = 0.0f;
-  if (a.mask[q] & kMaskIn) {
-    const int i = (int)(q / a.N), j = (int)(q - (int64_t)i * a.N);
-    const float freq = a.chfreq[c];
-    f = -(a.fg_scale *
-          attenuation_xy(a.beam_x[j], a.beam_y[i], freq, a.D, a.pbf, a.pbcut, a.pb));
-    if (a.gcf) f *= a.gcf[q];
+  if (a.mask[px] & kMaskIn) {
+    f = -(a.fg_scale * attenuation_xy(a.beam_x[j], a.beam_y[i], a.chfreq[c], a.D, a.pbf, a.pbcut,
+                                      a.pb));
+    if (a.gcf) f *= a.gcf[px];
     if (a.normalize) f /= (float)a.chnvis[c];
-    if (a.mode == 0) {
-      const float nudiv = freq / a.nu_0;
-      const float al = a.img[a.MN + q];
-      const float pw = al == 0.0f ? 1.0f : powf(nudiv, al);
-      if (a.flag_opt % 2 == 0) {
-        f *= pw;
-      } else {
-        const float i0 = a.img[q];
-        f = i0 > a.threshold ? f * (i0 * pw * a.fg_scale * logf(nudiv)) : 0.0f;
-      }
-    }
   }
-  a.fac[blockIdx.y * a.MN + q] = f;
+  a.fac[c * MN + q] = f;
 }
 
 // Per pixel and pair the w-term's coefficients of the transform's real and
@@ -428,7 +500,7 @@ __global__ void __launch_bounds__(256) k_nu_coefficients(int N, int pairs, float
                                                          float2* __restrict__ coef) {
   const int64_t px = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, MN = (int64_t)N * N;
   if (px >= MN) return;
-  const int i = (int)(px / N), j = (int)(px - (int64_t)i * N);
+  const int j = (int)(px / N), i = (int)(px - (int64_t)j * N);
   const float x = beam_x[j], y = beam_y[i], r2 = fmaf(x, x, y * y);
   // a / 2, a = wscale (z - 1)
   const float h = -0.5f * wscale * (r2 / (1.0f + sqrtf(1.0f - r2))), h2 = h * h;
@@ -444,81 +516,164 @@ __global__ void __launch_bounds__(256) k_nu_coefficients(int N, int pairs, float
 }
 
 struct ColArgs {
-  int N, log2n, lcb;  // 2^lcb columns per block
-  int64_t MN;
-  int nchan;          // channels of the group
-  int rmin, nrow;
-  int wterm;
+  int nchan, np, nrow, rmin;  // channels of the group, pairs
+  int wterm, alpha;           // alpha: the sum is the alpha plane's
   const float2* __restrict__ H;
   const float2* __restrict__ tw;
-  const float2* __restrict__ turn;
   const float* __restrict__ corr;
-  const float2* __restrict__ coef;  // [pair][MN]
-  const float* __restrict__ fac;    // [channel of the group][MN], or null: 1
-  const uint8_t* __restrict__ mask; // pixels written (kMaskIn), or null: all
+  const float2* __restrict__ coef;    // [pair][MN]
+  const float* __restrict__ fac;      // [channel of the group][MN], or null: 1
+  const float* __restrict__ chfreq;   // channel of the group
+  float nu_0, fg_scale, threshold;
+  const uint8_t* __restrict__ mask;   // pixels written (kMaskIn), or null: all
+  const float* __restrict__ img;      // the image's planes (chain rule), or null
   float* __restrict__ out;
 };
 
-template <int VPT, int NP>
-__global__ void __launch_bounds__(VPT == 16 ? 512 : 256, VPT == 16 ? 1 : 4) k_nu_cols(ColArgs a) {
-  extern __shared__ float2 buf[];
-  const int N = a.N, cb = 1 << a.lcb, j0 = blockIdx.x << a.lcb;
-  const int stride = fft_stride(N);
-  float acc[VPT / 2];
+// Column FFTs over the covered rows of 2N, the N outputs about the middle
+// kept, and the epilogue: every output's real and imaginary part with its
+// coefficients, the channel's factor and the chain rule
+// (src/functions.cu:3968-4024), summed over pairs and channels in registers.
+// kCols adjacent columns per block; kGroups sets of threads take the
+// (channel, pair) planes in turn and are added up at the end, so a small
+// image's few planes run side by side.
+template <int LG>
+struct ColShape {
+  static constexpr int kThreads = (1 << LG) / 16;  // per line
+  static constexpr int kCols = LG >= 13 ? 1 : (LG == 12 ? 2 : (LG == 11 ? 4 : 2));
+  static constexpr int kGroups = LG >= 11 ? 1 : 2;
+  static constexpr int kBlock = kThreads * kCols * kGroups;
+  // columns are this far apart: 16 / kCols more than a multiple of 16, so the
+  // lanes of a half warp, kCols columns wide, fall in distinct banks
+  static constexpr int kStride = (span16(1 << LG) + 15) / 16 * 16 + 16 / kCols;
+  static constexpr size_t kSmem =
+      sizeof(float2) * kGroups * kCols * kStride + sizeof(float) * 8 * kBlock;
+};
+
+// (nu / nu_0)^alpha out of line, for the kernels whose length in instructions
+// shows: the flat spectra of most images skip it
+__device__ __noinline__ float power(float nudiv, float al) {
+  return al == 0.0f ? 1.0f : powf(nudiv, al);
+}
+
+template <int LG>
+__global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 512 ? 2 : 1)
+    k_nu_cols(ColArgs a) {
+  using S = ColShape<LG>;
+  constexpr int n = 1 << LG, N = n / 2, T = S::kThreads, CB = S::kCols, G = S::kGroups;
+  extern __shared__ float2 smem_f2[];
+  const int cc = threadIdx.x % CB, j = (threadIdx.x / CB) % T, g = threadIdx.x / (CB * T);
+  float2* buf = smem_f2 + (g * CB + cc) * S::kStride;
+  const int col = blockIdx.x * CB + cc;
+  constexpr int64_t MN = (int64_t)N * N;
+  // the thread's pixels of the image's alpha plane, kept for all planes
+  float* al = reinterpret_cast<float*>(smem_f2 + G * CB * S::kStride) + threadIdx.x;
+  bool flat = true;
+  if (a.img) {
 #pragma unroll
-  for (int k = 0; k < VPT / 2; k++) acc[k] = 0.0f;
-  for (int c = 0; c < a.nchan; c++) {
-#pragma unroll 1
-    for (int q = 0; q < NP; q++) {
-      {
-        const float2* h = a.H + (size_t)(c * NP + q) * a.nrow * N + j0;
-        float2 v[VPT];
-#pragma unroll
-        for (int k = 0; k < VPT; k++) {
-          const int idx = threadIdx.x + k * blockDim.x;
-          const int p = idx >> a.lcb;
-          const int r = (p < N ? p : p - 2 * N) - a.rmin;
-          v[k] = (p < 2 * N && (unsigned)r < (unsigned)a.nrow)
-                     ? h[(size_t)r * N + (idx & (cb - 1))]
-                     : make_float2(0.0f, 0.0f);
-        }
-        __syncthreads();  // the last transform has been read
-#pragma unroll
-        for (int k = 0; k < VPT; k++) {
-          const int idx = threadIdx.x + k * blockDim.x;
-          const int p = idx >> a.lcb;
-          if (p < 2 * N) buf[(2 * (idx & (cb - 1)) + (p & 1)) * stride + fpad(p >> 1)] = v[k];
-        }
-      }
-      __syncthreads();
-      smem_fft<VPT>(buf, a.log2n, 2 * cb, a.tw);
-#pragma unroll
-      for (int k = 0; k < VPT / 2; k++) {
-        const int idx = threadIdx.x + k * blockDim.x;
-        const int i = idx >> a.lcb, cc = idx & (cb - 1);
-        if (i >= N) continue;
-        const int64_t px = (int64_t)N * i + j0 + cc;
-        const int m = fpad((i + N / 2) & (N - 1));
-        const float2 e = buf[2 * cc * stride + m];
-        const float2 o = cmul(buf[(2 * cc + 1) * stride + m], __ldg(a.turn + i));
-        float t;
-        if (a.wterm) {
-          const float2 kk = __ldg(a.coef + q * a.MN + px);
-          t = fmaf(kk.x, e.x + o.x, kk.y * (e.y + o.y));
-        } else {
-          t = q == 0 ? (e.x + o.x) * (__ldg(a.corr + i) * __ldg(a.corr + j0 + cc)) : 0.0f;
-        }
-        acc[k] = fmaf(a.fac ? __ldg(a.fac + c * a.MN + px) : 1.0f, t, acc[k]);
-      }
+    for (int s = 0; s < 8; s++) {
+      const float v = __ldg(a.img + MN + (int64_t)N * (j + s * T) + col);
+      al[s * S::kBlock] = v;
+      flat = flat && v == 0.0f;
     }
   }
+  // small sides, whose blocks run once through a plane or two: everything the
+  // end needs is on its way before the first transform
+  constexpr bool kAhead = LG <= 10;
+  float old[kAhead ? 8 : 1];
+  bool write[kAhead ? 8 : 1];
+  if constexpr (kAhead) {
 #pragma unroll
-  for (int k = 0; k < VPT / 2; k++) {
-    const int idx = threadIdx.x + k * blockDim.x;
-    const int i = idx >> a.lcb;
-    if (i >= N) continue;
-    const int64_t px = (int64_t)N * i + j0 + (idx & (cb - 1));
-    if (!a.mask || (a.mask[px] & kMaskIn)) a.out[px] += acc[k];
+    for (int s = 0; s < 8; s++) {
+      const int64_t px = (int64_t)N * (j + s * T) + col;
+      write[s] = !a.mask || (a.mask[px] & kMaskIn);
+      old[s] = a.out[px];
+    }
+  }
+  float acc[8];
+#pragma unroll
+  for (int s = 0; s < 8; s++) acc[s] = 0.0f;
+  const int planes = a.nchan * a.np;
+  for (int p0 = 0; p0 < planes; p0 += G) {
+    const int p = p0 + g;
+    const bool in = p < planes;
+    const int c = p / a.np, q = p - c * a.np;
+    float2 v[16];
+    {
+      // rows below 0 first in memory: row r of the plane at r - rmin
+      const float2* h = a.H + ((int64_t)p * a.nrow - a.rmin + j) * N + col;
+      const unsigned lo = (unsigned)(j - a.rmin);
+#pragma unroll
+      for (int e = 0; e < 16; e++) {
+        const int o = e < 8 ? e * T : e * T - n;
+        v[e] = in && lo + (unsigned)o < (unsigned)a.nrow ? h[(int64_t)o * N]
+                                                         : make_float2(0.0f, 0.0f);
+      }
+    }
+    const float2* kq = a.coef + q * MN + (int64_t)N * col + j;
+    const float* fc = a.fac ? a.fac + c * MN + (int64_t)N * col + j : nullptr;
+    float2 kk[kAhead ? 8 : 1];
+    float ff[kAhead ? 8 : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int s = 0; s < 8; s++) {
+        kk[s] = in ? __ldg(kq + s * T) : make_float2(0.0f, 0.0f);
+        ff[s] = in && fc ? __ldg(fc + s * T) : 1.0f;
+      }
+    }
+    __syncthreads();  // the last line has been read
+    fft16<LG>(v, buf, j, a.tw);
+    if (!in) continue;
+    const float nudiv = a.img ? a.chfreq[c] / a.nu_0 : 1.0f;
+    const float lg = a.alpha ? logf(nudiv) : 1.0f;
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      const float2 x = v[kept_output(s)];
+      float t;
+      if (a.wterm) {
+        const float2 k = kAhead ? kk[kAhead ? s : 0] : __ldg(kq + s * T);
+        t = fmaf(k.x, x.x, k.y * x.y);
+      } else {
+        t = q == 0 ? x.x * (__ldg(a.corr + j + s * T) * __ldg(a.corr + col)) : 0.0f;
+      }
+      float f = kAhead ? ff[kAhead ? s : 0] : (fc ? __ldg(fc + s * T) : 1.0f);
+      f *= lg;
+      if (!flat) {
+        const float av = al[s * S::kBlock];
+        if constexpr (kAhead) {
+          f *= power(nudiv, av);
+        } else if (av != 0.0f) {
+          f *= powf(nudiv, av);
+        }
+      }
+      acc[s] = fmaf(f, t, acc[s]);
+    }
+  }
+  if constexpr (G > 1) {
+    // the groups' sums, in order
+    float* part = reinterpret_cast<float*>(smem_f2);
+    __syncthreads();
+    if (g > 0) {
+#pragma unroll
+      for (int s = 0; s < 8; s++) part[((g - 1) * 8 + s) * T * CB + threadIdx.x % (T * CB)] = acc[s];
+    }
+    __syncthreads();
+    if (g > 0) return;
+    for (int o = 0; o < G - 1; o++)
+#pragma unroll
+      for (int s = 0; s < 8; s++) acc[s] += part[(o * 8 + s) * T * CB + threadIdx.x];
+  }
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    const int64_t px = (int64_t)N * (j + s * T) + col;
+    if (!(kAhead ? write[kAhead ? s : 0] : !a.mask || (a.mask[px] & kMaskIn))) continue;
+    float t = acc[s];
+    if (a.alpha) {
+      const float i0 = a.img[px];
+      if (!(i0 > a.threshold)) continue;
+      t *= i0 * a.fg_scale;
+    }
+    a.out[px] = (kAhead ? old[kAhead ? s : 0] : a.out[px]) + t;
   }
 }
 
@@ -594,49 +749,38 @@ std::vector<float> kernel_correction(int N) {
   return c;
 }
 
-template <int NP>
-gv_status spread(const SpreadArgs& a, cudaStream_t st) {
-  const size_t smem =
-      sizeof(float4) * kSpreadWarps * (size_t)(NP * kTilePts + NP * 32 + 32 * 5);
+template <int NP, int W>
+gv_status spread_warps(const SpreadArgs& a, cudaStream_t st) {
+  const size_t smem = sizeof(float4) * W * (size_t)(NP * kTilePts + NP * 32 + 32 * 5);
   if (smem > 48 * 1024)
-    GV_CUDA(cudaFuncSetAttribute(k_nu_spread<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GV_CUDA(cudaFuncSetAttribute(k_nu_spread<NP, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  k_nu_spread<NP><<<(a.ntasks + kSpreadWarps - 1) / kSpreadWarps, 32 * kSpreadWarps, smem, st>>>(a);
+  k_nu_spread<NP, W><<<a.ntasks, 32 * W, smem, st>>>(a);
   GV_LAUNCH("k_nu_spread");
   return GV_OK;
 }
 
-template <int VPT>
-gv_status rows(const Problem& P, const NuPlan& n, int nplanes, int threads, const float2* tw) {
-  const size_t smem = sizeof(float2) * 2 * fft_stride(P.N);
-  if (smem > 48 * 1024)
-    GV_CUDA(cudaFuncSetAttribute(k_nu_rows<VPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  k_nu_rows<VPT><<<dim3(n.nrow, nplanes), threads, smem, P.stream>>>(
-      P.N, P.log2n, n.cmin, n.ncol, n.nrow, n.d_F, tw, n.d_turn, n.d_H);
-  GV_LAUNCH("k_nu_rows");
-  return GV_OK;
+template <int NP>
+gv_status spread(const SpreadArgs& a, int warps, cudaStream_t st) {
+  return warps == 8 ? spread_warps<NP, 8>(a, st) : spread_warps<NP, 1>(a, st);
 }
 
-template <int VPT, int NP>
-gv_status cols(const ColArgs& a, int threads, cudaStream_t st) {
-  const size_t smem = sizeof(float2) * (size_t)(2 << a.lcb) * fft_stride(a.N);
+template <int LG>
+gv_status transforms(const Problem& P, const RowArgs& ra, const ColArgs& ca) {
+  constexpr int L = RowShape<LG>::kLines;
+  const size_t smem = sizeof(float2) * L * span16(1 << LG);
   if (smem > 48 * 1024)
-    GV_CUDA(cudaFuncSetAttribute(k_nu_cols<VPT, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GV_CUDA(cudaFuncSetAttribute(k_nu_rows<LG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  k_nu_cols<VPT, NP><<<a.N >> a.lcb, threads, smem, st>>>(a);
+  k_nu_rows<LG><<<(ra.lines + L - 1) / L, RowShape<LG>::kThreads * L, smem, P.stream>>>(ra);
+  GV_LAUNCH("k_nu_rows");
+  using S = ColShape<LG>;
+  if (S::kSmem > 48 * 1024)
+    GV_CUDA(cudaFuncSetAttribute(k_nu_cols<LG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)S::kSmem));
+  k_nu_cols<LG><<<P.N / S::kCols, S::kBlock, S::kSmem, P.stream>>>(ca);
   GV_LAUNCH("k_nu_cols");
   return GV_OK;
-}
-
-template <int VPT>
-gv_status cols_pairs(int pairs, const ColArgs& a, int threads, cudaStream_t st) {
-  switch (pairs) {
-    case 1: return cols<VPT, 1>(a, threads, st);
-    case 2: return cols<VPT, 2>(a, threads, st);
-    case 3: return cols<VPT, 3>(a, threads, st);
-    default: return cols<VPT, 4>(a, threads, st);
-  }
 }
 
 // largest |z - 1| over the image
@@ -655,11 +799,11 @@ void nu_free(Problem& P) {
   if (!P.nu) return;
   NuPlan* n = P.nu;
   cudaFree(n->d_tasks);
-  cudaFree(n->d_slot_off);
+  cudaFree(n->d_slot);
+  cudaFree(n->d_done);
   cudaFree(n->d_slots);
-  cudaFree(n->d_F);
   cudaFree(n->d_H);
-  cudaFree(n->d_turn);
+  cudaFree(n->d_twiddle);
   cudaFree(n->d_corr);
   cudaFree(n->d_coef);
   cudaFree(n->d_fac);
@@ -667,8 +811,8 @@ void nu_free(Problem& P) {
   P.nu = nullptr;
 }
 
-// The pixels' w-term coefficients, once the beam tables (the pixels' offsets)
-// are in place.
+// The pixels' w-term coefficients and factors, once the beam tables (the
+// pixels' offsets), the mask and the channels' tables are in place.
 gv_status nu_finish(Problem& P) {
   if (!P.nu) return GV_OK;
   const NuPlan& n = *P.nu;
@@ -676,6 +820,11 @@ gv_status nu_finish(Problem& P) {
   k_nu_coefficients<<<(unsigned)((MN + 255) / 256), 256, 0, P.stream>>>(
       P.N, n.pairs, (float)(2.0 * kPiD * n.wmax), P.d_beam_x, P.d_beam_y, n.d_corr, n.d_coef);
   GV_LAUNCH("k_nu_coefficients");
+  const FactorArgs fa{P.N, P.normalize, P.pb, P.D, P.pbf, P.pbcut, P.fg_scale, P.d_beam_x,
+                      P.d_beam_y, P.d_chfreq, P.d_chnvis, P.d_mask, P.d_gcf, n.d_fac};
+  k_nu_factors<<<dim3((unsigned)((MN + 255) / 256), (unsigned)P.chans.size()), 256, 0,
+                 P.stream>>>(fa);
+  GV_LAUNCH("k_nu_factors");
   return GV_OK;
 }
 
@@ -765,17 +914,20 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   const int rmax = std::max(rhi, -rlo);
   n->wrap = cmax > N - 1 || rmax > N - 1;
   n->cmin = n->wrap ? -N : -cmax;
-  n->ncol = n->wrap ? 2 * N : (2 * cmax + 1 + 1) & ~1;
+  n->ncol = n->wrap ? 2 * N : 2 * cmax + 1;
   n->rmin = n->wrap ? -N : -rmax;
   n->nrow = n->wrap ? 2 * N : 2 * rmax + 1;
   // ---- tasks ------------------------------------------------------------------
-  // a tile's visibilities in pieces of T: enough pieces to fill the GPU (32
-  // warps per SM) without more slots than the sums are worth
-  const int64_t want = P.Vgrid / std::max(1, 32 * P.num_sms);
-  const int T = (int)std::min<int64_t>(1024, std::max<int64_t>(32, want / 32 * 32));
+  // A tile's visibilities in pieces of T, a block each.  Few and well filled
+  // tiles: the blocks run nearly at once and their longest chain decides, so
+  // 8 warps share a piece of 512 (256^2, 104,400 visibilities in 290 tiles:
+  // the whole evaluation 89 us, against 110 with 4 warps and pieces of 128).
+  // Otherwise one warp a piece, so that none idles in a thin tile.
+  n->warps = R <= (size_t)(16 * P.num_sms) && P.Vgrid >= 64 * (int64_t)R ? 8 : 1;
+  const int T = n->warps == 8 ? 512 : 1024;
   std::vector<NuTask> tasks;
   const size_t tiles = (size_t)n->nty * n->ntx;
-  std::vector<int> off((size_t)C * tiles + 1, 0);
+  std::vector<int> slot((size_t)C * tiles, -1);
   n->task_off.assign(C + 1, 0);
   for (size_t r = 0; r < R; r++) {
     const uint32_t t = (uint32_t)(rkey[r] & 0x3FFFFFFu);
@@ -784,18 +936,17 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     const int64_t end = (r + 1 < R && (int)(rkey[r + 1] >> 26) == c) ? rstart[r + 1] : end_c;
     const int64_t cnt = end - rstart[r];
     const int parts = (int)((cnt + T - 1) / T);
+    const int first = (int)tasks.size();
     for (int k = 0; k < parts; k++) {
       const int64_t b = (int64_t)T * k;
-      tasks.push_back({(uint32_t)(rstart[r] + b), (int)std::min<int64_t>(T, cnt - b)});
+      tasks.push_back({(uint32_t)(rstart[r] + b), (int)std::min<int64_t>(T, cnt - b), first, parts});
     }
-    off[(size_t)c * tiles + (t / NTX - tya) * n->ntx + (t % NTX - txa) + 1] = parts;
+    slot[(size_t)c * tiles + (t / NTX - tya) * n->ntx + (t % NTX - txa)] = first;
     n->task_off[c + 1] += parts;
   }
-  for (size_t k = 1; k < off.size(); k++) off[k] += off[k - 1];
   for (int c = 0; c < C; c++) n->task_off[c + 1] += n->task_off[c];
   // ---- channel groups whose workspace stays bounded ------------------------------
   const size_t slot_b = sizeof(float2) * 2 * kTilePts * pairs;
-  const size_t f_b = sizeof(float2) * (size_t)pairs * n->nrow * n->ncol;
   const size_t h_b = sizeof(float2) * (size_t)pairs * n->nrow * N;
   const size_t fac_b = sizeof(float) * (size_t)N * N;
   n->groups.push_back(0);
@@ -804,7 +955,7 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     size_t used = 0;
     const int c0 = c;
     while (c < C) {
-      const size_t need = slot_b * (n->task_off[c + 1] - n->task_off[c]) + f_b + h_b + fac_b;
+      const size_t need = slot_b * (n->task_off[c + 1] - n->task_off[c]) + h_b;
       if (c > c0 && used + need > kWorkspace) break;
       used += need;
       c++;
@@ -813,23 +964,26 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     max_ch = std::max<size_t>(max_ch, c - c0);
     max_slots = std::max<size_t>(max_slots, n->task_off[c] - n->task_off[c0]);
   }
-  std::vector<float2> turn(N);
-  for (int j = 0; j < N; j++) {
-    const double t = kPiD * (j - N / 2) / N;
-    turn[j] = make_float2((float)std::cos(t), (float)std::sin(t));
-  }
+  const int lg = P.log2n + 1;
+  std::vector<float2> tw;
+  for (int l = fft16_first(lg); l < lg; l += 4)
+    for (int r = 1; r < 16; r++)
+      for (int k = 0; k < (1 << l); k++) {
+        const double t = 2.0 * kPiD * r * k / (double)(16 << l);
+        tw.push_back(make_float2((float)std::cos(t), (float)std::sin(t)));
+      }
   const std::vector<float> corr = kernel_correction(N);
   tap_polynomials(n->coef);
   auto upload = [&]() -> cudaError_t {
     cudaError_t e = cudaMalloc(&n->d_tasks, sizeof(NuTask) * tasks.size());
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_slot_off, sizeof(int) * off.size());
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_slot, sizeof(int) * slot.size());
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_done, sizeof(uint32_t) * tasks.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_slots, slot_b * max_slots);
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_F, f_b * max_ch);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_H, h_b * max_ch);
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_turn, sizeof(float2) * N);
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_twiddle, sizeof(float2) * tw.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_corr, sizeof(float) * N);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_coef, sizeof(float2) * (size_t)pairs * N * N);
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_fac, fac_b * max_ch);
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_fac, fac_b * C);
     return e;
   };
   const cudaError_t e = upload();
@@ -842,9 +996,9 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   if (e != cudaSuccess) return cuda_fail(e, "nu_setup");
   GV_CUDA(cudaMemcpy(n->d_tasks, tasks.data(), sizeof(NuTask) * tasks.size(),
                      cudaMemcpyHostToDevice));
-  GV_CUDA(cudaMemcpy(n->d_slot_off, off.data(), sizeof(int) * off.size(),
-                     cudaMemcpyHostToDevice));
-  GV_CUDA(cudaMemcpy(n->d_turn, turn.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+  GV_CUDA(cudaMemcpy(n->d_slot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice));
+  GV_CUDA(cudaMemset(n->d_done, 0, sizeof(uint32_t) * tasks.size()));
+  GV_CUDA(cudaMemcpy(n->d_twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   GV_CUDA(cudaMemcpy(n->d_corr, corr.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
   return GV_OK;
 }
@@ -867,59 +1021,40 @@ gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result
   sa.shift_x = N / 2 - (int)P.xobs;
   sa.shift_y = N / 2 - (int)P.yobs;
   std::copy(&n.coef[0][0], &n.coef[0][0] + sizeof(n.coef) / sizeof(float), &sa.coef[0][0]);
-  MergeArgs ma;
-  ma.slots = n.d_slots;
-  ma.slot_off = n.d_slot_off;
-  ma.F = n.d_F;
-  ma.N = N;
-  ma.pairs = np;
-  ma.cmin = n.cmin;
-  ma.ncol = n.ncol;
-  ma.rmin = n.rmin;
-  ma.nrow = n.nrow;
-  ma.wrap = n.wrap;
-  ma.tx0 = n.tx0;
-  ma.ntx = n.ntx;
-  ma.ty0 = n.ty0;
-  ma.nty = n.nty;
+  sa.done = n.d_done;
+  RowArgs ra;
+  ra.slots = n.d_slots;
+  ra.slot = n.d_slot;
+  ra.tw = n.d_twiddle;
+  ra.H = n.d_H;
+  ra.N = N;
+  ra.pairs = np;
+  ra.cmin = n.cmin;
+  ra.ncol = n.ncol;
+  ra.rmin = n.rmin;
+  ra.nrow = n.nrow;
+  ra.wrap = n.wrap;
+  ra.tx0 = n.tx0;
+  ra.ntx = n.ntx;
+  ra.ty0 = n.ty0;
+  ra.nty = n.nty;
+  const int64_t MN = (int64_t)P.M * N;
   ColArgs ca;
-  ca.N = N;
-  ca.log2n = P.log2n;
-  ca.MN = (int64_t)P.M * N;
-  ca.rmin = n.rmin;
+  ca.np = np;
   ca.nrow = n.nrow;
-  ca.H = n.d_H;
-  ca.tw = P.d_twiddle;
-  ca.turn = n.d_turn;
-  ca.corr = n.d_corr;
+  ca.rmin = n.rmin;
   ca.wterm = mode == 4 ? 0 : 1;
+  ca.alpha = mode == 0 && flag_opt % 2 != 0;
+  ca.H = n.d_H;
+  ca.tw = n.d_twiddle;
+  ca.corr = n.d_corr;
   ca.coef = n.d_coef;
-  ca.fac = mode <= 1 ? n.d_fac : nullptr;
+  ca.nu_0 = P.nu_0;
+  ca.fg_scale = P.fg_scale;
+  ca.threshold = P.threshold;
   ca.mask = mode <= 1 ? P.d_mask : nullptr;
-  ca.out = d_result + (mode == 0 ? (int64_t)(flag_opt % 2) * ca.MN : 0);
-  FactorArgs fa;
-  fa.N = N;
-  fa.MN = ca.MN;
-  fa.mode = mode;
-  fa.flag_opt = flag_opt;
-  fa.normalize = P.normalize;
-  fa.pb = P.pb;
-  fa.nu_0 = P.nu_0;
-  fa.D = P.D;
-  fa.pbf = P.pbf;
-  fa.pbcut = P.pbcut;
-  fa.fg_scale = P.fg_scale;
-  fa.threshold = P.threshold;
-  fa.beam_x = P.d_beam_x;
-  fa.beam_y = P.d_beam_y;
-  fa.chfreq = P.d_chfreq;
-  fa.chnvis = P.d_chnvis;
-  fa.mask = P.d_mask;
-  fa.img = d_img;
-  fa.gcf = P.d_gcf;
-  fa.fac = n.d_fac;
-  // columns per block: 256 blocks or more, 8192 values a block at most
-  ca.lcb = N <= 256 ? 0 : (N == 512 ? 1 : (N == 1024 ? 2 : (N == 2048 ? 1 : 0)));
+  ca.img = mode == 0 ? d_img : nullptr;
+  ca.out = d_result + (mode == 0 ? (int64_t)(flag_opt % 2) * MN : 0);
   std::vector<int> one = {only_channel, only_channel + 1};
   const std::vector<int>& groups = only_channel >= 0 ? one : n.groups;
   for (size_t g = 0; g + 1 < groups.size(); g++) {
@@ -927,30 +1062,31 @@ gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result
     const int t0 = n.task_off[c0];
     sa.tasks = n.d_tasks + t0;
     sa.ntasks = n.task_off[c1] - t0;
+    sa.t0 = t0;
     if (sa.ntasks == 0) continue;
     switch (np) {
-      case 1: GV_TRY(spread<1>(sa, P.stream)); break;
-      case 2: GV_TRY(spread<2>(sa, P.stream)); break;
-      case 3: GV_TRY(spread<3>(sa, P.stream)); break;
-      default: GV_TRY(spread<4>(sa, P.stream)); break;
+      case 1: GV_TRY(spread<1>(sa, n.warps, P.stream)); break;
+      case 2: GV_TRY(spread<2>(sa, n.warps, P.stream)); break;
+      case 3: GV_TRY(spread<3>(sa, n.warps, P.stream)); break;
+      default: GV_TRY(spread<4>(sa, n.warps, P.stream)); break;
     }
-    ma.c0 = c0;
-    ma.t0 = t0;
-    k_nu_merge<<<dim3((n.ncol + 127) / 128, n.nrow, nch * np), 128, 0, P.stream>>>(ma);
-    GV_LAUNCH("k_nu_merge");
-    if (N <= 256) GV_TRY(rows<2>(P, n, nch * np, 256, P.d_twiddle));
-    else if (N == 512) GV_TRY(rows<4>(P, n, nch * np, 256, P.d_twiddle));
-    else if (N == 1024) GV_TRY(rows<8>(P, n, nch * np, 256, P.d_twiddle));
-    else GV_TRY(rows<16>(P, n, nch * np, N == 2048 ? 256 : 512, P.d_twiddle));
-    if (mode <= 1) {
-      fa.c0 = c0;
-      k_nu_factors<<<dim3((unsigned)((ca.MN + 255) / 256), nch), 256, 0, P.stream>>>(fa);
-      GV_LAUNCH("k_nu_factors");
-    }
+    ra.c0 = c0;
+    ra.t0 = t0;
+    ra.lines = nch * np * n.nrow;
     ca.nchan = nch;
-    if (N <= 256) GV_TRY(cols_pairs<2>(np, ca, 256, P.stream));
-    else if (N == 512) GV_TRY(cols_pairs<8>(np, ca, 256, P.stream));
-    else GV_TRY(cols_pairs<16>(np, ca, 512, P.stream));
+    ca.fac = mode <= 1 ? n.d_fac + c0 * MN : nullptr;
+    ca.chfreq = P.d_chfreq + c0;
+    switch (P.log2n) {
+      case 4: GV_TRY(transforms<5>(P, ra, ca)); break;
+      case 5: GV_TRY(transforms<6>(P, ra, ca)); break;
+      case 6: GV_TRY(transforms<7>(P, ra, ca)); break;
+      case 7: GV_TRY(transforms<8>(P, ra, ca)); break;
+      case 8: GV_TRY(transforms<9>(P, ra, ca)); break;
+      case 9: GV_TRY(transforms<10>(P, ra, ca)); break;
+      case 10: GV_TRY(transforms<11>(P, ra, ca)); break;
+      case 11: GV_TRY(transforms<12>(P, ra, ca)); break;
+      default: GV_TRY(transforms<13>(P, ra, ca)); break;
+    }
   }
   return GV_OK;
 }

@@ -137,4 +137,98 @@ __device__ void smem_fft(float2* buf, int log2n, int ncol, const float2* __restr
   else if (log2n - lNs == 1) stockham_pass<1, VPT>(buf, log2n, ncol, lNs, tw);
 }
 
+// ---- 16 values a thread, radix 16 -----------------------------------------
+// Inverse FFT of a line of n = 2^LG elements by n / 16 threads, thread j
+// holding elements j + e n / 16 (e < 16) in v before and after every pass: a
+// first pass of radix 2^((LG - 1) % 4 + 1), then radix 16.  Against the
+// radix-8 passes above: the first pass reads its elements from where the
+// caller has them and the last leaves them in registers, so a 4096-point line
+// crosses shared memory twice instead of five times, with 4 barriers instead
+// of 10; the twiddles lie pass by pass in the order the lanes read them.
+//
+// Shared-memory position of element e: one float2 of padding after every 16,
+// which puts every write and read of a half warp into distinct banks.
+__device__ __forceinline__ int pad16(int e) { return e + (e >> 4); }
+__host__ __device__ constexpr int span16(int n) { return n + (n >> 4); }
+
+// multiplication by e^{2 pi i s / 16}, 0 <= s < 8 (compile-time after unrolling)
+__device__ __forceinline__ float2 rot16(float2 d, int s) {
+  constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f;
+  if (s == 1) return cmul(d, make_float2(c1, s1));
+  if (s == 3) return cmul(d, make_float2(s1, c1));
+  if (s == 5) return cmul(d, make_float2(-s1, c1));
+  if (s == 7) return cmul(d, make_float2(-c1, s1));
+  return rot_turn(d, s >> 1, 8);
+}
+
+// 16-point inverse DFT in registers; X[r] = v[brev_c<4>(r)]
+__device__ __forceinline__ void dft16(float2 (&v)[16]) {
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    const float2 a = v[s], b = v[s + 8];
+    v[s] = make_float2(a.x + b.x, a.y + b.y);
+    v[s + 8] = rot16(make_float2(a.x - b.x, a.y - b.y), s);
+  }
+  float2(&lo)[8] = reinterpret_cast<float2(&)[8]>(v[0]);
+  float2(&hi)[8] = reinterpret_cast<float2(&)[8]>(v[8]);
+  dft_inv<3>(lo);
+  dft_inv<3>(hi);
+}
+
+__host__ __device__ constexpr int fft16_first(int lg) { return (lg - 1) % 4 + 1; }
+
+// Entries of the twiddle table of a 2^lg-point line: for every pass after the
+// first, with Ns = the product of the radices before it,
+// e^{2 pi i r k / (16 Ns)} at (r - 1) Ns + k, 1 <= r < 16, k < Ns.
+__host__ __device__ constexpr int fft16_twiddles(int lg) {
+  int n = 0;
+  for (int l = fft16_first(lg); l < lg; l += 4) n += 15 << l;
+  return n;
+}
+
+// All passes of a line; `buf` holds span16(2^LG) float2 for it, and every
+// thread of the block makes the same calls.  On return element x of the
+// result with x = j + r n / 16 is v[brev_c<4>(r)].
+template <int LG>
+__device__ __forceinline__ void fft16(float2 (&v)[16], float2* buf, int j,
+                                      const float2* __restrict__ tw) {
+  constexpr int T = (1 << LG) / 16, L0 = fft16_first(LG), R0 = 1 << L0, M0 = 16 / R0;
+  if constexpr (L0 == 4) {
+    dft16(v);
+  } else {
+#pragma unroll
+    for (int m = 0; m < M0; m++) {
+      float2 u[R0];
+#pragma unroll
+      for (int r = 0; r < R0; r++) u[r] = v[m + r * M0];
+      dft_inv<L0>(u);
+#pragma unroll
+      for (int r = 0; r < R0; r++) v[m + r * M0] = u[r];
+    }
+  }
+  // y[R0 (j + m T) + r] of item m
+#pragma unroll
+  for (int m = 0; m < M0; m++)
+#pragma unroll
+    for (int r = 0; r < R0; r++)
+      buf[pad16(R0 * (j + m * T) + r)] = v[m + brev_c<L0>(r) * M0];
+#pragma unroll
+  for (int l = L0; l < LG; l += 4) {
+    const int k = j & ((1 << l) - 1);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = buf[pad16(j + r * T)];
+#pragma unroll
+    for (int r = 1; r < 16; r++) v[r] = cmul(v[r], __ldg(tw + ((r - 1) << l) + k));
+    tw += 15 << l;
+    dft16(v);
+    if (l + 4 < LG) {
+      __syncthreads();
+      const int base = ((j >> l) << (l + 4)) + k;
+#pragma unroll
+      for (int r = 0; r < 16; r++) buf[pad16(base + (r << l))] = v[brev_c<4>(r)];
+    }
+  }
+}
+
 }  // namespace gv

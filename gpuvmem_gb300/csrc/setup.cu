@@ -686,7 +686,6 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     GV_CUDA(cudaMemcpy(P.d_rot_u, ru.data(), sizeof(float) * P.N, cudaMemcpyHostToDevice));
     GV_CUDA(cudaMemcpy(P.d_rot_v, rv.data(), sizeof(float) * P.M, cudaMemcpyHostToDevice));
   }
-  GV_TRY(nu_finish(P));
   GV_CUDA(cudaMalloc(&P.d_grid, sizeof(float2) * MN * C));
   {
     std::vector<float> f(C);
@@ -713,6 +712,7 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     GV_CUDA(cudaMemcpy(P.d_kc_off, kc.data(), sizeof(int64_t) * (C + 1), cudaMemcpyHostToDevice));
     GV_CUDA(cudaMemcpy(P.d_kc_one, k1.data(), sizeof(int64_t) * 2 * C, cudaMemcpyHostToDevice));
   }
+  GV_TRY(nu_finish(P));
   GV_CUDA(cudaMalloc(&P.d_flags, sizeof(uint32_t) * kNumFlags));
   GV_CUDA(cudaMemsetAsync(P.d_flags, 0, sizeof(uint32_t) * kNumFlags, st));
   {
