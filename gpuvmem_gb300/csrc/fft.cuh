@@ -65,7 +65,7 @@ __device__ __forceinline__ constexpr int brev_c(int r) {
 // lines of a multi-column buffer are fft_stride(n) apart (four more, so four
 // columns read row by row do not share banks either).
 __device__ __forceinline__ int fpad(int e) { return e + (e >> 3); }
-__host__ __device__ __forceinline__ int fft_span(int n) { return n + (n >> 3); }
+__host__ __device__ constexpr int fft_span(int n) { return n + (n >> 3); }
 __host__ __device__ __forceinline__ int fft_stride(int n) { return fft_span(n) + 4; }
 
 // One Stockham autosort pass of radix R = 2^LR over `ncol` columns of length
@@ -135,6 +135,73 @@ __device__ void smem_fft(float2* buf, int log2n, int ncol, const float2* __restr
   }
   if (log2n - lNs == 2) stockham_pass<2, VPT>(buf, log2n, ncol, lNs, tw);
   else if (log2n - lNs == 1) stockham_pass<1, VPT>(buf, log2n, ncol, lNs, tw);
+}
+
+// ---- 8 values a thread, the passes above ------------------------------------
+// The same transform as smem_fft (the same butterflies and twiddles on the
+// same values, so the same bits) of a line of n = 2^LG elements by n / 8
+// threads, thread j holding elements j + e n / 8 (e < 8) in v before the first
+// pass and after the last, in natural order of e.  The first pass takes its
+// elements from the caller's registers and the last leaves them there, so a
+// 2048-point line crosses shared memory three times instead of five, with 6
+// barriers instead of 10; the twiddles lie pass by pass in lane order (a
+// strided table costs a sector per lane).  `buf` holds fft_span(2^LG) float2.
+//
+// Table: for every pass after the first, with Ns the product of the radices
+// before it and R its radix, e^{2 pi i r k / (R Ns)} at (r - 1) Ns + k,
+// 1 <= r < R, k < Ns.
+__host__ __device__ constexpr int fft8_radix(int lg, int l) { return lg - l >= 3 ? 3 : lg - l; }
+__host__ __device__ constexpr int fft8_twiddles(int lg) {
+  int n = 0;
+  for (int l = 3; l < lg; l += 3) n += ((1 << fft8_radix(lg, l)) - 1) << l;
+  return n;
+}
+
+template <int LG, int L>
+__device__ __forceinline__ void fft8_passes(float2 (&v)[8], float2* buf, int j,
+                                            const float2* __restrict__ tw) {
+  constexpr int T = (1 << LG) / 8, LR = fft8_radix(LG, L), R = 1 << LR, M = 8 / R;
+  // the last pass' results: element ((j >> L - 3) << L) + k + r 2^(L - 3)
+  const int kw = j & ((1 << (L - 3)) - 1), base = ((j >> (L - 3)) << L) + kw;
+#pragma unroll
+  for (int r = 0; r < 8; r++) buf[fpad(base + (r << (L - 3)))] = v[brev_c<3>(r)];
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 8; e++) v[e] = buf[fpad(j + e * T)];
+  if constexpr (LR == 3) {
+    const int k = j & ((1 << L) - 1);
+#pragma unroll
+    for (int r = 1; r < 8; r++) v[r] = cmul(v[r], __ldg(tw + ((r - 1) << L) + k));
+    dft_inv<3>(v);
+    if constexpr (L + 3 < LG) {
+      __syncthreads();
+      fft8_passes<LG, L + 3>(v, buf, j, tw + (7 << L));
+    } else {
+      float2 u[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) u[r] = v[brev_c<3>(r)];
+#pragma unroll
+      for (int r = 0; r < 8; r++) v[r] = u[r];
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      float2 u[R];
+      u[0] = v[m];
+#pragma unroll
+      for (int r = 1; r < R; r++) u[r] = cmul(v[m + r * M], __ldg(tw + ((r - 1) << L) + j + m * T));
+      dft_inv<LR>(u);
+#pragma unroll
+      for (int r = 0; r < R; r++) v[m + r * M] = u[brev_c<LR>(r)];
+    }
+  }
+}
+
+template <int LG>
+__device__ __forceinline__ void fft8(float2 (&v)[8], float2* buf, int j,
+                                     const float2* __restrict__ tw) {
+  dft_inv<3>(v);
+  fft8_passes<LG, 3>(v, buf, j, tw);
 }
 
 // ---- 16 values a thread, radix 16 -----------------------------------------

@@ -114,6 +114,11 @@ struct Problem {
   float* d_rho = nullptr;        // [MN] z - 1 + r^2/2 per pixel
   float2* d_grid = nullptr;      // [C][MN] model grids
   float2* d_twiddle = nullptr;   // [n] e^{+2 pi i m/n} (objective.cu smem_fft)
+  float2* d_tw8 = nullptr;       // fft8_twiddles(log2n): twiddles pass by pass (fft8)
+  float* d_atten = nullptr;      // [C][MN] beam of every pixel and channel
+  uint8_t* d_need = nullptr;     // [N + N] columns, then rows, of the grids that are read
+  int* d_col_blocks = nullptr;   // the column pass' blocks with a needed column
+  int col_blocks = 0;
   float* d_beam_x = nullptr;     // [N] beam_coord of each column (attenuation)
   float* d_beam_y = nullptr;     // [M] beam_coord of each row
   float* d_rot_u = nullptr;      // [N] phase_rotate's u of each column (k_cols_fft)
@@ -348,6 +353,7 @@ struct XtSource {
   float floor_cmp;  // float_below(-eta * minpix): v > floor_cmp as in FP64
   int positivity;
 };
+gv_status objective_setup(Problem& P);
 gv_status chi2_launch(Problem& P, float* d_img, int flag_opt, bool store_res,
                       const XtSource* xs = nullptr, double* term_out = nullptr,
                       uint32_t zero_terms = 0u);

@@ -35,10 +35,8 @@ namespace gv {
 
 namespace {
 
-// values per thread of the FFT passes: the separate row and column kernels
-// (up to 4096 values over 256 threads) and the fused small-image kernel (up
-// to 512 values over 256 threads)
-constexpr int kVptLarge = 16;
+// values per thread of the fused small-image kernel's FFT passes (up to 512
+// values over 256 threads)
 constexpr int kVptSmall = 2;
 
 // evaluateXt at one pixel (k_eval_xt's arithmetic): xt = pcom + x xicom,
@@ -153,90 +151,95 @@ __device__ __forceinline__ void row_task(const StageParams& sp, const float* __r
   for (int j = threadIdx.x; j < n; j += blockDim.x) out[j] = buf[fpad(j)];
 }
 
-// Pass 1 for row i = blockIdx.x and every channel: the row's pixels (or the
-// line search's xt) are read once -- each thread loads all of its pixels
-// before it stores anything, so the loads are in flight together -- clipped
-// (the clip written back once), then per channel staged as
-// I_nu * A * fg_scale (* GCF) in shared memory and FFT'd into the channel's
-// grid.  The same arithmetic per pixel and channel as row_task.  VPT: the
-// row's values per thread (n / blockDim.x, at least 2).
-template <int VPT>
-__global__ void __launch_bounds__(256, VPT >= 16 ? 3 : 4)
+// (nu / nu_0)^alpha out of line: most images have flat spectra and skip it
+__device__ __noinline__ float spectral_power(float nudiv, float al) { return powf(nudiv, al); }
+
+// Pass 1 for a row and every channel: the row's pixels (or the line search's
+// xt) are read once, clipped (the clip written back once), then per channel
+// staged as I_nu * A * fg_scale (* GCF) in registers and transformed, and the
+// columns that some visibility reads go to the channel's grid.  The same
+// arithmetic per pixel and channel as row_task; the beam comes from a table of
+// the same values (134 MB read at 2048^2 x 8 channels, where its exponentials
+// were a quarter of the pass).  n / 8 threads a row, kLines rows a block.
+// 2048^2 x 8 channels: ROWS_BEFORE -> ROWS_AFTER us, bound by instruction issue and the
+// table's bytes.
+template <int LG>
+struct RowPass {
+  static constexpr int kThreads = (1 << LG) / 8;  // per line
+  static constexpr int kLines = kThreads >= 64 ? 1 : (kThreads == 2 ? 16 : 64 / kThreads);
+  static constexpr int kBlock = kThreads * kLines;
+};
+
+template <int LG>
+__global__ void __launch_bounds__(RowPass<LG>::kBlock,
+                                  RowPass<LG>::kBlock > 384 ? 1 : 768 / RowPass<LG>::kBlock)
     k_rows_fft(StageParams sp, const float* __restrict__ chfreq, int C, float* __restrict__ img,
-               const uint8_t* __restrict__ mask, const float2* __restrict__ tw,
+               const uint8_t* __restrict__ mask, const float* __restrict__ atten,
+               const uint8_t* __restrict__ need, const float2* __restrict__ tw,
                float2* __restrict__ grid) {
-  extern __shared__ float2 buf[];  // the row (fft_span(n)), its clipped I_nu0, alpha, beam radius
-  const int n = sp.N, i = blockIdx.x;
-  float* s_i0 = reinterpret_cast<float*>(buf + fft_span(n));
-  float* s_al = s_i0 + n;
-  float* s_arc = s_al + n;
-  const float by = __ldg(sp.beam_y + i);
+  constexpr int n = 1 << LG, T = RowPass<LG>::kThreads, L = RowPass<LG>::kLines;
+  constexpr int64_t MN = (int64_t)n * n;
+  __shared__ float2 line[L * fft_span(n)];
+  const int j = threadIdx.x % T, i = blockIdx.x * L + threadIdx.x / T;
+  float2* buf = line + (threadIdx.x / T) * fft_span(n);
   const ClipRule cr{sp.eta > 0.0f ? 0.0f : (float)(-1.0 * sp.eta * sp.minpix), sp.threshold,
                     sp.flag_opt};
   const bool from_xt = sp.xs.pcom != nullptr;
   const float x = from_xt ? __ldcg(sp.xs.x_dev) : 0.0f;
-  {
-    float i0[VPT], al[VPT];
+  const int64_t q0 = (int64_t)n * i + j;
+  float i0[8], al[8];
+  bool flat = true;
+  unsigned cols = 0;  // bit e: column j + e T is read by the degridding
 #pragma unroll
-    for (int k = 0; k < VPT; k++) {
-      const int j = threadIdx.x + k * blockDim.x;
-      if (j < n) {
-        const int64_t q = (int64_t)n * i + j;
-        if (from_xt) {
-          xt_pixel(sp.xs, x, sp.MN, q, i0[k], al[k]);
-        } else {
-          i0[k] = img[q];
-          al[k] = img[sp.MN + q];
-        }
-      }
+  for (int e = 0; e < 8; e++) {
+    const int64_t q = q0 + e * T;
+    if (from_xt) {
+      xt_pixel(sp.xs, x, MN, q, i0[e], al[e]);
+    } else {
+      i0[e] = img[q];
+      al[e] = img[MN + q];
     }
+    cols |= need[j + e * T] ? 1u << e : 0u;
+  }
 #pragma unroll
-    for (int k = 0; k < VPT; k++) {
-      const int j = threadIdx.x + k * blockDim.x;
-      if (j < n) {
-        // clip2IWNoise, src/functions.cu:2694-2719 (mutates the image: only
-        // the pixels it changes are written back)
-        const int64_t q = (int64_t)n * i + j;
-        const float i0_in = i0[k], al_in = al[k];
-        clip_pixel(mask[q], cr, i0[k], al[k]);
-        if (sp.write_clip && from_xt) {
-          img[q] = i0[k];
-          img[sp.MN + q] = al[k];
-        } else if (sp.write_clip) {
-          if (i0[k] != i0_in) img[q] = i0[k];
-          if (al[k] != al_in) img[sp.MN + q] = al[k];
-        }
-        s_i0[j] = i0[k];  // read back by this thread only
-        s_al[j] = al[k];
-        s_arc[j] = beam_arc(__ldg(sp.beam_x + j), by);
-      }
+  for (int e = 0; e < 8; e++) {
+    // clip2IWNoise, src/functions.cu:2694-2719 (mutates the image: only the
+    // pixels it changes are written back)
+    const int64_t q = q0 + e * T;
+    const float i0_in = i0[e], al_in = al[e];
+    clip_pixel(mask[q], cr, i0[e], al[e]);
+    if (sp.write_clip && from_xt) {
+      img[q] = i0[e];
+      img[MN + q] = al[e];
+    } else if (sp.write_clip) {
+      if (i0[e] != i0_in) img[q] = i0[e];
+      if (al[e] != al_in) img[MN + q] = al[e];
     }
+    flat = flat && al[e] == 0.0f;
   }
   const float floor_inu = -1.0f * sp.eta * sp.minpix;
   for (int c = 0; c < C; c++) {
-    const float freq = chfreq[c];
-    const float nudiv = freq / sp.nu_0;
-    const BeamAt beam = beam_at(freq, sp.D, sp.pbf, sp.pbcut, sp.pb);
-    // unrolled by two only: the transcendental functions of many pixels at
-    // once would raise the register count and lower the occupancy
-#pragma unroll 2
-    for (int k = 0; k < VPT; k++) {
-      const int j = threadIdx.x + k * blockDim.x;
-      if (j < n) {
-        buf[fpad(j)] = make_float2(
-            stage_value(sp, s_i0[j], s_al[j], s_arc[j], beam, nudiv, floor_inu, (int64_t)n * i + j),
-            0.0f);
-      }
-    }
-    __syncthreads();
-    smem_fft<VPT>(buf, sp.log2n, 1, tw);
-    float2* out = grid + (int64_t)c * sp.MN + (int64_t)n * i;
+    const float nudiv = chfreq[c] / sp.nu_0;
+    const float* at = atten + c * MN + q0;
+    float2 v[8];
 #pragma unroll
-    for (int k = 0; k < VPT; k++) {
-      const int j = threadIdx.x + k * blockDim.x;
-      if (j < n) out[j] = buf[fpad(j)];
+    for (int e = 0; e < 8; e++) v[e].x = __ldg(at + e * T);
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      // calculateInu, apply_beam2I, fg_scale, apply_GCF as in stage_value
+      float inu = i0[e];
+      if (!flat && al[e] != 0.0f) inu *= spectral_power(nudiv, al[e]);
+      if (inu < floor_inu) inu = floor_inu;
+      float s = inu * v[e].x * sp.fg_scale;
+      if (sp.gcf) s *= sp.gcf[q0 + e * T];
+      v[e] = make_float2(s, 0.0f);
     }
-    __syncthreads();
+    if (c > 0) __syncthreads();  // the last channel's line has been read
+    fft8<LG>(v, buf, j, tw);
+    float2* out = grid + c * MN + q0;
+#pragma unroll
+    for (int e = 0; e < 8; e++)
+      if (cols >> e & 1u) out[e * T] = v[e];
   }
 }
 
@@ -289,16 +292,43 @@ __device__ __forceinline__ void col_task(int N, int log2n, int cb, const float* 
   }
 }
 
-// Pass 2: column FFTs of `cb` adjacent columns, then phase_rotate (512
-// threads, at most 64 registers each, so two blocks share an SM).
-__global__ void __launch_bounds__(512, 2) k_cols_fft(int N, int log2n, int64_t MN, int cb,
-                                                     const float* __restrict__ rot_u,
-                                                     const float* __restrict__ rot_v,
-                                                     const float2* __restrict__ tw_g,
-                                                     float2* __restrict__ grid) {
-  extern __shared__ float2 sm[];
-  col_task<false, kVptLarge>(N, log2n, cb, rot_u, rot_v, tw_g, grid + (int64_t)blockIdx.y * MN, sm,
-                  blockIdx.x * cb);
+// Pass 2: column FFTs of kCols adjacent columns, then phase_rotate, for the
+// blocks of columns that some visibility reads (`blocks`: a problem's
+// visibilities cover 49 of 256 columns at 256^2 and 306 of 2048 at 2048^2);
+// of their results the rows that are read go out.  2048^2 x 8 channels:
+// COLS_BEFORE -> COLS_AFTER us.
+template <int LG>
+struct ColPass {
+  static constexpr int kThreads = (1 << LG) / 8;  // per column
+  static constexpr int kCols = kThreads >= 512 ? 1 : (kThreads >= 256 ? 2 : (kThreads >= 64 ? 4 : 2));
+  // a column's line: a multiple of 16 and 16 / kCols more, so the lanes of a
+  // half warp, kCols columns wide, read distinct banks
+  static constexpr int kStride = (fft_span(1 << LG) + 15) / 16 * 16 + 16 / kCols;
+};
+
+template <int LG>
+__global__ void __launch_bounds__(ColPass<LG>::kThreads * ColPass<LG>::kCols)
+    k_cols_fft(const int* __restrict__ blocks, const uint8_t* __restrict__ need_row,
+               const float* __restrict__ rot_u, const float* __restrict__ rot_v,
+               const float2* __restrict__ tw, float2* __restrict__ grid) {
+  constexpr int n = 1 << LG, T = ColPass<LG>::kThreads, CB = ColPass<LG>::kCols;
+  __shared__ float2 line[CB * ColPass<LG>::kStride];
+  const int cc = threadIdx.x % CB, j = threadIdx.x / CB;
+  const int col = blocks[blockIdx.x] * CB + cc;
+  float2* G = grid + (int64_t)blockIdx.y * n * n + (int64_t)j * n + col;
+  float2 v[8];
+  unsigned rows = 0;
+#pragma unroll
+  for (int e = 0; e < 8; e++) {
+    v[e] = G[(int64_t)e * T * n];
+    rows |= need_row[j + e * T] ? 1u << e : 0u;
+  }
+  fft8<LG>(v, line + cc * ColPass<LG>::kStride, j, tw);
+  const float u = __ldg(rot_u + col);
+#pragma unroll
+  for (int e = 0; e < 8; e++)
+    if (rows >> e & 1u)
+      G[(int64_t)e * T * n] = phase_rotated(v[e], u, __ldg(rot_v + j + e * T));
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -884,18 +914,6 @@ __global__ void __launch_bounds__(256, 2) k_objective_fused_batch(FusedBatch<Img
 
 }  // namespace
 
-// Columns per block of the column pass: 8192 / n (8K complex values, 64 KB
-// of shared memory: at 2048^2 four columns, so each row segment a warp reads
-// is one 32-byte sector), fewer while the launch would have under two blocks
-// per SM (small images: 256^2 runs 256 one-column blocks).
-static int cols_per_block(int n, int channels, int num_sms) {
-  int cb = 8192 / n;
-  if (cb < 1) cb = 1;
-  if (cb > 16) cb = 16;
-  while (cb > 1 && (int64_t)(n / cb) * channels < 2 * (int64_t)num_sms) cb >>= 1;
-  return cb;
-}
-
 static StageParams stage_params(const Problem& P, int flag_opt, int write_clip,
                                 const XtSource* xs) {
   StageParams sp;
@@ -925,36 +943,37 @@ static StageParams stage_params(const Problem& P, int flag_opt, int write_clip,
   return sp;
 }
 
+template <int LG>
+static gv_status grids_of_side(Problem& P, const StageParams& sp, float* d_img) {
+  const int C = (int)P.chans.size();
+  using R = RowPass<LG>;
+  k_rows_fft<LG><<<P.N / R::kLines, R::kBlock, 0, P.stream>>>(
+      sp, P.d_chfreq, C, d_img, P.d_mask, P.d_atten, P.d_need, P.d_tw8, P.d_grid);
+  GV_LAUNCH("k_rows_fft");
+  using K = ColPass<LG>;
+  if (P.col_blocks == 0) return GV_OK;  // no visibility on the grid
+  k_cols_fft<LG><<<dim3(P.col_blocks, C), K::kThreads * K::kCols, 0, P.stream>>>(
+      P.d_col_blocks, P.d_need + P.N, P.d_rot_u, P.d_rot_v, P.d_tw8, P.d_grid);
+  GV_LAUNCH("k_cols_fft");
+  return GV_OK;
+}
+
 // Model grids of all channels for image d_img (clip written back when
 // write_clip).
 gv_status model_grids_launch(Problem& P, float* d_img, int flag_opt, int write_clip,
                              const XtSource* xs = nullptr) {
-  const int n = P.N, C = (int)P.chans.size();
   const StageParams sp = stage_params(P, flag_opt, write_clip, xs);
-  // row pass: one block of 256 threads per row, n / 256 values a thread;
-  // shared memory: the row's values, its clipped I_nu0 and alpha, beam radii
-  const size_t sm1 = sizeof(float2) * fft_span(n) + 3 * sizeof(float) * n;
-  auto rows = [&](auto kern) -> gv_status {
-    if (sm1 > 48 * 1024)
-      GV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-    kern<<<n, 256, sm1, P.stream>>>(sp, P.d_chfreq, C, d_img, P.d_mask, P.d_twiddle, P.d_grid);
-    GV_LAUNCH("k_rows_fft");
-    return GV_OK;
-  };
-  gv_status s = n <= 512 ? rows(k_rows_fft<2>)
-                         : (n <= 1024 ? rows(k_rows_fft<4>)
-                                      : (n <= 2048 ? rows(k_rows_fft<8>) : rows(k_rows_fft<16>)));
-  if (s != GV_OK) return s;
-  // column pass: cb columns per block, 16 values a thread
-  const int cb = cols_per_block(n, C, P.num_sms);
-  const int threads2 = cb * n > 4096 ? 512 : 256;
-  const size_t sm2 = sizeof(float2) * (size_t)cb * fft_stride(n);
-  if (sm2 > 48 * 1024)
-    GV_CUDA(cudaFuncSetAttribute(k_cols_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
-  k_cols_fft<<<dim3(n / cb, C), threads2, sm2, P.stream>>>(n, P.log2n, sp.MN, cb, P.d_rot_u,
-                                                           P.d_rot_v, P.d_twiddle, P.d_grid);
-  GV_LAUNCH("k_cols_fft");
-  return GV_OK;
+  switch (P.log2n) {
+    case 4: return grids_of_side<4>(P, sp, d_img);
+    case 5: return grids_of_side<5>(P, sp, d_img);
+    case 6: return grids_of_side<6>(P, sp, d_img);
+    case 7: return grids_of_side<7>(P, sp, d_img);
+    case 8: return grids_of_side<8>(P, sp, d_img);
+    case 9: return grids_of_side<9>(P, sp, d_img);
+    case 10: return grids_of_side<10>(P, sp, d_img);
+    case 11: return grids_of_side<11>(P, sp, d_img);
+    default: return grids_of_side<12>(P, sp, d_img);
+  }
 }
 
 // k_degrid's blocks per channel
@@ -979,6 +998,99 @@ static DegridArgs degrid_args(Problem& P, bool store_res, double* term_out, uint
 static int prior_blocks(const Problem& P) {
   const int64_t MN = (int64_t)P.M * P.N;
   return (int)std::min<int64_t>((MN + 255) / 256, P.part_stride);
+}
+
+// Tables of the row and column passes: the channels' beams, the columns and
+// rows of the model grid that the visibilities read, the twiddles by pass.
+__global__ void __launch_bounds__(256) k_attenuation(int N, const float* __restrict__ chfreq,
+                                                     const float* __restrict__ beam_x,
+                                                     const float* __restrict__ beam_y, float D,
+                                                     float pbf, float cutoff, int pb,
+                                                     float* __restrict__ atten) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, MN = (int64_t)N * N;
+  if (q >= MN) return;
+  const int i = (int)(q / N), j = (int)(q - (int64_t)i * N);
+  const BeamAt beam = beam_at(chfreq[blockIdx.y], D, pbf, cutoff, pb);
+  atten[blockIdx.y * MN + q] = attenuation_at(beam_arc(beam_x[j], beam_y[i]), beam);
+}
+
+__global__ void __launch_bounds__(256) k_needed(int N, const ChanRange* __restrict__ ranges,
+                                                const float4* __restrict__ deg,
+                                                uint32_t* __restrict__ need) {
+  const ChanRange rg = ranges[blockIdx.y];
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < rg.ngrid;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t cell = __float_as_uint(deg[rg.off + k].x);
+    const int i1 = cell & 0xffff, j1 = cell >> 16;
+    const int at[4] = {i1, (i1 + 1) & (N - 1), N + j1, N + ((j1 + 1) & (N - 1))};
+    for (int t : at)
+      if (!(__ldcg(need + (t >> 5)) >> (t & 31) & 1u)) atomicOr(need + (t >> 5), 1u << (t & 31));
+  }
+}
+
+gv_status objective_setup(Problem& P) {
+  const int N = P.N, C = (int)P.chans.size();
+  const int64_t MN = (int64_t)N * N;
+  GV_CUDA(cudaMalloc(&P.d_atten, sizeof(float) * MN * C));
+  k_attenuation<<<dim3((unsigned)((MN + 255) / 256), C), 256, 0, P.stream>>>(
+      N, P.d_chfreq, P.d_beam_x, P.d_beam_y, P.D, P.pbf, P.pbcut, P.pb, P.d_atten);
+  GV_LAUNCH("k_attenuation");
+  // bits of the needed columns, then rows, then the same as bytes
+  const int words = 2 * N / 32;
+  uint32_t* bits = nullptr;
+  GV_CUDA(cudaMalloc(&bits, sizeof(uint32_t) * words));
+  std::vector<uint32_t> h(words);
+  const auto mark = [&]() -> gv_status {
+    GV_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * words, P.stream));
+    k_needed<<<dim3(2 * P.num_sms, C), 256, 0, P.stream>>>(N, P.d_ranges, P.d_deg, bits);
+    GV_LAUNCH("k_needed");
+    GV_CUDA(cudaMemcpyAsync(h.data(), bits, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost,
+                            P.stream));
+    GV_CUDA(cudaStreamSynchronize(P.stream));
+    return GV_OK;
+  };
+  const gv_status s = mark();
+  cudaFree(bits);
+  if (s != GV_OK) return s;
+  std::vector<uint8_t> need(2 * N);
+  for (int t = 0; t < 2 * N; t++) need[t] = h[t >> 5] >> (t & 31) & 1u;
+  const int cb = P.log2n >= 12 ? ColPass<12>::kCols
+                 : P.log2n == 11 ? ColPass<11>::kCols
+                 : P.log2n >= 9 ? ColPass<9>::kCols : ColPass<8>::kCols;
+  static_assert(ColPass<10>::kCols == ColPass<9>::kCols && ColPass<4>::kCols == ColPass<8>::kCols &&
+                    ColPass<5>::kCols == ColPass<8>::kCols &&
+                    ColPass<6>::kCols == ColPass<8>::kCols &&
+                    ColPass<7>::kCols == ColPass<8>::kCols,
+                "columns per block");
+  std::vector<int> blocks;
+  for (int b = 0; b < N / cb; b++)
+    for (int c = 0; c < cb; c++)
+      if (need[b * cb + c]) {
+        blocks.push_back(b);
+        break;
+      }
+  P.col_blocks = (int)blocks.size();
+  std::vector<float2> tw;
+  for (int l = 3; l < P.log2n; l += 3) {
+    const int R = 1 << fft8_radix(P.log2n, l);
+    for (int r = 1; r < R; r++)
+      for (int k = 0; k < (1 << l); k++) {
+        // the m-th n-th root as in d_twiddle
+        const int m = r * (k << (P.log2n - l - fft8_radix(P.log2n, l)));
+        const double a = 2.0 * kPiD * m / N;
+        tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+      }
+  }
+  GV_CUDA(cudaMalloc(&P.d_need, need.size()));
+  GV_CUDA(cudaMalloc(&P.d_tw8, sizeof(float2) * tw.size()));
+  GV_CUDA(cudaMemcpy(P.d_need, need.data(), need.size(), cudaMemcpyHostToDevice));
+  GV_CUDA(cudaMemcpy(P.d_tw8, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
+  if (P.col_blocks) {
+    GV_CUDA(cudaMalloc(&P.d_col_blocks, sizeof(int) * blocks.size()));
+    GV_CUDA(cudaMemcpy(P.d_col_blocks, blocks.data(), sizeof(int) * blocks.size(),
+                       cudaMemcpyHostToDevice));
+  }
+  return GV_OK;
 }
 
 // Whether the objective of P runs as k_objective_fused: images up to

@@ -290,6 +290,10 @@ void free_problem(Problem& P) {
   cudaFree(P.d_rho);
   cudaFree(P.d_grid);
   cudaFree(P.d_twiddle);
+  cudaFree(P.d_tw8);
+  cudaFree(P.d_atten);
+  cudaFree(P.d_need);
+  cudaFree(P.d_col_blocks);
   cudaFree(P.d_beam_x);  // one allocation with d_beam_y, d_rot_u, d_rot_v
   cudaFree(P.d_epi);
   cudaFree(P.d_part);
@@ -713,6 +717,7 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     GV_CUDA(cudaMemcpy(P.d_kc_one, k1.data(), sizeof(int64_t) * 2 * C, cudaMemcpyHostToDevice));
   }
   GV_TRY(nu_finish(P));
+  GV_TRY(objective_setup(P));
   GV_CUDA(cudaMalloc(&P.d_flags, sizeof(uint32_t) * kNumFlags));
   GV_CUDA(cudaMemsetAsync(P.d_flags, 0, sizeof(uint32_t) * kNumFlags, st));
   {
