@@ -331,7 +331,9 @@ class Problem:
         Returns the n values of f."""
         import torch
         n = len(imgs)
-        for i in range(n):
+        # the images of one tensor are alike: looked at once
+        stacked = isinstance(imgs, torch.Tensor) and n > 0
+        for i in range(1 if stacked else n):
             t = imgs[i]
             if (t.dtype != torch.float32 or not t.is_cuda or not t.is_contiguous()
                     or t.numel() != 2 * self.N * self.M):
@@ -339,7 +341,11 @@ class Problem:
                                  f"2 x {self.N} x {self.M} values")
             if t.device != self.device:
                 raise ValueError(f"image {i} is on {t.device}, the problem on {self.device}")
-        ptrs = (C.c_void_p * n)(*[imgs[i].data_ptr() for i in range(n)])
+        if stacked:
+            p0, step = imgs.data_ptr(), imgs.stride(0) * 4
+            ptrs = (C.c_void_p * n)(*[p0 + i * step for i in range(n)])
+        else:
+            ptrs = (C.c_void_p * n)(*[imgs[i].data_ptr() for i in range(n)])
         f = (C.c_double * max(n, 1))()
         check(lib().gv_objective_many(self.h, ptrs, n, flag_opt, f, None))
         return [f[i] for i in range(n)]

@@ -41,7 +41,6 @@ struct gv_batch {
   cudaStream_t cap = nullptr;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
-  uint32_t* h_err = nullptr;  // pinned, one word per problem
   std::vector<BatchGraph> graphs;
   uint64_t clock = 0;
   int use_graph = 1;
@@ -59,19 +58,16 @@ void destroy(gv_batch* b) {
   for (auto e : b->join) cudaEventDestroy(e);
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->cap) cudaStreamDestroy(b->cap);
-  if (b->h_err) cudaFreeHost(b->h_err);
   delete b;
 }
 
 // one problem's evaluation, its scalars and error word copied to the host
-gv_status branch(gv::Problem& P, float* img, float* xi, int iter, int flag, uint32_t* h_err,
+gv_status branch(gv::Problem& P, float* img, float* xi, int iter, int flag,
                  bool objective = true) {
-  if (objective) GV_TRY(gv::objective_launch(P, img, flag, true));
-  GV_TRY(gv::gradient_launch(P, img, xi, iter, flag));
-  GV_CUDA(cudaMemcpyAsync(P.h_scal, P.d_scal, sizeof(double) * gv::kNumScal,
-                          cudaMemcpyDeviceToHost, P.stream));
-  GV_CUDA(cudaMemcpyAsync(h_err, P.d_flags + gv::kFlagErr, sizeof(uint32_t),
-                          cudaMemcpyDeviceToHost, P.stream));
+  if (objective) GV_TRY(gv::objective_launch(P, img, flag, true, xi, iter));
+  GV_TRY(gv::gradient_launch(P, img, xi, iter, flag, objective));
+  GV_TRY(gv::side_joined(P));
+  GV_CUDA(cudaMemcpyAsync(P.h_scal, P.d_scal, gv::kScalBytes, cudaMemcpyDeviceToHost, P.stream));
   return GV_OK;
 }
 
@@ -142,7 +138,6 @@ gv_status gv_batch_create(gv_problem* const* problems, int32_t n, gv_batch** out
     if (e != cudaSuccess) break;
     b->join.push_back(ev);
   }
-  if (e == cudaSuccess) e = cudaMallocHost(&b->h_err, sizeof(uint32_t) * n);
   if (const char* env = std::getenv("GV_BATCH_FUSED")) b->fused_objective = std::atoi(env) != 0;
   if (e != cudaSuccess) {
     destroy(b);
@@ -201,7 +196,7 @@ gv_status gv_batch_evaluate(gv_batch* b, float* const* d_imgs, float* const* d_x
     for (int i = 0; i < n && s == GV_OK; i++) {
       gv::Problem& P = gv::problem_of(b->probs[i]);
       P.stream = b->streams[i];
-      s = branch(P, img[i], xi[i], iter, flag_opt, b->h_err + i);
+      s = branch(P, img[i], xi[i], iter, flag_opt);
     }
     for (int i = 0; i < n; i++) cudaStreamSynchronize(b->streams[i]);
     restore();
@@ -234,7 +229,8 @@ gv_status gv_batch_evaluate(gv_batch* b, float* const* d_imgs, float* const* d_x
         P.stream = b->streams[i];
         e = cudaStreamWaitEvent(b->streams[i], b->fork, 0);
         if (e == cudaSuccess)
-          s = branch(P, img[i], xi[i], iter, flag_opt, b->h_err + i, tables == nullptr);
+          s = branch(P, img[i], xi[i], iter, flag_opt, tables == nullptr);
+        P.side_open = 0;
         if (s == GV_OK && e == cudaSuccess) e = cudaEventRecord(b->join[i], b->streams[i]);
         if (s == GV_OK && e == cudaSuccess) e = cudaStreamWaitEvent(b->cap, b->join[i], 0);
       }
@@ -283,11 +279,12 @@ gv_status gv_batch_evaluate(gv_batch* b, float* const* d_imgs, float* const* d_x
     for (size_t t = 0; t < P.terms.size(); t++)
       tot += (double)P.terms[t].lambda * P.h_scal[gv::kSlotTerm0 + t];
     f[i] = tot;
-    if (b->h_err[i] != 0 && st == GV_OK) {
+    const uint32_t err = reinterpret_cast<const uint32_t*>(P.h_scal + gv::kNumScal)[gv::kFlagErr];
+    if (err != 0 && st == GV_OK) {
       cudaMemsetAsync(P.d_flags + gv::kFlagErr, 0, sizeof(uint32_t), P.stream);
       gv::set_error("a kernel of batch problem " + std::to_string(i) +
                     " gave up on a bounded wait (device error word " +
-                    std::to_string(b->h_err[i]) + ")");
+                    std::to_string(err) + ")");
       st = GV_ERR_DEVICE;
     }
   }

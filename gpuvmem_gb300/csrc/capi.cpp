@@ -209,7 +209,8 @@ gv_status gv_objective(gv_problem* p, float* d_img, int32_t flag_opt, double* f,
   gv_status s = P.use_graphs ? gv::eval_graph(P, d_img, nullptr, 0, flag_opt, 1, true)
                              : gv::objective_launch(P, d_img, flag_opt, true);
   if (s != GV_OK) return s;
-  s = gv::fetch_scalars(P, gv::kSlotTerm0 + (int)P.terms.size());
+  s = P.use_graphs ? gv::finish_graph(P)
+                   : gv::fetch_scalars(P, gv::kSlotTerm0 + (int)P.terms.size());
   if (s != GV_OK) return s;
   double tot = 0.0;
   for (size_t t = 0; t < P.terms.size(); t++) {
@@ -238,7 +239,13 @@ gv_status gv_objective_many(gv_problem* p, const float* const* d_imgs, int32_t c
     P.h_many_cap = need;
   }
   const size_t bytes = sizeof(float) * 2 * (size_t)P.M * (size_t)P.N;
-  for (int32_t i = 0; i < count; i++) {
+  const int32_t batch = gv::many_at_once(P);
+  if (batch > 1) {
+    for (int32_t i = 0; i < count; i += batch)
+      GV_TRY(gv::objective_many_launch(P, d_imgs + i, std::min(batch, count - i), flag_opt,
+                                       P.h_many + (size_t)i * nt));
+  }
+  for (int32_t i = 0; batch <= 1 && i < count; i++) {
     GV_CUDA(cudaMemcpyAsync(P.d_tmp, d_imgs[i], bytes, cudaMemcpyDeviceToDevice, P.stream));
     gv_status s = P.use_graphs ? gv::eval_graph(P, P.d_tmp, nullptr, 0, flag_opt, 1, false)
                                : gv::objective_launch(P, P.d_tmp, flag_opt, false);
@@ -266,7 +273,7 @@ gv_status gv_gradient(gv_problem* p, float* d_img, float* d_xi, int32_t iter, in
   gv_status s = P.use_graphs ? gv::eval_graph(P, d_img, d_xi, iter, flag_opt, 2, false)
                              : gv::gradient_launch(P, d_img, d_xi, iter, flag_opt);
   if (s != GV_OK) return s;
-  return gv::check_device_error(P);
+  return P.use_graphs ? gv::finish_graph(P) : gv::check_device_error(P);
 }
 
 gv_status gv_evaluate(gv_problem* p, float* d_img, float* d_xi, int32_t iter, int32_t flag_opt,
@@ -279,8 +286,8 @@ gv_status gv_evaluate(gv_problem* p, float* d_img, float* d_xi, int32_t iter, in
   }
   gv_status s = gv::eval_graph(P, d_img, d_xi, iter, flag_opt, 3, true);
   if (s != GV_OK) return s;
-  s = gv::fetch_scalars(P, gv::kSlotTerm0 + (int)P.terms.size());
-  if (s != GV_OK) return s;
+  s = gv::finish_graph(P);
+  if (s != GV_OK && s != GV_ERR_DEVICE) return s;
   double tot = 0.0;
   for (size_t t = 0; t < P.terms.size(); t++) {
     const double v = P.h_scal[gv::kSlotTerm0 + t];
@@ -288,7 +295,7 @@ gv_status gv_evaluate(gv_problem* p, float* d_img, float* d_xi, int32_t iter, in
     tot += (double)P.terms[t].lambda * v;
   }
   *f = tot;
-  return gv::check_device_error(P);
+  return s;
 }
 
 gv_status gv_problem_set_graphs(gv_problem* p, int32_t enable) {

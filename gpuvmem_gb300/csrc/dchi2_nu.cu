@@ -766,7 +766,7 @@ gv_status spread(const SpreadArgs& a, int warps, cudaStream_t st) {
 }
 
 template <int LG>
-gv_status transforms(const Problem& P, const RowArgs& ra, const ColArgs& ca) {
+gv_status transforms(Problem& P, const RowArgs& ra, const ColArgs& ca) {
   constexpr int L = RowShape<LG>::kLines;
   const size_t smem = sizeof(float2) * L * span16(1 << LG);
   if (smem > 48 * 1024)
@@ -774,6 +774,7 @@ gv_status transforms(const Problem& P, const RowArgs& ra, const ColArgs& ca) {
                                  (int)smem));
   k_nu_rows<LG><<<(ra.lines + L - 1) / L, RowShape<LG>::kThreads * L, smem, P.stream>>>(ra);
   GV_LAUNCH("k_nu_rows");
+  GV_TRY(side_joined(P));  // the priors' gradient is where the sums are added
   using S = ColShape<LG>;
   if (S::kSmem > 48 * 1024)
     GV_CUDA(cudaFuncSetAttribute(k_nu_cols<LG>, cudaFuncAttributeMaxDynamicSharedMemorySize,

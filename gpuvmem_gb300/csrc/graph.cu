@@ -52,9 +52,17 @@ void graph_cache_free(Problem& P) {
   P.graphs = nullptr;
 }
 
+gv_status finish_graph(Problem& P) {
+  GV_CUDA(cudaStreamSynchronize(P.stream));
+  const uint32_t* flags = reinterpret_cast<const uint32_t*>(P.h_scal + kNumScal);
+  return flags[kFlagErr] ? check_device_error(P) : GV_OK;
+}
+
 // what: 1 = objective, 2 = gradient, 3 = objective + gradient; store: the
 // objective keeps its weighted residuals for the next gradient.  The objective's
-// scalars land in d_scal as with objective_launch; the caller fetches them.
+// scalars land in d_scal as with objective_launch and, with the flags, in
+// h_scal: one copy inside the graph, and finish_graph waits once, where a
+// fetch of the scalars and one of the error word took two copies and waits.
 gv_status eval_graph(Problem& P, float* d_img, float* d_xi, int iter, int flag_opt, int what,
                      bool store) {
   GraphCache& c = cache(P);
@@ -77,8 +85,18 @@ gv_status eval_graph(Problem& P, float* d_img, float* d_xi, int iter, int flag_o
       P.stream = saved;
       return cuda_fail(e, "cudaStreamBeginCapture");
     }
-    gv_status s = (what & 1) ? objective_launch(P, d_img, flag_opt, store) : GV_OK;
-    if (s == GV_OK && (what & 2)) s = gradient_launch(P, d_img, d_xi, iter, flag_opt);
+    const bool both = what == 3;
+    gv_status s = (what & 1) ? objective_launch(P, d_img, flag_opt, store,
+                                                both ? d_xi : nullptr, iter)
+                             : GV_OK;
+    if (s == GV_OK && (what & 2)) s = gradient_launch(P, d_img, d_xi, iter, flag_opt, both);
+    if (s == GV_OK) s = side_joined(P);
+    if (s == GV_OK) {
+      const cudaError_t ce =
+          cudaMemcpyAsync(P.h_scal, P.d_scal, kScalBytes, cudaMemcpyDeviceToHost, P.stream);
+      if (ce != cudaSuccess) s = cuda_fail(ce, "eval_graph");
+    }
+    P.side_open = 0;
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(c.cap, &graph);
     P.stream = saved;

@@ -125,10 +125,15 @@ struct Problem {
   float* d_rot_v = nullptr;      // [M] phase_rotate's v of each row
   double* d_part = nullptr;      // reduction partials
   int part_stride = 0;           // partials per channel / term
-  double* d_scal = nullptr;      // [kNumScal]
-  double* h_scal = nullptr;      // pinned mirror
+  double* d_scal = nullptr;      // [kNumScal], then d_flags: one copy fetches both
+  double* h_scal = nullptr;      // pinned mirror of d_scal and d_flags
   double* h_many = nullptr;      // pinned term values of gv_objective_many
   size_t h_many_cap = 0;         // doubles h_many holds
+  void* d_many = nullptr;        // gv_objective_many's grids and sums (allocated on demand)
+  int many_cap = 0;              // images d_many holds
+  cudaStream_t side = nullptr;   // second branch of captured evaluations (priors)
+  cudaEvent_t side_fork = nullptr, side_join = nullptr;
+  int side_open = 0;             // work on `side` that P.stream has not joined yet
   float* d_tmp = nullptr;        // [2*MN] scratch image (dchi2 channel etc.)
   float* d_opt = nullptr;        // optimiser workspace (allocated on demand)
   size_t opt_bytes = 0;
@@ -359,7 +364,22 @@ gv_status chi2_launch(Problem& P, float* d_img, int flag_opt, bool store_res,
                       uint32_t zero_terms = 0u);
 gv_status prior_value_launch(Problem& P, int t, const float* d_img, int slot);
 gv_status prior_grad_launch(Problem& P, int t, const float* d_img, float* d_dphi);
-gv_status objective_launch(Problem& P, float* d_img, int flag_opt, bool store_res);
+// The gradient of the active priors of a gradient call (iter, flag_opt),
+// written over both planes of d_xi.
+gv_status prior_grads_launch(Problem& P, const float* d_img, float* d_xi, int iter, int flag_opt);
+// With xi (its gradient call's iter in xi_iter) the objective also leaves the
+// priors' gradient in it, beside the Chi2 kernels where P.stream is being
+// captured; gradient_launch then adds DChi2 (priors_done).
+gv_status objective_launch(Problem& P, float* d_img, int flag_opt, bool store_res,
+                           float* d_xi = nullptr, int xi_iter = 0);
+// The work on P.side joins P.stream (before anything that reads its results).
+gv_status side_joined(Problem& P);
+// Objective values of `count` images at once, term values [image][nterms] to
+// d_many's end (many_values); GV_ERR_UNSUPPORTED where the terms or the sizes
+// want one image at a time.
+int many_at_once(const Problem& P);
+gv_status objective_many_launch(Problem& P, const float* const* d_imgs, int count, int flag_opt,
+                                double* h_values);
 // Batches: the objectives of several problems (store_res on) in one
 // cooperative launch.  batch_objective_args writes a problem's arguments
 // (batch_arg_bytes() bytes, host) and its task counts per phase, or returns
@@ -378,6 +398,11 @@ gv_status ls_objective_launch(Problem& P, float* d_xt, int flag_opt, const XtSou
                               cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, LsState* ls,
                               cudaGraphConditionalHandle cond, bool* stepped);
 gv_status fetch_scalars(Problem& P, int n);
+// Bytes of d_scal and d_flags.
+constexpr size_t kScalBytes = sizeof(double) * kNumScal + sizeof(uint32_t) * kNumFlags;
+// After eval_graph, which copies d_scal and d_flags to h_scal: waits, and turns
+// a device error word into a status.
+gv_status finish_graph(Problem& P);
 
 // Device-wide sort / scan / run-length primitives (sortscan.cu).  Scratch
 // sizes first, then the call; nothing is allocated inside.
@@ -396,7 +421,8 @@ gv_status run_length_encode(void* scratch, size_t bytes, const uint32_t* keys, i
                             int* nruns, cudaStream_t st);
 gv_status dchi2_launch(Problem& P, const float* d_img, int flag_opt, float* d_result);
 gv_status dchi2_channel_launch(Problem& P, int c, float* d_out);
-gv_status gradient_launch(Problem& P, float* d_img, float* d_xi, int iter, int flag_opt);
+gv_status gradient_launch(Problem& P, float* d_img, float* d_xi, int iter, int flag_opt,
+                          bool priors_done = false);
 gv_status dirty_launch(Problem& P, float* d_out, bool psf = false);
 
 // dchi2 engines

@@ -163,6 +163,13 @@ __device__ __noinline__ float spectral_power(float nudiv, float al) { return pow
 // were a quarter of the pass).  n / 8 threads a row, kLines rows a block.
 // 2048^2 x 8 channels: 348 -> 129 us, bound by instruction issue and the
 // table's bytes.
+// Images evaluated in one launch (blockIdx.y of the row pass): one, or the
+// candidates of gv_objective_many.
+constexpr int kMaxImages = 16;
+struct Images {
+  float* p[kMaxImages];
+};
+
 template <int LG>
 struct RowPass {
   static constexpr int kThreads = (1 << LG) / 8;  // per line
@@ -173,7 +180,7 @@ struct RowPass {
 template <int LG>
 __global__ void __launch_bounds__(RowPass<LG>::kBlock,
                                   RowPass<LG>::kBlock > 384 ? 1 : 768 / RowPass<LG>::kBlock)
-    k_rows_fft(StageParams sp, const float* __restrict__ chfreq, int C, float* __restrict__ img,
+    k_rows_fft(StageParams sp, const float* __restrict__ chfreq, int C, Images imgs,
                const uint8_t* __restrict__ mask, const float* __restrict__ atten,
                const uint8_t* __restrict__ need, const float2* __restrict__ tw,
                float2* __restrict__ grid) {
@@ -181,6 +188,8 @@ __global__ void __launch_bounds__(RowPass<LG>::kBlock,
   constexpr int64_t MN = (int64_t)n * n;
   __shared__ float2 line[L * fft_span(n)];
   const int j = threadIdx.x % T, i = blockIdx.x * L + threadIdx.x / T;
+  float* __restrict__ img = imgs.p[blockIdx.y];
+  grid += (int64_t)blockIdx.y * C * MN;
   float2* buf = line + (threadIdx.x / T) * fft_span(n);
   const ClipRule cr{sp.eta > 0.0f ? 0.0f : (float)(-1.0 * sp.eta * sp.minpix), sp.threshold,
                     sp.flag_opt};
@@ -383,7 +392,7 @@ struct DegridArgs {
   int store;
   double* __restrict__ part;
   int part_stride;
-  uint32_t* __restrict__ cmax;
+  uint32_t* __restrict__ cmax;  // scale of the GEMM's operands, or null (not used)
   uint32_t* __restrict__ done;
   const int64_t* __restrict__ nvis;
   int normalize;
@@ -473,10 +482,10 @@ __device__ __forceinline__ void degrid_task(const DegridArgs& a, int b, int nb, 
     if (a.store) {
       const float2 cv = make_float2(d.w * rr, d.w * ri);
       __stcs(a.cvr + rg.off + k, cv);
-      mx = fmaxf(mx, fmaxf(fabsf(cv.x), fabsf(cv.y)));
+      if (a.cmax) mx = fmaxf(mx, fmaxf(fabsf(cv.x), fabsf(cv.y)));
     }
   }
-  if (a.store) {
+  if (a.store && a.cmax) {
     for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, s));
     if ((threadIdx.x & 31) == 0 && mx > 0.0f) atomicMax(a.cmax, __float_as_uint(mx));
   }
@@ -680,13 +689,16 @@ struct PriorSet {
 
 // Values of n prior terms, block b of nb of term t: the block's partial, and
 // the last of the nb * n blocks to finish sums each term's partials in a
-// fixed order.
-template <class Img>
+// fixed order.  part_off, out_off: where the partials and values of this image
+// lie from those of the set; place(I) puts the image in.
+template <class Img, class Place>
 __device__ __forceinline__ void prior_task(const PriorSet<Img>& ps, const uint8_t* __restrict__ mask,
-                                           uint32_t* __restrict__ done, int b, int nb, int t) {
+                                           uint32_t* __restrict__ done, int b, int nb, int t,
+                                           int64_t part_off, int64_t out_off, Place&& place) {
   const PriorParams& pp = ps.pp[t];
   Img I = ps.img[t];
   I.bind();
+  place(I);
   CompSum acc;
   for (int64_t q = b * (int64_t)blockDim.x + threadIdx.x; q < pp.MN;
        q += (int64_t)nb * blockDim.x) {
@@ -695,15 +707,21 @@ __device__ __forceinline__ void prior_task(const PriorSet<Img>& ps, const uint8_
     acc.add(prior_pixel(pp, I, i, j));
   }
   const double bsum = block_sum(acc.value());
-  if (threadIdx.x == 0) ps.part[t][b] = bsum;
+  if (threadIdx.x == 0) ps.part[t][part_off + b] = bsum;
   if (last_block_done(done, nb * ps.n)) {
     for (int u = 0; u < ps.n; u++) {
       double v = 0.0;
-      for (int k = threadIdx.x; k < nb; k += blockDim.x) v += __ldcg(ps.part[u] + k);
+      for (int k = threadIdx.x; k < nb; k += blockDim.x) v += __ldcg(ps.part[u] + part_off + k);
       v = block_sum(v);
-      if (threadIdx.x == 0) *ps.out[u] = v;
+      if (threadIdx.x == 0) ps.out[u][out_off] = v;
     }
   }
+}
+
+template <class Img>
+__device__ __forceinline__ void prior_task(const PriorSet<Img>& ps, const uint8_t* __restrict__ mask,
+                                           uint32_t* __restrict__ done, int b, int nb, int t) {
+  prior_task(ps, mask, done, b, nb, t, 0, 0, [](Img&) {});
 }
 
 // Values of n prior terms (blockIdx.y = term).
@@ -723,6 +741,35 @@ __global__ void __launch_bounds__(256) k_prior_grad(PriorParams pp, const float*
     const int i = (int)(q / pp.N), j = (int)(q - (int64_t)i * pp.N);
     const float g = prior_grad_pixel(pp, I, i, j) * pp.lambda;
     dphi[q] += g;  // AddToDPhi, src/functions.cu:3890
+  }
+}
+
+// The gradients of several priors in one pass, written over both planes of
+// dphi (Chi2's gradient is added to it afterwards): a launch for all priors
+// where each had its own, over a buffer cleared before.
+struct PriorGrads {
+  int n;
+  PriorParams pp[kMaxTerms];
+  int from[kMaxTerms], to[kMaxTerms];  // image planes
+};
+
+__global__ void __launch_bounds__(256) k_prior_grads(PriorGrads pg, int64_t MN, int N,
+                                                     const float* __restrict__ img,
+                                                     const uint8_t* __restrict__ mask,
+                                                     float* __restrict__ dphi) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < MN;
+       q += (int64_t)gridDim.x * blockDim.x) {
+    float g[2] = {0.0f, 0.0f};
+    if (mask[q] & kMaskIn) {
+      const int i = (int)(q / N), j = (int)(q - (int64_t)i * N);
+      for (int t = 0; t < pg.n; t++) {
+        const float v = prior_grad_pixel(pg.pp[t], img + MN * pg.from[t], i, j) * pg.pp[t].lambda;
+        if (pg.to[t]) g[1] += v;
+        else g[0] += v;
+      }
+    }
+    dphi[q] = g[0];
+    dphi[MN + q] = g[1];
   }
 }
 
@@ -874,7 +921,8 @@ __global__ void __launch_bounds__(256, 2) k_objective_fused_batch(FusedBatch<Img
   const int* offB = fb.off + fb.np + 1;
   const int* offC = fb.off + 2 * (fb.np + 1);
   if (fb.clear_cmax && blockIdx.x == 0)
-    for (int p = threadIdx.x; p < fb.np; p += blockDim.x) *fb.args[p].da.cmax = 0u;
+    for (int p = threadIdx.x; p < fb.np; p += blockDim.x)
+      if (fb.args[p].da.cmax) *fb.args[p].da.cmax = 0u;
   // A: rows of every channel of every problem, then its prior-value tasks
   for (int t = blockIdx.x; t < __ldg(offA + fb.np); t += gridDim.x) {
     const int p = task_problem(offA, fb.np, t);
@@ -943,37 +991,87 @@ static StageParams stage_params(const Problem& P, int flag_opt, int write_clip,
   return sp;
 }
 
+// The row (pass 1) or column pass (pass 2) of `count` images into `grid`.
 template <int LG>
-static gv_status grids_of_side(Problem& P, const StageParams& sp, float* d_img) {
+static gv_status pass_of_side(Problem& P, int pass, const StageParams& sp, const Images& imgs,
+                              int count, float2* grid) {
   const int C = (int)P.chans.size();
   using R = RowPass<LG>;
-  k_rows_fft<LG><<<P.N / R::kLines, R::kBlock, 0, P.stream>>>(
-      sp, P.d_chfreq, C, d_img, P.d_mask, P.d_atten, P.d_need, P.d_tw8, P.d_grid);
-  GV_LAUNCH("k_rows_fft");
   using K = ColPass<LG>;
-  if (P.col_blocks == 0) return GV_OK;  // no visibility on the grid
-  k_cols_fft<LG><<<dim3(P.col_blocks, C), K::kThreads * K::kCols, 0, P.stream>>>(
-      P.d_col_blocks, P.d_need + P.N, P.d_rot_u, P.d_rot_v, P.d_tw8, P.d_grid);
-  GV_LAUNCH("k_cols_fft");
+  if (pass == 1) {
+    k_rows_fft<LG><<<dim3(P.N / R::kLines, count), R::kBlock, 0, P.stream>>>(
+        sp, P.d_chfreq, C, imgs, P.d_mask, P.d_atten, P.d_need, P.d_tw8, grid);
+    GV_LAUNCH("k_rows_fft");
+  } else if (P.col_blocks > 0) {  // else no visibility lies on the grid
+    k_cols_fft<LG><<<dim3(P.col_blocks, C * count), K::kThreads * K::kCols, 0, P.stream>>>(
+        P.d_col_blocks, P.d_need + P.N, P.d_rot_u, P.d_rot_v, P.d_tw8, grid);
+    GV_LAUNCH("k_cols_fft");
+  }
   return GV_OK;
 }
 
-// Model grids of all channels for image d_img (clip written back when
-// write_clip).
-gv_status model_grids_launch(Problem& P, float* d_img, int flag_opt, int write_clip,
-                             const XtSource* xs = nullptr) {
-  const StageParams sp = stage_params(P, flag_opt, write_clip, xs);
+static gv_status grid_pass(Problem& P, int pass, const StageParams& sp, const Images& imgs,
+                           int count, float2* grid) {
   switch (P.log2n) {
-    case 4: return grids_of_side<4>(P, sp, d_img);
-    case 5: return grids_of_side<5>(P, sp, d_img);
-    case 6: return grids_of_side<6>(P, sp, d_img);
-    case 7: return grids_of_side<7>(P, sp, d_img);
-    case 8: return grids_of_side<8>(P, sp, d_img);
-    case 9: return grids_of_side<9>(P, sp, d_img);
-    case 10: return grids_of_side<10>(P, sp, d_img);
-    case 11: return grids_of_side<11>(P, sp, d_img);
-    default: return grids_of_side<12>(P, sp, d_img);
+    case 4: return pass_of_side<4>(P, pass, sp, imgs, count, grid);
+    case 5: return pass_of_side<5>(P, pass, sp, imgs, count, grid);
+    case 6: return pass_of_side<6>(P, pass, sp, imgs, count, grid);
+    case 7: return pass_of_side<7>(P, pass, sp, imgs, count, grid);
+    case 8: return pass_of_side<8>(P, pass, sp, imgs, count, grid);
+    case 9: return pass_of_side<9>(P, pass, sp, imgs, count, grid);
+    case 10: return pass_of_side<10>(P, pass, sp, imgs, count, grid);
+    case 11: return pass_of_side<11>(P, pass, sp, imgs, count, grid);
+    default: return pass_of_side<12>(P, pass, sp, imgs, count, grid);
   }
+}
+
+// Model grids of all channels for image d_img (clip written back when
+// write_clip); `between` runs after the row pass, which leaves the clipped
+// image, with the rest of the objective still to come.
+template <class F>
+static gv_status model_grids_launch(Problem& P, float* d_img, int flag_opt, int write_clip,
+                                    const XtSource* xs, F&& between) {
+  const StageParams sp = stage_params(P, flag_opt, write_clip, xs);
+  Images one{};
+  one.p[0] = d_img;
+  GV_TRY(grid_pass(P, 1, sp, one, 1, P.d_grid));
+  GV_TRY(between());
+  return grid_pass(P, 2, sp, one, 1, P.d_grid);
+}
+
+// ---- several images at once (gv_objective_many) ------------------------------
+// The passes of one small image leave the GPU nearly idle (256^2, one channel:
+// 43 us an image, one after another with a copy and a graph each); the
+// candidates are independent, so each pass takes them all in one launch:
+// 511 -> 122 us for 12.  Per image the blocks, and so the sums, are those of a
+// single evaluation.
+struct ManyArgs {
+  DegridArgs da;           // of the first image
+  PriorSet<ClipImage> ps;  // likewise (the image pointers from imgs)
+  Images imgs;
+  const uint8_t* mask;
+  int64_t grid_stride, part_stride;  // per image: float2 of grid, doubles of partials
+  int nterms;
+  double* values;     // [image][nterms]
+  uint32_t* done;     // [image][2]
+};
+
+__global__ void __launch_bounds__(256) k_degrid_many(ManyArgs m) {
+  const int im = blockIdx.z;
+  DegridArgs a = m.da;
+  a.grid += im * m.grid_stride;
+  a.part += im * m.part_stride;
+  a.done = m.done + 2 * im;
+  a.chi2_out = a.term_out = m.values + im * m.nterms;
+  a.term_slots = a.term_out;
+  degrid_task<false>(a, blockIdx.x, gridDim.x, blockIdx.y, gridDim.y);
+}
+
+__global__ void __launch_bounds__(256) k_prior_values_many(ManyArgs m) {
+  const int im = blockIdx.z;
+  const float* img = m.imgs.p[im];
+  prior_task(m.ps, m.mask, m.done + 2 * im + 1, blockIdx.x, gridDim.x, blockIdx.y,
+             im * m.part_stride, im * m.nterms, [img](ClipImage& I) { I.p = img; });
 }
 
 // k_degrid's blocks per channel
@@ -989,7 +1087,8 @@ static int degrid_blocks(const Problem& P) {
 static DegridArgs degrid_args(Problem& P, bool store_res, double* term_out, uint32_t zero_terms) {
   const int64_t MN = (int64_t)P.M * P.N;
   return DegridArgs{P.N, MN, P.d_ranges, P.d_deg, P.d_vo, P.d_grid, P.d_cvr,
-                    store_res ? 1 : 0, P.d_part, P.part_stride, P.d_flags + kFlagCvrMax,
+                    store_res ? 1 : 0, P.d_part, P.part_stride,
+                    P.nu ? nullptr : P.d_flags + kFlagCvrMax,
                     P.d_flags + kFlagDegridDone, P.d_chnvis, P.normalize,
                     P.d_scal + kSlotChi2, term_out, zero_terms, P.d_scal + kSlotTerm0,
                     nullptr, nullptr, 0};
@@ -1165,7 +1264,8 @@ static gv_status fused_launch(Problem& P, float* d_img, int flag_opt, bool store
     const int tasks = std::max(n * C + f.nb_prior * kMaxTerms, f.nb_deg * C);
     blocks = std::max(1, std::min(P.num_sms * std::min(occ, 2), tasks));
   }
-  if (store_res) GV_CUDA(cudaMemsetAsync(P.d_flags + kFlagCvrMax, 0, sizeof(uint32_t), P.stream));
+  if (store_res && !P.nu)
+    GV_CUDA(cudaMemsetAsync(P.d_flags + kFlagCvrMax, 0, sizeof(uint32_t), P.stream));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(256);
@@ -1181,21 +1281,30 @@ static gv_status fused_launch(Problem& P, float* d_img, int flag_opt, bool store
   return GV_OK;
 }
 
+template <class F>
+static gv_status chi2_passes(Problem& P, float* d_img, int flag_opt, bool store_res,
+                             const XtSource* xs, double* term_out, uint32_t zero_terms,
+                             F&& between) {
+  GV_TRY(model_grids_launch(P, d_img, flag_opt, 1, xs, between));
+  const int C = (int)P.chans.size();
+  const int nb = degrid_blocks(P);
+  if (store_res && !P.nu)
+    GV_CUDA(cudaMemsetAsync(P.d_flags + kFlagCvrMax, 0, sizeof(uint32_t), P.stream));
+  const DegridArgs da = degrid_args(P, store_res, term_out, zero_terms);
+  k_degrid<<<dim3(nb, C), P.degrid_threads, 0, P.stream>>>(da);
+  GV_LAUNCH("k_degrid");
+  return GV_OK;
+}
+
+static gv_status nothing() { return GV_OK; }
+
 gv_status chi2_launch(Problem& P, float* d_img, int flag_opt, bool store_res,
                       const XtSource* xs, double* term_out, uint32_t zero_terms) {
   if (fused_ok(P)) {
     PriorSet<PlainImage> none{};
     return fused_launch(P, d_img, flag_opt, store_res, xs, term_out, zero_terms, none);
   }
-  gv_status s = model_grids_launch(P, d_img, flag_opt, 1, xs);
-  if (s != GV_OK) return s;
-  const int C = (int)P.chans.size();
-  const int nb = degrid_blocks(P);
-  if (store_res) GV_CUDA(cudaMemsetAsync(P.d_flags + kFlagCvrMax, 0, sizeof(uint32_t), P.stream));
-  const DegridArgs da = degrid_args(P, store_res, term_out, zero_terms);
-  k_degrid<<<dim3(nb, C), P.degrid_threads, 0, P.stream>>>(da);
-  GV_LAUNCH("k_degrid");
-  return GV_OK;
+  return chi2_passes(P, d_img, flag_opt, store_res, xs, term_out, zero_terms, nothing);
 }
 
 static PriorParams prior_params(const Problem& P, const Term& t) {
@@ -1226,7 +1335,7 @@ static gv_status prior_values_launch(Problem& P, cudaStream_t st, const PriorSet
 
 // Values of the terms ts[0..n) of image d_img, into d_scal[slot[k]].
 static gv_status prior_values_plain(Problem& P, const int* ts, const int* slots, int n,
-                                    const float* d_img) {
+                                    const float* d_img, cudaStream_t st) {
   PriorSet<PlainImage> ps{};
   ps.n = n;
   const int64_t MN = (int64_t)P.M * P.N;
@@ -1237,11 +1346,11 @@ static gv_status prior_values_plain(Problem& P, const int* ts, const int* slots,
     ps.part[k] = prior_part(P, ts[k]);
     ps.out[k] = P.d_scal + slots[k];
   }
-  return prior_values_launch(P, P.stream, ps);
+  return prior_values_launch(P, st, ps);
 }
 
 gv_status prior_value_launch(Problem& P, int t, const float* d_img, int slot) {
-  return prior_values_plain(P, &t, &slot, 1, d_img);
+  return prior_values_plain(P, &t, &slot, 1, d_img, P.stream);
 }
 
 gv_status prior_grad_launch(Problem& P, int t, const float* d_img, float* d_dphi) {
@@ -1337,46 +1446,161 @@ gv_status batch_objective_launch(int np, const void* d_args, const int* d_off, i
   return GV_OK;
 }
 
+// Images per launch of gv_objective_many: 16, fewer where their grids would
+// take more than 1 GB, 1 (one after another) where one image fills the GPU or
+// the terms are not Chi2 and priors of its clipped image.
+int many_at_once(const Problem& P) {
+  if (P.terms.empty() || P.terms[0].kind != GV_FI_CHI2 || fused_ok(P)) return 1;
+  const int64_t grid = (int64_t)P.M * P.N * (int64_t)P.chans.size();
+  return (int)std::min<int64_t>(kMaxImages, (int64_t(1) << 27) / grid);
+}
+
+gv_status objective_many_launch(Problem& P, const float* const* d_imgs, int count, int flag_opt,
+                                double* h_values) {
+  const int C = (int)P.chans.size(), nt = (int)P.terms.size();
+  const int64_t MN = (int64_t)P.M * P.N;
+  const size_t grid_b = sizeof(float2) * (size_t)MN * C;
+  const size_t part_n = (size_t)P.part_stride * (C + kMaxTerms);
+  const size_t each = grid_b + sizeof(double) * (part_n + kMaxTerms) + 2 * sizeof(uint32_t);
+  if (P.many_cap < count) {
+    GV_CUDA(cudaStreamSynchronize(P.stream));
+    cudaFree(P.d_many);
+    P.d_many = nullptr;
+    P.many_cap = 0;
+    GV_CUDA(cudaMalloc(&P.d_many, each * count));
+    P.many_cap = count;
+    GV_CUDA(cudaMemsetAsync(P.d_many, 0, each * count, P.stream));
+  }
+  const int cap = P.many_cap;
+  float2* grid = static_cast<float2*>(P.d_many);
+  double* part = reinterpret_cast<double*>(grid + (size_t)MN * C * cap);
+  double* values = part + part_n * cap;
+  uint32_t* done = reinterpret_cast<uint32_t*>(values + (size_t)kMaxTerms * cap);
+  ManyArgs m{};
+  for (int k = 0; k < count; k++) m.imgs.p[k] = const_cast<float*>(d_imgs[k]);
+  const StageParams sp = stage_params(P, flag_opt, 0, nullptr);
+  GV_TRY(grid_pass(P, 1, sp, m.imgs, count, grid));
+  GV_TRY(grid_pass(P, 2, sp, m.imgs, count, grid));
+  const uint32_t zero = gated_terms(P);
+  m.da = degrid_args(P, false, nullptr, zero);
+  m.da.grid = grid;
+  m.da.part = part;
+  m.mask = P.d_mask;
+  m.grid_stride = MN * C;
+  m.part_stride = (int64_t)part_n;
+  m.nterms = nt;
+  m.values = values;
+  m.done = done;
+  k_degrid_many<<<dim3(degrid_blocks(P), C, count), P.degrid_threads, 0, P.stream>>>(m);
+  GV_LAUNCH("k_degrid_many");
+  clip_prior_set(P, nullptr, flag_opt, zero, &m.ps);
+  if (m.ps.n > 0) {
+    for (int u = 0, t = 1; t < nt; t++) {
+      if (zero & (1u << t)) continue;
+      m.ps.part[u] = part + (size_t)P.part_stride * (C + t);
+      m.ps.out[u] = values + t;
+      u++;
+    }
+    k_prior_values_many<<<dim3(prior_blocks(P), m.ps.n, count), 256, 0, P.stream>>>(m);
+    GV_LAUNCH("k_prior_values_many");
+  }
+  GV_CUDA(cudaMemcpyAsync(h_values, values, sizeof(double) * nt * count, cudaMemcpyDeviceToHost,
+                          P.stream));
+  return GV_OK;
+}
+
+gv_status prior_grads_launch(Problem& P, const float* d_img, float* d_xi, int iter,
+                             int flag_opt) {
+  const int64_t MN = (int64_t)P.M * P.N;
+  const cudaStream_t st = P.side_open ? P.side : P.stream;
+  PriorGrads pg{};
+  for (const Term& tm : P.terms) {
+    if (tm.kind == GV_FI_CHI2 || !(iter > 0) || tm.lambda == 0.0f ||
+        (flag_opt % 2) != tm.image_index)
+      continue;
+    pg.pp[pg.n] = prior_params(P, tm);
+    pg.from[pg.n] = tm.image_index;
+    // TVariation::addToDphi adds into plane 0 whatever imageToAdd is
+    // (src/totalvariation.cu:48)
+    pg.to[pg.n] = tm.kind == GV_FI_TV ? 0 : tm.image_to_add;
+    pg.n++;
+  }
+  if (pg.n == 0) {
+    GV_CUDA(cudaMemsetAsync(d_xi, 0, sizeof(float) * 2 * MN, st));
+    return GV_OK;
+  }
+  const int nb = (int)std::min<int64_t>((MN + 255) / 256, 8 * P.num_sms);
+  k_prior_grads<<<nb, 256, 0, st>>>(pg, MN, P.N, d_img, P.d_mask, d_xi);
+  GV_LAUNCH("k_prior_grads");
+  return GV_OK;
+}
+
+// While P.stream is being captured the priors take a branch of their own from
+// here on (P.side), which side_joined ends; otherwise they stay on P.stream.
+static gv_status side_opened(Problem& P) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  GV_CUDA(cudaStreamIsCapturing(P.stream, &cs));
+  if (cs != cudaStreamCaptureStatusActive) return GV_OK;
+  if (!P.side) GV_CUDA(cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking));
+  if (!P.side_fork) GV_CUDA(cudaEventCreateWithFlags(&P.side_fork, cudaEventDisableTiming));
+  if (!P.side_join) GV_CUDA(cudaEventCreateWithFlags(&P.side_join, cudaEventDisableTiming));
+  GV_CUDA(cudaEventRecord(P.side_fork, P.stream));
+  GV_CUDA(cudaStreamWaitEvent(P.side, P.side_fork, 0));
+  P.side_open = 1;
+  return GV_OK;
+}
+
+gv_status side_joined(Problem& P) {
+  if (!P.side_open) return GV_OK;
+  P.side_open = 0;
+  GV_CUDA(cudaEventRecord(P.side_join, P.side));
+  GV_CUDA(cudaStreamWaitEvent(P.stream, P.side_join, 0));
+  return GV_OK;
+}
+
 // ObjectiveFunction::calcFunction; values land in d_scal[kSlotTerm0 + t].
-// Terms are evaluated in list order; consecutive active priors share one
-// launch.
-gv_status objective_launch(Problem& P, float* d_img, int flag_opt, bool store_res) {
+// Chi2, the first term, clips the image in its row pass; the active priors'
+// values (one launch) and, with d_xi, their gradient need nothing more of it
+// and run beside its other passes in a captured evaluation.
+gv_status objective_launch(Problem& P, float* d_img, int flag_opt, bool store_res, float* d_xi,
+                           int xi_iter) {
   // Chi2 also writes its term slot and zeroes the slots of the priors the
   // iteration gating leaves out
   bool has_chi2 = false;
   uint32_t zero = 0u;
-  for (size_t t = 0; t < P.terms.size(); t++) {
-    if (P.terms[t].kind == GV_FI_CHI2) has_chi2 = true;
-    else if (!(P.iteration > 0 && P.terms[t].lambda != 0.0f)) zero |= 1u << t;
-  }
-  PriorSet<ClipImage> ps{};
-  if (fused_ok(P) && clip_prior_set(P, d_img, flag_opt, zero, &ps))
-    return fused_launch(P, d_img, flag_opt, store_res, nullptr, P.d_scal + kSlotTerm0, zero, ps);
   int run[kMaxTerms], slots[kMaxTerms], nrun = 0;
-  auto flush = [&]() -> gv_status {
-    const int n = nrun;
-    nrun = 0;
-    return n ? prior_values_plain(P, run, slots, n, d_img) : GV_OK;
-  };
   for (size_t t = 0; t < P.terms.size(); t++) {
-    const Term& tm = P.terms[t];
-    gv_status s = GV_OK;
-    if (tm.kind == GV_FI_CHI2) {
-      s = flush();
-      if (s == GV_OK) s = chi2_launch(P, d_img, flag_opt, store_res, nullptr, P.d_scal + kSlotTerm0 + t, zero);
-    } else if (has_chi2 && (zero & (1u << t))) {
-      // zeroed by the chi2 kernel
-    } else if (P.iteration > 0 && tm.lambda != 0.0f) {
-      if (nrun == kMaxTerms) s = flush();
-      run[nrun] = (int)t;
-      slots[nrun] = kSlotTerm0 + (int)t;
-      nrun++;
+    if (P.terms[t].kind == GV_FI_CHI2) {
+      has_chi2 = true;
+    } else if (!(P.iteration > 0 && P.terms[t].lambda != 0.0f)) {
+      zero |= 1u << t;
+      if (!has_chi2)
+        GV_CUDA(cudaMemsetAsync(P.d_scal + kSlotTerm0 + t, 0, sizeof(double), P.stream));
     } else {
-      GV_CUDA(cudaMemsetAsync(P.d_scal + kSlotTerm0 + t, 0, sizeof(double), P.stream));
+      run[nrun] = (int)t;
+      slots[nrun++] = kSlotTerm0 + (int)t;
     }
-    if (s != GV_OK) return s;
   }
-  return flush();
+  auto priors = [&]() -> gv_status {
+    if (nrun > 0)
+      GV_TRY(prior_values_plain(P, run, slots, nrun, d_img, P.side_open ? P.side : P.stream));
+    return d_xi ? prior_grads_launch(P, d_img, d_xi, xi_iter, flag_opt) : GV_OK;
+  };
+  if (!has_chi2) return priors();
+  PriorSet<ClipImage> ps{};
+  if (fused_ok(P) && clip_prior_set(P, d_img, flag_opt, zero, &ps)) {
+    GV_TRY(fused_launch(P, d_img, flag_opt, store_res, nullptr, P.d_scal + kSlotTerm0, zero, ps));
+    return d_xi ? prior_grads_launch(P, d_img, d_xi, xi_iter, flag_opt) : GV_OK;
+  }
+  const bool branch = nrun > 0 || d_xi;
+  GV_TRY(chi2_passes(P, d_img, flag_opt, store_res, nullptr, P.d_scal + kSlotTerm0, zero,
+                     [&]() -> gv_status {
+                       if (branch) GV_TRY(side_opened(P));
+                       return P.side_open ? priors() : GV_OK;
+                     }));
+  if (!P.side_open) return priors();
+  // with d_xi the gradient still to come joins the branch
+  return d_xi ? GV_OK : side_joined(P);
 }
 
 // One objective evaluation of the line search at the controller's point:
@@ -1442,7 +1666,7 @@ gv_status ls_objective_launch(Problem& P, float* d_xt, int flag_opt, const XtSou
     if (ps.n > 0) GV_CUDA(cudaStreamWaitEvent(P.stream, join, 0));
     return GV_OK;
   }
-  gv_status s = model_grids_launch(P, d_xt, flag_opt, 1, &xs);
+  gv_status s = model_grids_launch(P, d_xt, flag_opt, 1, &xs, nothing);
   if (s != GV_OK) return s;
   // the degridding waits for the prior values too: its last block adds the
   // terms up and steps the search
@@ -1482,6 +1706,7 @@ gv_status fetch_scalars(Problem& P, int n) {
 gv_status dchi2_run(Problem& P, const float* d_img, int flag_opt, float* d_result,
                     int only_channel, int mode) {
   if (P.nu) return dchi2_nu(P, d_img, flag_opt, d_result, only_channel, mode);
+  GV_TRY(side_joined(P));  // the priors' gradient is in d_result
   if (P.engine == 2) return dchi2_tc(P, d_img, flag_opt, d_result, only_channel, mode);
   return dchi2_direct(P, d_img, flag_opt, d_result, only_channel, mode);
 }
@@ -1502,21 +1727,16 @@ gv_status dirty_launch(Problem& P, float* d_out, bool psf) {
 }
 
 // ObjectiveFunction::calcGradient (include/classes/objectivefunction.cuh:28-57)
-gv_status gradient_launch(Problem& P, float* d_img, float* d_xi, int iter, int flag_opt) {
-  const int64_t MN = (int64_t)P.M * P.N;
+gv_status gradient_launch(Problem& P, float* d_img, float* d_xi, int iter, int flag_opt,
+                          bool priors_done) {
   P.iteration = iter;  // setIteration(iter) on every Fi
-  GV_CUDA(cudaMemsetAsync(d_xi, 0, sizeof(float) * 2 * MN, P.stream));
-  for (size_t t = 0; t < P.terms.size(); t++) {
-    const Term& tm = P.terms[t];
-    gv_status s = GV_OK;
-    if (tm.kind == GV_FI_CHI2) {
-      s = dchi2_launch(P, d_img, flag_opt, d_xi);
-    } else if (iter > 0 && tm.lambda != 0.0f && (flag_opt % 2) == tm.image_index) {
-      s = prior_grad_launch(P, (int)t, d_img, d_xi);
-    }
-    if (s != GV_OK) return s;
+  if (!priors_done) {
+    GV_TRY(side_opened(P));
+    GV_TRY(prior_grads_launch(P, d_img, d_xi, iter, flag_opt));
   }
-  return GV_OK;
+  if (!P.terms.empty() && P.terms[0].kind == GV_FI_CHI2)
+    GV_TRY(dchi2_launch(P, d_img, flag_opt, d_xi));
+  return side_joined(P);
 }
 
 }  // namespace gv

@@ -519,7 +519,7 @@ class Solver {
     gv_status s = P_.use_graphs ? eval_graph(P_, img, nullptr, 0, o_.flag, 1, store_res)
                                 : objective_launch(P_, img, o_.flag, store_res);
     if (s != GV_OK) return s;
-    s = fetch_scalars(P_, kSlotTerm0 + (int)P_.terms.size());
+    s = P_.use_graphs ? finish_graph(P_) : fetch_scalars(P_, kSlotTerm0 + (int)P_.terms.size());
     if (s != GV_OK) return s;
     double f = 0.0;
     for (size_t t = 0; t < P_.terms.size(); t++)

@@ -307,10 +307,13 @@ void free_problem(Problem& P) {
   cudaFree(P.d_kc_off);
   cudaFree(P.d_kc_one);
   cudaFree(P.d_E);
-  cudaFree(P.d_flags);
   cudaFree(P.tc_partial);
   if (P.h_scal) cudaFreeHost(P.h_scal);
   if (P.h_many) cudaFreeHost(P.h_many);
+  cudaFree(P.d_many);
+  if (P.side) cudaStreamDestroy(P.side);
+  if (P.side_fork) cudaEventDestroy(P.side_fork);
+  if (P.side_join) cudaEventDestroy(P.side_join);
   nu_free(P);
   graph_cache_free(P);
   ls_cache_free(P);
@@ -718,8 +721,9 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
   }
   GV_TRY(nu_finish(P));
   GV_TRY(objective_setup(P));
-  GV_CUDA(cudaMalloc(&P.d_flags, sizeof(uint32_t) * kNumFlags));
-  GV_CUDA(cudaMemsetAsync(P.d_flags, 0, sizeof(uint32_t) * kNumFlags, st));
+  GV_CUDA(cudaMalloc(&P.d_scal, kScalBytes));
+  P.d_flags = reinterpret_cast<uint32_t*>(P.d_scal + kNumScal);
+  GV_CUDA(cudaMemsetAsync(P.d_scal, 0, kScalBytes, st));
   {
     const unsigned gb = (unsigned)((V + 255) / 256);
     k_dirty_max<<<gb, 256, 0, st>>>(V, P.d_deg, P.d_vo, P.d_flags + kFlagDirtyMax,
@@ -763,9 +767,7 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
   P.part_stride = 4 * P.num_sms;
   const int nslots = C + kMaxTerms + 8;
   GV_CUDA(cudaMalloc(&P.d_part, sizeof(double) * (size_t)P.part_stride * nslots));
-  GV_CUDA(cudaMalloc(&P.d_scal, sizeof(double) * kNumScal));
-  GV_CUDA(cudaMemsetAsync(P.d_scal, 0, sizeof(double) * kNumScal, st));
-  GV_CUDA(cudaMallocHost(&P.h_scal, sizeof(double) * kNumScal));
+  GV_CUDA(cudaMallocHost(&P.h_scal, kScalBytes));
   GV_CUDA(cudaMalloc(&P.d_tmp, sizeof(float) * 2 * MN));
   // DChi2's direct-sum engine: the tensor-core GEMM where it covers the
   // geometry, else the SIMT kernel.  With dchi2_engine 0 the non-uniform FFT
