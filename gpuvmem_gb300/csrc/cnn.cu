@@ -55,8 +55,50 @@ struct GemmLayout {
   static constexpr uint32_t kSmem = 1024 + 2 * kStage;
 };
 
+// byte offset of the 16-byte chunk holding columns 8*g..8*g+7 of row r in a
+// K-major 128B-swizzled tile (64 columns a row, atoms of 8 rows 1024 B apart)
+__device__ __forceinline__ uint32_t kmajor_off(int r, int g) {
+  return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((g ^ (r & 7)) << 4));
+}
+
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  return make_uint4(bf16x2(v[0], v[1]), bf16x2(v[2], v[3]), bf16x2(v[4], v[5]),
+                    bf16x2(v[6], v[7]));
+}
+
+// Eight neighbours of an image row, columns x + dx .. x + dx + 7 (|dx| <= 1,
+// zero outside the row of W): `p` points at column x, 16-byte aligned, x and
+// W multiples of 8.  Two 16-byte loads and at most one more, where eight
+// loads one by one set the pace of the GEMMs' staging.
+__device__ __forceinline__ void row8(const float* __restrict__ p, int x, int dx, int W,
+                                     float (&v)[8]) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+  const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  if (dx == 0) {
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else if (dx > 0) {
+    v[0] = a.y; v[1] = a.z; v[2] = a.w; v[3] = b.x;
+    v[4] = b.y; v[5] = b.z; v[6] = b.w;
+    v[7] = x + 8 < W ? __ldg(p + 8) : 0.0f;
+  } else {
+    v[0] = x > 0 ? __ldg(p - 1) : 0.0f;
+    v[1] = a.x; v[2] = a.y; v[3] = a.z; v[4] = a.w;
+    v[5] = b.x; v[6] = b.y; v[7] = b.z;
+  }
+}
+
 // D[m][n] = sum_k A[m][k] B[k][n] over this CTA's K range; op.a(m,k),
 // op.b(k,n) fetch FP32 operands, op.store(m, n, v, split) writes a result.
+// How the tiles are staged (op.fast: aligned tensors whose rows are multiples
+// of eight pixels; otherwise, and at ragged edges, element by element):
+//   Op::kPixelRows  the rows of A are pixels (forward, data gradient): a
+//                   thread keeps its eight pixels and takes the taps' offsets
+//                   from a table made once per chunk; B is the weights, which
+//                   op.packed holds as ready BF16 tile images;
+//   otherwise       the columns of A and B are pixels (weight gradient): both
+//                   tiles K-major, so that eight neighbours of a row are one
+//                   16-byte store; a thread keeps its row's channel and tap.
 template <class Op, int BN>
 __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int K, int klen,
                                                        uint32_t* err) {
@@ -67,11 +109,21 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
   __shared__ uint64_t bar[2];
   __shared__ uint32_t tslot;
   __shared__ int s_abort;
+  __shared__ int4 tab[2][kBK];  // the chunk's taps, or its groups of eight pixels
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
   const int kbeg = blockIdx.z * klen;
   const int kend = min(K, kbeg + klen);
   const int nch = kend > kbeg ? (kend - kbeg + kBK - 1) / kBK : 0;
+  const bool fast = op.fast;
+  auto make_table = [&](int c) {
+    const int k0 = kbeg + c * kBK;
+    if (Op::kPixelRows) {
+      if (tid < kBK) tab[c & 1][tid] = k0 + tid < kend ? op.tap(k0 + tid) : make_int4(0, 2, 0, 0);
+    } else {
+      if (tid < kBK / 8) tab[c & 1][tid] = op.pixel(k0 + 8 * tid);
+    }
+  };
   if (warp == 0) {
     tmem_alloc<false>(&tslot, BN);
     tmem_relinquish<false>();
@@ -82,11 +134,20 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (fast && nch > 0) make_table(0);
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tacc = tslot;
-  constexpr uint32_t idesc = make_idesc_bf16(kBM, BN);
+  // this thread's pixels (rows m0 + 8 (tid & 15) ...) or row
+  const int mg = m0 + (tid & 15) * 8;
+  const bool mine = Op::kPixelRows ? mg + 7 < M : m0 + (tid & 127) < M;
+  const int4 at = !fast || !mine ? make_int4(0, 0, 0, 0)
+                  : Op::kPixelRows ? op.pixel(mg)
+                                   : op.tap(m0 + (tid & 127));
+  const bool kmajor = !Op::kPixelRows && fast;
+  const uint32_t idesc = kmajor ? make_idesc_bf16(kBM, BN) & ~((1u << 15) | (1u << 16))
+                                : make_idesc_bf16(kBM, BN);
   bool ok = true;
   for (int c = 0; c < nch; c++) {
     const int st = c & 1;
@@ -99,37 +160,76 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
     uint8_t* sa = base + st * L::kStage;
     uint8_t* sb = sa + L::kTileA;
     const int k0 = kbeg + c * kBK;
-    for (int idx = tid; idx < (kBM / 8) * kBK; idx += kGemmThreads) {
-      const int og = idx & (kBM / 8 - 1), kk = idx / (kBM / 8);
-      const int k = k0 + kk;
-      float v[8];
-      const int mg = m0 + og * 8;
-      if (k < kend && mg + 7 < M && op.rows8()) {
-        op.a8(mg, k, v);
-      } else {
+    if (Op::kPixelRows && fast) {
+#pragma unroll
+      for (int i = 0; i < kBK / 16; i++) {
+        const int kk = (tid >> 4) + 16 * i;
+        const int4 t = tab[st][kk];
+        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (mine) {
+          if (t.y != 2 && (unsigned)(at.y + t.y) < (unsigned)op.H)
+            row8(op.src() + at.x + t.x, at.z, t.z, op.W, v);
+        } else if (k0 + kk < kend) {
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            if (mg + j < M) v[j] = op.a(mg + j, k0 + kk);
+        }
+        *reinterpret_cast<uint4*>(sa + tile_off((tid & 15) >> 3, tid & 7, kk, L::kSboA)) = pack8(v);
+      }
+    } else if (kmajor) {
+      const int r = tid & 127;
+#pragma unroll
+      for (int i = 0; i < kBK / 16; i++) {
+        const int g = (tid >> 7) + 2 * i;
+        const int4 p = tab[st][g];  // {offset of the pixels in a plane set, y, x, batch}
+        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (mine && k0 + 8 * g < kend && (unsigned)(p.y + at.y) < (unsigned)op.H)
+          row8(op.src() + p.x + at.x, p.z, at.z, op.W, v);
+        *reinterpret_cast<uint4*>(sa + kmajor_off(r, g)) = pack8(v);
+      }
+    } else {
+      for (int idx = tid; idx < (kBM / 8) * kBK; idx += kGemmThreads) {
+        const int og = idx & (kBM / 8 - 1), kk = idx / (kBM / 8);
+        const int k = k0 + kk;
+        float v[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          const int m = mg + i;
+          const int m = m0 + og * 8 + i;
           v[i] = (k < kend && m < M) ? op.a(m, k) : 0.0f;
         }
+        *reinterpret_cast<uint4*>(sa + tile_off(og >> 3, og & 7, kk, L::kSboA)) = pack8(v);
       }
-      *reinterpret_cast<uint4*>(sa + tile_off(og >> 3, og & 7, kk, L::kSboA)) =
-          make_uint4(bf16x2(v[0], v[1]), bf16x2(v[2], v[3]), bf16x2(v[4], v[5]),
-                     bf16x2(v[6], v[7]));
     }
-    for (int idx = tid; idx < (BN / 8) * kBK; idx += kGemmThreads) {
-      const int og = idx % (BN / 8), kk = idx / (BN / 8);
-      const int k = k0 + kk;
-      float v[8];
+    if (Op::kPixelRows && op.packed) {
+      // the tile image as it lies in shared memory
+      const uint4* src = op.packed + ((size_t)blockIdx.y * ((K + kBK - 1) / kBK) + k0 / kBK) *
+                                         (L::kTileB / 16);
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int n = n0 + og * 8 + i;
-        v[i] = (k < kend && n < N) ? op.b(k, n) : 0.0f;
+      for (int i = 0; i < (int)(L::kTileB / 16) / kGemmThreads; i++)
+        reinterpret_cast<uint4*>(sb)[tid + i * kGemmThreads] = __ldg(src + tid + i * kGemmThreads);
+    } else if (kmajor) {
+#pragma unroll
+      for (int i = 0; i < (BN / 8) * kBK / kGemmThreads; i++) {
+        const int r = tid % BN, g = tid / BN + (kGemmThreads / BN) * i;
+        const int4 p = tab[st][g];
+        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (n0 + r < N && k0 + 8 * g < kend) row8(op.grad_row(n0 + r, p), p.z, 0, op.W, v);
+        *reinterpret_cast<uint4*>(sb + kmajor_off(r, g)) = pack8(v);
       }
-      *reinterpret_cast<uint4*>(sb + tile_off(og >> 3, og & 7, kk, L::kSboB)) =
-          make_uint4(bf16x2(v[0], v[1]), bf16x2(v[2], v[3]), bf16x2(v[4], v[5]),
-                     bf16x2(v[6], v[7]));
+    } else {
+      for (int idx = tid; idx < (BN / 8) * kBK; idx += kGemmThreads) {
+        const int og = idx % (BN / 8), kk = idx / (BN / 8);
+        const int k = k0 + kk;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int n = n0 + og * 8 + i;
+          v[i] = (k < kend && n < N) ? op.b(k, n) : 0.0f;
+        }
+        *reinterpret_cast<uint4*>(sb + tile_off(og >> 3, og & 7, kk, L::kSboB)) = pack8(v);
+      }
     }
+    if (fast && c + 1 < nch) make_table(c + 1);
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
@@ -137,8 +237,10 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
       const uint32_t aa = smem_u32(sa), ba = smem_u32(sb);
 #pragma unroll
       for (int t = 0; t < kBK / 16; t++) {
-        const uint64_t ad = make_desc(aa + t * 2 * L::kSboA, 1024, L::kSboA);
-        const uint64_t bd = make_desc(ba + t * 2 * L::kSboB, 1024, L::kSboB);
+        const uint64_t ad = kmajor ? make_desc(aa + t * 32, 16, 1024)
+                                   : make_desc(aa + t * 2 * L::kSboA, 1024, L::kSboA);
+        const uint64_t bd = kmajor ? make_desc(ba + t * 32, 16, 1024)
+                                   : make_desc(ba + t * 2 * L::kSboB, 1024, L::kSboB);
         mma_f16<false>(tacc, ad, bd, idesc, (c > 0 || t > 0) ? 1u : 0u);
       }
       mma_commit<false>(&bar[st]);
@@ -153,7 +255,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
     const int q = warp & 3, h = warp >> 2;
     const int m = m0 + 32 * q + lane;
 #pragma unroll 1
-    for (int cb = h * (BN / 2); cb < (h + 1) * (BN / 2); cb += 32) {
+    for (int cb = h * (BN / 2); cb < (h + 1) * (BN / 2) && n0 + cb < N; cb += 32) {
       float v[32];
       if (nch > 0) {
         tmem_ld32(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)cb, v);
@@ -162,10 +264,11 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
         for (int j = 0; j < 32; j++) v[j] = 0.0f;
       }
       if (m < M) {
+        const auto at_m = op.row(m);
 #pragma unroll 4
         for (int j = 0; j < 32; j++) {
           const int n = n0 + cb + j;
-          if (n < N) op.store(m, n, v[j], (int)blockIdx.z);
+          if (n < N) op.store(at_m, n, v[j], (int)blockIdx.z);
         }
       }
     }
@@ -183,19 +286,39 @@ struct View {
   int C, c0;
 };
 
+__device__ __host__ inline bool rows_of_eight(const float* p, int W) {
+  return W % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+}
+
 // forward: y = act(conv(x) + bias); with split-K (part set) each split
 // stores its partial sum to part[split][n][m] and k_conv_fwd_finish adds
 // the splits, the bias and the activation
 struct ConvFwdOp {
+  static constexpr bool kPixelRows = true;
   const float* x;
   int xC, xc0;
   const float* w;
+  const uint4* packed;  // BF16 tile images of w (k_pack_weights), or null
   const float* bias;
   float* y;
   int yC, yc0;
   int Cin, Cout, H, W, ks, relu;
   float* part;
   int M;
+  bool fast;
+  __device__ const float* src() const { return x; }
+  // a pixel: {offset of its plane set's first channel and itself, y, x}
+  __device__ int4 pixel(int m) const {
+    const int HW = H * W;
+    const int b = m / HW, r = m - b * HW, y0 = r / W;
+    return make_int4((b * xC + xc0) * HW + r, y0, r - y0 * W, 0);
+  }
+  // a row of the weights: {offset of its channel and row, dy, dx}
+  __device__ int4 tap(int k) const {
+    const int kk = ks * ks, cin = k / kk, t = k - cin * kk;
+    const int dy = t / ks - ks / 2, dx = t % ks - ks / 2;
+    return make_int4(cin * H * W + dy * W, dy, dx, 0);
+  }
   __device__ float a(int m, int k) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW, y0 = r / W, x0 = r - y0 * W;
@@ -204,33 +327,22 @@ struct ConvFwdOp {
     if ((unsigned)yy >= (unsigned)H || (unsigned)xx >= (unsigned)W) return 0.0f;
     return x[((size_t)(b * xC + xc0 + cin) * H + yy) * W + xx];
   }
-  // a(m + i, k) for i < 8, when rows m..m+7 are in one image row (rows8):
-  // the index arithmetic once for the eight
-  __device__ bool rows8() const { return (W & 7) == 0; }
-  __device__ void a8(int m, int k, float* v) const {
-    const int HW = H * W;
-    const int b = m / HW, r = m - b * HW, y0 = r / W, x0 = r - y0 * W;
-    const int kk = ks * ks, cin = k / kk, t = k - cin * kk;
-    const int yy = y0 + t / ks - ks / 2, dx = t % ks - ks / 2;
-    const bool rowok = (unsigned)yy < (unsigned)H;
-    const float* row = x + ((size_t)(b * xC + xc0 + cin) * H + (rowok ? yy : 0)) * W;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int xx = x0 + i + dx;
-      v[i] = (rowok && (unsigned)xx < (unsigned)W) ? row[xx] : 0.0f;
-    }
-  }
   __device__ float b(int k, int n) const { return w[(size_t)n * Cin * ks * ks + k]; }
-  __device__ void store(int m, int n, float v, int split) const {
-    if (part) {
-      part[((size_t)split * Cout + n) * M + m] = v;
-      return;
-    }
+  __device__ const float* grad_row(int, const int4&) const { return nullptr; }
+  // where row m of the result goes: {m, offset of its pixel in y}
+  __device__ int2 row(int m) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW;
+    return make_int2(m, (b * yC + yc0) * HW + r);
+  }
+  __device__ void store(const int2& at, int n, float v, int split) const {
+    if (part) {
+      part[((size_t)split * Cout + n) * M + at.x] = v;
+      return;
+    }
     v += bias[n];
     if (relu) v = fmaxf(v, 0.0f);
-    y[(size_t)(b * yC + yc0 + n) * HW + r] = v;
+    y[(size_t)at.y + (size_t)n * H * W] = v;
   }
 };
 
@@ -249,14 +361,31 @@ __global__ void k_conv_fwd_finish(int M, int N, int nsplit, const float* __restr
   y[(size_t)(b * yC + yc0 + n) * HW + r] = s;
 }
 
-// backward data: dx (+)= conv of dz with the taps flipped
+// backward data: dx = conv of dz with the taps flipped; with `act` (the
+// activation whose gradient dx is) masked by its ReLU
 struct ConvBwdDataOp {
+  static constexpr bool kPixelRows = true;
   const float* dz;
   int zC, zc0;
   const float* w;
+  const uint4* packed;
   float* dx;
   int xC, xc0;
-  int Cin, Cout, H, W, ks, accumulate;
+  const float* act;
+  int aC, ac0;
+  int Cin, Cout, H, W, ks;
+  bool fast;
+  __device__ const float* src() const { return dz; }
+  __device__ int4 pixel(int m) const {
+    const int HW = H * W;
+    const int b = m / HW, r = m - b * HW, y0 = r / W;
+    return make_int4((b * zC + zc0) * HW + r, y0, r - y0 * W, 0);
+  }
+  __device__ int4 tap(int k) const {
+    const int kk = ks * ks, co = k / kk, t = k - co * kk;
+    const int dy = ks / 2 - t / ks, dx = ks / 2 - t % ks;
+    return make_int4(co * H * W + dy * W, dy, dx, 0);
+  }
   __device__ float a(int m, int k) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW, y0 = r / W, x0 = r - y0 * W;
@@ -265,41 +394,47 @@ struct ConvBwdDataOp {
     if ((unsigned)yy >= (unsigned)H || (unsigned)xx >= (unsigned)W) return 0.0f;
     return dz[((size_t)(b * zC + zc0 + co) * H + yy) * W + xx];
   }
-  __device__ bool rows8() const { return (W & 7) == 0; }
-  __device__ void a8(int m, int k, float* v) const {
-    const int HW = H * W;
-    const int b = m / HW, r = m - b * HW, y0 = r / W, x0 = r - y0 * W;
-    const int kk = ks * ks, co = k / kk, t = k - co * kk;
-    const int yy = y0 - t / ks + ks / 2, dx = -(t % ks) + ks / 2;
-    const bool rowok = (unsigned)yy < (unsigned)H;
-    const float* row = dz + ((size_t)(b * zC + zc0 + co) * H + (rowok ? yy : 0)) * W;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int xx = x0 + i + dx;
-      v[i] = (rowok && (unsigned)xx < (unsigned)W) ? row[xx] : 0.0f;
-    }
-  }
   __device__ float b(int k, int n) const {
     const int kk = ks * ks, co = k / kk, t = k - co * kk;
     return w[((size_t)co * Cin + n) * kk + t];
   }
-  __device__ void store(int m, int n, float v, int) const {
+  __device__ const float* grad_row(int, const int4&) const { return nullptr; }
+  __device__ int2 row(int m) const {
     const int HW = H * W;
-    const int b = m / HW, r = m - b * HW;
-    float* o = dx + (size_t)(b * xC + xc0 + n) * HW + r;
-    *o = accumulate ? *o + v : v;
+    const int b = m / HW;
+    return make_int2(b, m - b * HW);
+  }
+  __device__ void store(const int2& at, int n, float v, int) const {
+    const int HW = H * W;
+    if (act && !(act[(size_t)(at.x * aC + ac0 + n) * HW + at.y] > 0.0f)) v = 0.0f;
+    dx[(size_t)(at.x * xC + xc0 + n) * HW + at.y] = v;
   }
 };
 
 // backward weight: partial[split][cout][cin*ks*ks] = sum over this split's
 // pixels of dz * x (shifted)
 struct ConvBwdWeightOp {
+  static constexpr bool kPixelRows = false;
   const float* x;
   int xC, xc0;
   const float* dz;
   int zC, zc0;
   float* partial;
   int Cin, Cout, H, W, ks;
+  bool fast;
+  static constexpr const uint4* packed = nullptr;
+  __device__ const float* src() const { return x; }
+  // eight pixels: {their offset in x's first channel, y, x, batch}
+  __device__ int4 pixel(int k) const {
+    const int HW = H * W;
+    const int b = k / HW, r = k - b * HW, y0 = r / W;
+    return make_int4((b * xC + xc0) * HW + r, y0, r - y0 * W, b);
+  }
+  __device__ int4 tap(int m) const {
+    const int kk = ks * ks, cin = m / kk, t = m - cin * kk;
+    const int dy = t / ks - ks / 2, dx = t % ks - ks / 2;
+    return make_int4(cin * H * W + dy * W, dy, dx, 0);
+  }
   __device__ float a(int m, int k) const {
     const int kk = ks * ks, cin = m / kk, t = m - cin * kk;
     const int HW = H * W;
@@ -308,13 +443,15 @@ struct ConvBwdWeightOp {
     if ((unsigned)yy >= (unsigned)H || (unsigned)xx >= (unsigned)W) return 0.0f;
     return x[((size_t)(b * xC + xc0 + cin) * H + yy) * W + xx];
   }
-  __device__ bool rows8() const { return false; }  // rows are (cin, tap) pairs
-  __device__ void a8(int, int, float*) const {}
   __device__ float b(int k, int n) const {
     const int HW = H * W;
     const int b = k / HW, r = k - b * HW;
     return dz[(size_t)(b * zC + zc0 + n) * HW + r];
   }
+  __device__ const float* grad_row(int n, const int4& p) const {
+    return dz + (size_t)(p.w * zC + zc0 + n) * H * W + p.y * W + p.z;
+  }
+  __device__ int row(int m) const { return m; }
   __device__ void store(int m, int n, float v, int split) const {
     const size_t wn = (size_t)Cout * Cin * ks * ks;
     partial[split * wn + (size_t)n * Cin * ks * ks + m] = v;
@@ -332,94 +469,152 @@ __global__ void k_sum_splits(size_t n, int nsplit, const float* __restrict__ par
   out[i] = s;
 }
 
-__global__ void k_bias_grad(int B, int HW, View dz, float* __restrict__ db) {
-  const int c = blockIdx.x;
-  float s = 0.0f;
-  for (int b = 0; b < B; b++) {
-    const float* p = dz.p + (size_t)(b * dz.C + dz.c0 + c) * HW;
-    for (int i = threadIdx.x; i < HW; i += blockDim.x) s += p[i];
+// db[c] = sum over pixels of dz, as 256 threads striding over each plane of
+// the batch add it: thread t takes pixels t, t + 256, ..., then a butterfly
+// within each warp and one over the warps.  A block stands for one of those
+// 8 warps (blockIdx.x), so that a channel's sum is not one block's: all its
+// threads bring the next 128 steps of the warp's 32 running sums into shared
+// memory while the first warp adds the last ones.  16 channels of 256^2,
+// batch 8, in one block each: some 600 us; so: 30 us.
+constexpr int kBiasSteps = 128;
+__global__ void __launch_bounds__(256) k_bias_grad(int B, int HW, View dz, float* __restrict__ part,
+                                                   uint32_t* __restrict__ done,
+                                                   float* __restrict__ db) {
+  __shared__ float stage[2][kBiasSteps][32];
+  const int c = blockIdx.y, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int S = (HW + 255) / 256, total = B * S;  // steps a plane, of the batch
+  const int t0 = blockIdx.x * 32 + lane;           // the thread stood for
+  float next[kBiasSteps / 8];
+  auto fetch = [&](int s0) {
+#pragma unroll
+    for (int k = 0; k < kBiasSteps / 8; k++) {
+      const int s = s0 + row + 8 * k, b = s / S, i = t0 + 256 * (s - b * S);
+      next[k] = s < total && i < HW ? dz.p[(size_t)(b * dz.C + dz.c0 + c) * HW + i] : 0.0f;
+    }
+  };
+  fetch(0);
+  float sum = 0.0f;
+  int st = 0;
+  for (int s0 = 0; s0 < total; s0 += kBiasSteps, st ^= 1) {
+#pragma unroll
+    for (int k = 0; k < kBiasSteps / 8; k++) stage[st][row + 8 * k][lane] = next[k];
+    if (s0 + kBiasSteps < total) fetch(s0 + kBiasSteps);
+    __syncthreads();
+    if (row == 0) {
+#pragma unroll 16
+      for (int k = 0; k < kBiasSteps; k++) sum += stage[st][k][lane];
+    }
   }
-  __shared__ float red[32];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) db[c] = s;
+  if (row == 0) {
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) part[c * 8 + blockIdx.x] = sum;
+  }
+  if (!last_block_done(done, gridDim.x * gridDim.y)) return;
+  for (int k = threadIdx.x; k < (int)gridDim.y; k += blockDim.x) {
+    float w[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) w[i] = __ldcg(part + k * 8 + i);
+    db[k] = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
   }
 }
 
-// dz = g * (y > 0) over a slice of C channels (in place when g == dz)
-__global__ void k_relu_mask(int B, int C, int HW, View g, View y, View dz) {
-  const size_t n = (size_t)B * C * HW;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i % HW);
-    const size_t bc = i / HW;
-    const int c = (int)(bc % C), b = (int)(bc / C);
-    const float yv = y.p[(size_t)(b * y.C + y.c0 + c) * HW + r];
-    const float gv = g.p[(size_t)(b * g.C + g.c0 + c) * HW + r];
-    dz.p[(size_t)(b * dz.C + dz.c0 + c) * HW + r] = yv > 0.0f ? gv : 0.0f;
+// The resampling kernels: blockIdx.y = batch and channel, a thread per pixel
+// of the smaller side.  y = 2x2 average of x (x is H x W, y is H/2 x W/2)
+__global__ void __launch_bounds__(256) k_pool2(int C, int H, int W, View x, View y) {
+  const int c = blockIdx.y % C, b = blockIdx.y / C, Ho = H / 2, Wo = W / 2;
+  const float* xp = x.p + (size_t)(b * x.C + x.c0 + c) * H * W;
+  float* yp = y.p + (size_t)(b * y.C + y.c0 + c) * Ho * Wo;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Ho * Wo; i += gridDim.x * blockDim.x) {
+    const int yo = i / Wo, xo = i - yo * Wo;
+    const float2 u = *reinterpret_cast<const float2*>(xp + (size_t)2 * yo * W + 2 * xo);
+    const float2 v = *reinterpret_cast<const float2*>(xp + (size_t)(2 * yo + 1) * W + 2 * xo);
+    yp[i] = 0.25f * ((u.x + u.y) + (v.x + v.y));
   }
 }
 
-// y = 2x2 average of x (x is H x W, y is H/2 x W/2)
-__global__ void k_pool2(int B, int C, int H, int W, View x, View y) {
-  const int Ho = H / 2, Wo = W / 2;
-  const size_t n = (size_t)B * C * Ho * Wo;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int xo = (int)(i % Wo), yo = (int)((i / Wo) % Ho);
-    const size_t bc = i / ((size_t)Wo * Ho);
-    const int c = (int)(bc % C), b = (int)(bc / C);
-    const float* s = x.p + ((size_t)(b * x.C + x.c0 + c) * H + 2 * yo) * W + 2 * xo;
-    y.p[((size_t)(b * y.C + y.c0 + c) * Ho + yo) * Wo + xo] =
-        0.25f * ((s[0] + s[1]) + (s[W] + s[W + 1]));
-  }
-}
-
-// dx (+)= dy / 4 broadcast over each 2x2 block
-__global__ void k_pool2_bwd(int B, int C, int H, int W, View dy, View dx, int accumulate) {
-  const size_t n = (size_t)B * C * H * W;
-  const int Ho = H / 2, Wo = W / 2;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int xx = (int)(i % W), yy = (int)((i / W) % H);
-    const size_t bc = i / ((size_t)W * H);
-    const int c = (int)(bc % C), b = (int)(bc / C);
-    const float g =
-        0.25f * dy.p[((size_t)(b * dy.C + dy.c0 + c) * Ho + yy / 2) * Wo + xx / 2];
-    float* o = dx.p + ((size_t)(b * dx.C + dx.c0 + c) * H + yy) * W + xx;
-    *o = accumulate ? *o + g : g;
+// dx += dy / 4 broadcast over each 2x2 block, then masked by the ReLU of act
+// (dx's activation)
+__global__ void __launch_bounds__(256) k_pool2_bwd(int C, int H, int W, View dy, View dx,
+                                                   View act) {
+  const int c = blockIdx.y % C, b = blockIdx.y / C, Ho = H / 2, Wo = W / 2;
+  const float* gp = dy.p + (size_t)(b * dy.C + dy.c0 + c) * Ho * Wo;
+  float* xp = dx.p + (size_t)(b * dx.C + dx.c0 + c) * H * W;
+  const float* ap = act.p + (size_t)(b * act.C + act.c0 + c) * H * W;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Ho * Wo; i += gridDim.x * blockDim.x) {
+    const int yo = i / Wo, xo = i - yo * Wo;
+    const float g = 0.25f * gp[i];
+#pragma unroll
+    for (int d = 0; d < 2; d++) {
+      const size_t o = (size_t)(2 * yo + d) * W + 2 * xo;
+      const float2 v = *reinterpret_cast<const float2*>(xp + o);
+      const float2 y = *reinterpret_cast<const float2*>(ap + o);
+      *reinterpret_cast<float2*>(xp + o) =
+          make_float2(y.x > 0.0f ? v.x + g : 0.0f, y.y > 0.0f ? v.y + g : 0.0f);
+    }
   }
 }
 
 // y = nearest 2x upsample of x (x is H x W)
-__global__ void k_up2(int B, int C, int H, int W, View x, View y) {
-  const int Ho = 2 * H, Wo = 2 * W;
-  const size_t n = (size_t)B * C * Ho * Wo;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int xo = (int)(i % Wo), yo = (int)((i / Wo) % Ho);
-    const size_t bc = i / ((size_t)Wo * Ho);
-    const int c = (int)(bc % C), b = (int)(bc / C);
-    y.p[((size_t)(b * y.C + y.c0 + c) * Ho + yo) * Wo + xo] =
-        x.p[((size_t)(b * x.C + x.c0 + c) * H + yo / 2) * W + xo / 2];
+__global__ void __launch_bounds__(256) k_up2(int C, int H, int W, View x, View y) {
+  const int c = blockIdx.y % C, b = blockIdx.y / C, Wo = 2 * W;
+  const float* xp = x.p + (size_t)(b * x.C + x.c0 + c) * H * W;
+  float* yp = y.p + (size_t)(b * y.C + y.c0 + c) * 4 * H * W;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H * W; i += gridDim.x * blockDim.x) {
+    const int yy = i / W, xx = i - yy * W;
+    const float2 v = make_float2(xp[i], xp[i]);
+    *reinterpret_cast<float2*>(yp + (size_t)2 * yy * Wo + 2 * xx) = v;
+    *reinterpret_cast<float2*>(yp + (size_t)(2 * yy + 1) * Wo + 2 * xx) = v;
   }
 }
 
-// dx = sum of dy over each 2x2 block (dx is H x W)
-__global__ void k_up2_bwd(int B, int C, int H, int W, View dy, View dx) {
-  const size_t n = (size_t)B * C * H * W;
-  const int Wo = 2 * W;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int xx = (int)(i % W), yy = (int)((i / W) % H);
-    const size_t bc = i / ((size_t)W * H);
-    const int c = (int)(bc % C), b = (int)(bc / C);
-    const float* s = dy.p + ((size_t)(b * dy.C + dy.c0 + c) * (2 * H) + 2 * yy) * Wo + 2 * xx;
-    dx.p[((size_t)(b * dx.C + dx.c0 + c) * H + yy) * W + xx] = (s[0] + s[1]) + (s[Wo] + s[Wo + 1]);
+// dx = sum of dy over each 2x2 block (dx is H x W), masked by the ReLU of act
+__global__ void __launch_bounds__(256) k_up2_bwd(int C, int H, int W, View dy, View dx, View act) {
+  const int c = blockIdx.y % C, b = blockIdx.y / C, Wo = 2 * W;
+  const float* gp = dy.p + (size_t)(b * dy.C + dy.c0 + c) * 4 * H * W;
+  float* xp = dx.p + (size_t)(b * dx.C + dx.c0 + c) * H * W;
+  const float* ap = act.p + (size_t)(b * act.C + act.c0 + c) * H * W;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H * W; i += gridDim.x * blockDim.x) {
+    const int yy = i / W, xx = i - yy * W;
+    const float2 u = *reinterpret_cast<const float2*>(gp + (size_t)2 * yy * Wo + 2 * xx);
+    const float2 v = *reinterpret_cast<const float2*>(gp + (size_t)(2 * yy + 1) * Wo + 2 * xx);
+    xp[i] = ap[i] > 0.0f ? (u.x + u.y) + (v.x + v.y) : 0.0f;
+  }
+}
+
+// BF16 tile images of the weights as the GEMMs' B operand (forward and data
+// gradient), one 16-byte group of eight columns at a time; made when the
+// parameters change, so that a tile is a copy instead of 64 strided loads a row.
+struct PackEntry {
+  size_t w;      // offset of the layer's weights
+  int cin, cout, ks, backward;
+  int bn, tiles, chunks;
+  size_t out;    // offset of the images (16-byte units)
+};
+
+__global__ void __launch_bounds__(256) k_pack_weights(const PackEntry* __restrict__ entries,
+                                                      const float* __restrict__ params,
+                                                      uint4* __restrict__ packed) {
+  const PackEntry e = entries[blockIdx.y];
+  const int kk = e.ks * e.ks, K = (e.backward ? e.cout : e.cin) * kk;
+  const int N = e.backward ? e.cin : e.cout;
+  const int per = e.bn / 8 * kBK;  // groups of a tile
+  const float* w = params + e.w;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < e.tiles * e.chunks * per;
+       i += gridDim.x * blockDim.x) {
+    const int tile = i / per, r = i - tile * per;  // n tile * chunks + chunk
+    const int og = r % (e.bn / 8), kr = r / (e.bn / 8);
+    const int k = (tile % e.chunks) * kBK + kr, n0 = (tile / e.chunks) * e.bn + og * 8;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int n = n0 + j;
+      float x = 0.0f;
+      if (k < K && n < N)
+        x = e.backward ? w[((size_t)(k / kk) * e.cin + n) * kk + k % kk] : w[(size_t)n * K + k];
+      v[j] = x;
+    }
+    packed[e.out + (size_t)tile * per + tile_off(og >> 3, og & 7, kr, (e.bn / 64) * 1024) / 16] =
+        pack8(v);
   }
 }
 
@@ -466,6 +661,7 @@ struct Ctx {
   int num_sms;
   float* part;  // split-K scratch for the weight gradient
   size_t part_floats;
+  uint32_t* done = nullptr;  // block counter of k_bias_grad
 };
 
 template <class Op, int BN>
@@ -488,24 +684,32 @@ gv_status launch_gemm(const Ctx& c, const Op& op, int M, int N, int K, int nspli
   return launch_gemm_bn<Op, 256>(c, op, M, N, K, nsplit);  // column tiles of 256
 }
 
+// grid of the per-channel kernels: n pixels a channel, `planes` of them
+inline dim3 plane_grid(int n, int planes) {
+  return dim3((unsigned)std::min((n + 255) / 256, 64), (unsigned)planes);
+}
+
+inline int tile_columns(int N) { return N <= 64 ? 64 : (N <= 128 ? 128 : 256); }
+
 inline int ew_blocks(size_t n, const Ctx& c) {
   return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, (size_t)8 * c.num_sms));
 }
 
-gv_status conv_forward(const Ctx& c, View x, const float* w, const float* bias, View y, int B,
-                       int Cin, int Cout, int H, int W, int ks, int relu) {
+gv_status conv_forward(const Ctx& c, View x, const float* w, const uint4* packed,
+                       const float* bias, View y, int B, int Cin, int Cout, int H, int W, int ks,
+                       int relu) {
   const int M = B * H * W, N = Cout, K = Cin * ks * ks;
   // a grid of fewer tiles than SMs (deep levels, small batches) splits K
   // over up to two CTAs per SM, at least two K blocks a split
-  const int bn = N <= 64 ? 64 : (N <= 128 ? 128 : 256);
+  const int bn = tile_columns(N);
   const int tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
   int nsplit = 1;
   if (c.part && tiles < c.num_sms) {
     nsplit = std::min(K / (2 * kBK), (2 * c.num_sms + tiles - 1) / tiles);
     nsplit = std::max(1, std::min<int>(nsplit, (int)(c.part_floats / ((size_t)M * N))));
   }
-  ConvFwdOp op{x.p, x.C, x.c0, w, bias, y.p, y.C, y.c0, Cin, Cout, H, W, ks, relu,
-               nsplit > 1 ? c.part : nullptr, M};
+  ConvFwdOp op{x.p, x.C, x.c0, w, packed, bias, y.p, y.C, y.c0, Cin, Cout, H, W, ks, relu,
+               nsplit > 1 ? c.part : nullptr, M, rows_of_eight(x.p, W)};
   gv_status s = launch_gemm(c, op, M, N, K, nsplit);
   if (s != GV_OK || nsplit <= 1) return s;
   // the kernel launched ceil(K / klen) splits; sum exactly those
@@ -517,9 +721,10 @@ gv_status conv_forward(const Ctx& c, View x, const float* w, const float* bias, 
   return GV_OK;
 }
 
-gv_status conv_backward_data(const Ctx& c, View dz, const float* w, View dx, int B, int Cin,
-                             int Cout, int H, int W, int ks, int accumulate) {
-  ConvBwdDataOp op{dz.p, dz.C, dz.c0, w, dx.p, dx.C, dx.c0, Cin, Cout, H, W, ks, accumulate};
+gv_status conv_backward_data(const Ctx& c, View dz, const float* w, const uint4* packed, View dx,
+                             View act, int B, int Cin, int Cout, int H, int W, int ks) {
+  ConvBwdDataOp op{dz.p, dz.C, dz.c0, w, packed, dx.p, dx.C, dx.c0, act.p, act.C, act.c0, Cin, Cout,
+                   H, W, ks, rows_of_eight(dz.p, W)};
   return launch_gemm(c, op, B * H * W, Cin, Cout * ks * ks);
 }
 
@@ -530,7 +735,8 @@ gv_status conv_backward_weight(const Ctx& c, View x, View dz, float* dw, float* 
   const size_t wn = (size_t)M * N;
   int nsplit = std::max(1, std::min(K / 1024, (2 * c.num_sms + tiles - 1) / tiles));
   nsplit = std::max(1, std::min<int>(nsplit, (int)(c.part_floats / wn)));
-  ConvBwdWeightOp op{x.p, x.C, x.c0, dz.p, dz.C, dz.c0, c.part, Cin, Cout, H, W, ks};
+  ConvBwdWeightOp op{x.p, x.C, x.c0, dz.p, dz.C, dz.c0, c.part, Cin, Cout, H, W, ks,
+                     rows_of_eight(x.p, W) && rows_of_eight(dz.p, W)};
   gv_status s = launch_gemm(c, op, M, N, K, nsplit);
   if (s != GV_OK) return s;
   // the kernel launched ceil(K / klen) splits; sum exactly those
@@ -538,7 +744,8 @@ gv_status conv_backward_weight(const Ctx& c, View x, View dz, float* dw, float* 
   const int nz = (K + klen - 1) / klen;
   k_sum_splits<<<(unsigned)((wn + 255) / 256), 256, 0, c.stream>>>(wn, nz, c.part, dw);
   GV_LAUNCH("k_sum_splits");
-  k_bias_grad<<<Cout, 256, 0, c.stream>>>(B, H * W, dz, db);
+  // the splits' scratch is free again
+  k_bias_grad<<<dim3(8, Cout), 256, 0, c.stream>>>(B, H * W, dz, c.part, c.done, db);
   GV_LAUNCH("k_bias_grad");
   return GV_OK;
 }
@@ -575,7 +782,21 @@ struct UNet {
 
   int C(int l) const { return c0 << l; }
   int S(int l) const { return H >> l; }
-  Ctx ctx() const { return Ctx{stream, err, num_sms, part, part_floats}; }
+  // BF16 tile images of the weights: forward, then data gradient, per layer
+  std::vector<PackEntry> entries;
+  PackEntry* d_entries = nullptr;
+  uint4* packed = nullptr;
+  Ctx ctx() const { return Ctx{stream, err, num_sms, part, part_floats, err + 1}; }
+  const uint4* image(int layer, int backward) const {
+    return packed + entries[2 * layer + backward].out;
+  }
+  // after every change of the parameters
+  gv_status pack() {
+    k_pack_weights<<<dim3(32, (unsigned)entries.size()), 256, 0, stream>>>(d_entries, params,
+                                                                           packed);
+    GV_LAUNCH("k_pack_weights");
+    return GV_OK;
+  }
 
   gv_status alloc(float** p, size_t n) {
     GV_CUDA(cudaMalloc(p, std::max<size_t>(n, 1) * sizeof(float)));
@@ -671,9 +892,24 @@ struct UNet {
     GV_TRY(alloc(&part, part_floats));
     GV_CUDA(cudaMalloc(&loss_part, sizeof(double) * 1024));
     allocs.push_back(loss_part);
-    GV_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
+    GV_CUDA(cudaMalloc(&err, 2 * sizeof(uint32_t)));  // error word, block counter
     allocs.push_back(err);
-    GV_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), stream));
+    GV_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(uint32_t), stream));
+    size_t images = 0;
+    for (const Layer& ly : layers)
+      for (int back = 0; back < 2; back++) {
+        const int N = back ? ly.cin : ly.cout, K = (back ? ly.cout : ly.cin) * ly.ks * ly.ks;
+        const int bn = tile_columns(N), tiles = (N + bn - 1) / bn, chunks = (K + kBK - 1) / kBK;
+        entries.push_back({ly.w, ly.cin, ly.cout, ly.ks, back, bn, tiles, chunks, images});
+        images += (size_t)tiles * chunks * (bn / 8) * kBK;
+      }
+    GV_CUDA(cudaMalloc(&packed, sizeof(uint4) * images));
+    allocs.push_back(packed);
+    GV_CUDA(cudaMalloc(&d_entries, sizeof(PackEntry) * entries.size()));
+    allocs.push_back(d_entries);
+    GV_CUDA(cudaMemcpy(d_entries, entries.data(), sizeof(PackEntry) * entries.size(),
+                       cudaMemcpyHostToDevice));
+    GV_TRY(pack());
     GV_CUDA(cudaMallocHost(&h_loss, sizeof(double) * 1024));
     return GV_OK;
   }
@@ -734,119 +970,97 @@ struct UNet {
     return GV_OK;
   }
 
+  gv_status layer_forward(const Ctx& c, int k, View x, View y, int B, int s) {
+    const Layer& ly = layers[k];
+    return conv_forward(c, x, params + ly.w, image(k, 0), params + ly.b, y, B, ly.cin, ly.cout, s,
+                        s, ly.ks, ly.relu);
+  }
+
   // the forward pass on the network's input buffer in[0]
   gv_status forward_pass(int B) {
     const Ctx c = ctx();
     for (int l = 0; l < L; l++) {
       const int s = S(l), ci = l == 0 ? cin : C(l - 1);
-      const Layer& l1 = layers[enc_layer(l, 0)];
-      const Layer& l2 = layers[enc_layer(l, 1)];
-      GV_TRY(conv_forward(c, View{in[l], ci, 0}, params + l1.w, params + l1.b, View{a[l], C(l), 0},
-                          B, ci, C(l), s, s, 3, 1));
-      GV_TRY(conv_forward(c, View{a[l], C(l), 0}, params + l2.w, params + l2.b, enc_view(l), B,
-                          C(l), C(l), s, s, 3, 1));
+      GV_TRY(layer_forward(c, enc_layer(l, 0), View{in[l], ci, 0}, View{a[l], C(l), 0}, B, s));
+      GV_TRY(layer_forward(c, enc_layer(l, 1), View{a[l], C(l), 0}, enc_view(l), B, s));
       if (l + 1 < L) {
-        const size_t n = (size_t)B * C(l) * (s / 2) * (s / 2);
-        k_pool2<<<ew_blocks(n, c), 256, 0, stream>>>(B, C(l), s, s, enc_view(l),
-                                                     View{in[l + 1], C(l), 0});
+        k_pool2<<<plane_grid(s * s / 4, B * C(l)), 256, 0, stream>>>(C(l), s, s, enc_view(l),
+                                                                     View{in[l + 1], C(l), 0});
         GV_LAUNCH("k_pool2");
       }
     }
     for (int l = L - 2; l >= 0; l--) {
       const int s = S(l), cc = C(l + 1) + C(l);
-      const size_t n = (size_t)B * C(l + 1) * s * s;
-      k_up2<<<ew_blocks(n, c), 256, 0, stream>>>(B, C(l + 1), s / 2, s / 2, dec_view(l + 1),
-                                                 View{cat[l], cc, 0});
+      k_up2<<<plane_grid(s * s / 4, B * C(l + 1)), 256, 0, stream>>>(
+          C(l + 1), s / 2, s / 2, dec_view(l + 1), View{cat[l], cc, 0});
       GV_LAUNCH("k_up2");
-      const Layer& l1 = layers[dec_layer(l, 0)];
-      const Layer& l2 = layers[dec_layer(l, 1)];
-      GV_TRY(conv_forward(c, View{cat[l], cc, 0}, params + l1.w, params + l1.b, View{b[l], C(l), 0},
-                          B, cc, C(l), s, s, 3, 1));
-      GV_TRY(conv_forward(c, View{b[l], C(l), 0}, params + l2.w, params + l2.b, dec_view(l), B,
-                          C(l), C(l), s, s, 3, 1));
+      GV_TRY(layer_forward(c, dec_layer(l, 0), View{cat[l], cc, 0}, View{b[l], C(l), 0}, B, s));
+      GV_TRY(layer_forward(c, dec_layer(l, 1), View{b[l], C(l), 0}, dec_view(l), B, s));
     }
-    const Layer& lo = layers[out_layer()];
-    return conv_forward(c, dec_view(0), params + lo.w, params + lo.b, View{out, 1, 0}, B, C(0), 1,
-                        H, W, 1, 0);
+    return layer_forward(c, out_layer(), dec_view(0), View{out, 1, 0}, B, H);
   }
 
-  // gradients of the loss with respect to every parameter, given dout
+  // weight, bias and data gradient of layer k from dz (its pre-activation's
+  // gradient); dx is masked by the ReLU of act where act is set
+  gv_status layer_backward(const Ctx& c, int k, View x, View dz, View dx, View act, int B, int s) {
+    const Layer& ly = layers[k];
+    GV_TRY(conv_backward_weight(c, x, dz, grads + ly.w, grads + ly.b, B, ly.cin, ly.cout, s, s,
+                                ly.ks));
+    if (!dx.p) return GV_OK;
+    return conv_backward_data(c, dz, params + ly.w, image(k, 1), dx, act, B, ly.cin, ly.cout, s, s,
+                              ly.ks);
+  }
+
+  // gradients of the loss with respect to every parameter, given dout.  Every
+  // gradient of an activation is masked by that activation's ReLU where it is
+  // made (the data-gradient GEMM's epilogue or the resampling), so it is the
+  // next layer's dz as it stands.
   gv_status backward(int B) {
     const Ctx c = ctx();
-    const Layer& lo = layers[out_layer()];
-    GV_TRY(conv_backward_weight(c, dec_view(0), View{dout, 1, 0}, grads + lo.w, grads + lo.b, B,
-                                C(0), 1, H, W, 1));
-    GV_TRY(conv_backward_data(c, View{dout, 1, 0}, params + lo.w, ddec_view(0), B, C(0), 1, H, W,
-                              1, 0));
+    const View none{nullptr, 0, 0};
+    GV_TRY(layer_backward(c, out_layer(), dec_view(0), View{dout, 1, 0}, ddec_view(0), dec_view(0),
+                          B, H));
     for (int l = 0; l <= L - 2; l++) {
       const int s = S(l), cc = C(l + 1) + C(l);
-      const Layer& l1 = layers[dec_layer(l, 0)];
-      const Layer& l2 = layers[dec_layer(l, 1)];
-      const size_t nl = (size_t)B * C(l) * s * s;
-      // second decoder conv: ReLU mask, weight and data gradients
-      k_relu_mask<<<ew_blocks(nl, c), 256, 0, stream>>>(B, C(l), s * s, ddec_view(l), dec_view(l),
-                                                        ddec_view(l));
-      GV_LAUNCH("k_relu_mask");
-      GV_TRY(conv_backward_weight(c, View{b[l], C(l), 0}, ddec_view(l), grads + l2.w,
-                                  grads + l2.b, B, C(l), C(l), s, s, 3));
-      GV_TRY(conv_backward_data(c, ddec_view(l), params + l2.w, View{dbuf[l], C(l), 0}, B, C(l),
-                                C(l), s, s, 3, 0));
-      k_relu_mask<<<ew_blocks(nl, c), 256, 0, stream>>>(B, C(l), s * s, View{dbuf[l], C(l), 0},
-                                                        View{b[l], C(l), 0},
-                                                        View{dbuf[l], C(l), 0});
-      GV_LAUNCH("k_relu_mask");
-      GV_TRY(conv_backward_weight(c, View{cat[l], cc, 0}, View{dbuf[l], C(l), 0}, grads + l1.w,
-                                  grads + l1.b, B, cc, C(l), s, s, 3));
-      GV_TRY(conv_backward_data(c, View{dbuf[l], C(l), 0}, params + l1.w, View{dcat[l], cc, 0}, B,
-                                cc, C(l), s, s, 3, 0));
+      const View bv{b[l], C(l), 0}, dbv{dbuf[l], C(l), 0}, dcatv{dcat[l], cc, 0};
+      GV_TRY(layer_backward(c, dec_layer(l, 1), bv, ddec_view(l), dbv, bv, B, s));
+      GV_TRY(layer_backward(c, dec_layer(l, 0), View{cat[l], cc, 0}, dbv, dcatv, none, B, s));
       // the upsampled part of the concat feeds dec_{l+1}
-      const size_t nu = (size_t)B * C(l + 1) * (s / 2) * (s / 2);
-      k_up2_bwd<<<ew_blocks(nu, c), 256, 0, stream>>>(B, C(l + 1), s / 2, s / 2,
-                                                      View{dcat[l], cc, 0}, ddec_view(l + 1));
+      k_up2_bwd<<<plane_grid(s * s / 4, B * C(l + 1)), 256, 0, stream>>>(
+          C(l + 1), s / 2, s / 2, dcatv, ddec_view(l + 1), dec_view(l + 1));
       GV_LAUNCH("k_up2_bwd");
     }
     for (int l = L - 1; l >= 0; l--) {
       const int s = S(l), ci = l == 0 ? cin : C(l - 1);
-      const Layer& l1 = layers[enc_layer(l, 0)];
-      const Layer& l2 = layers[enc_layer(l, 1)];
-      const size_t nl = (size_t)B * C(l) * s * s;
       if (l + 1 < L) {
         // enc_l also feeds the pool of level l+1: add that gradient
-        k_pool2_bwd<<<ew_blocks(nl, c), 256, 0, stream>>>(B, C(l), s, s, View{din[l + 1], C(l), 0},
-                                                          denc_view(l), 1);
+        k_pool2_bwd<<<plane_grid(s * s / 4, B * C(l)), 256, 0, stream>>>(
+            C(l), s, s, View{din[l + 1], C(l), 0}, denc_view(l), enc_view(l));
         GV_LAUNCH("k_pool2_bwd");
       }
-      k_relu_mask<<<ew_blocks(nl, c), 256, 0, stream>>>(B, C(l), s * s, denc_view(l), enc_view(l),
-                                                        denc_view(l));
-      GV_LAUNCH("k_relu_mask");
-      GV_TRY(conv_backward_weight(c, View{a[l], C(l), 0}, denc_view(l), grads + l2.w, grads + l2.b,
-                                  B, C(l), C(l), s, s, 3));
-      GV_TRY(conv_backward_data(c, denc_view(l), params + l2.w, View{da[l], C(l), 0}, B, C(l), C(l),
-                                s, s, 3, 0));
-      k_relu_mask<<<ew_blocks(nl, c), 256, 0, stream>>>(B, C(l), s * s, View{da[l], C(l), 0},
-                                                        View{a[l], C(l), 0}, View{da[l], C(l), 0});
-      GV_LAUNCH("k_relu_mask");
-      GV_TRY(conv_backward_weight(c, View{in[l], ci, 0}, View{da[l], C(l), 0}, grads + l1.w,
-                                  grads + l1.b, B, ci, C(l), s, s, 3));
-      if (l > 0)
-        GV_TRY(conv_backward_data(c, View{da[l], C(l), 0}, params + l1.w, View{din[l], ci, 0}, B,
-                                  ci, C(l), s, s, 3, 0));
+      const View av{a[l], C(l), 0}, dav{da[l], C(l), 0};
+      GV_TRY(layer_backward(c, enc_layer(l, 1), av, denc_view(l), dav, av, B, s));
+      GV_TRY(layer_backward(c, enc_layer(l, 0), View{in[l], ci, 0}, dav,
+                            l > 0 ? View{din[l], ci, 0} : none, none, B, s));
     }
     return GV_OK;
   }
 
-  gv_status loss(const float* d_target, int B, bool grad, double* out_loss) {
+  // the loss' partial sums on their way to the host (loss_value, after a
+  // synchronisation) and its gradient in dout
+  static constexpr int kLossBlocks = 256;
+  gv_status loss_launch(const float* d_target, int B) {
     const size_t n = (size_t)B * H * W;
-    const int nb = 256;
-    k_mse<<<nb, 256, 0, stream>>>(n, out, d_target, grad ? dout : nullptr, loss_part);
+    k_mse<<<kLossBlocks, 256, 0, stream>>>(n, out, d_target, dout, loss_part);
     GV_LAUNCH("k_mse");
-    GV_CUDA(cudaMemcpyAsync(h_loss, loss_part, sizeof(double) * nb, cudaMemcpyDeviceToHost,
-                            stream));
-    GV_CUDA(cudaStreamSynchronize(stream));
+    GV_CUDA(cudaMemcpyAsync(h_loss, loss_part, sizeof(double) * kLossBlocks,
+                            cudaMemcpyDeviceToHost, stream));
+    return GV_OK;
+  }
+  double loss_value(int B) const {
     double s = 0.0;
-    for (int i = 0; i < nb; i++) s += h_loss[i];
-    if (out_loss) *out_loss = s / (double)n;
-    return check();
+    for (int i = 0; i < kLossBlocks; i++) s += h_loss[i];
+    return s / (double)((size_t)B * H * W);
   }
 
   gv_status adam(float lr) {
@@ -857,7 +1071,7 @@ struct UNet {
     k_adam<<<ew_blocks(nparams, c), 256, 0, stream>>>(nparams, params, grads, m, v, lr, b1, b2,
                                                       eps, c1, c2);
     GV_LAUNCH("k_adam");
-    return GV_OK;
+    return pack();
   }
 
   gv_status check() {
@@ -895,7 +1109,7 @@ gv::cnn::Ctx standalone_ctx(void* stream, uint32_t* err, float* part, size_t par
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return gv::cnn::Ctx{(cudaStream_t)stream, err, sms, part, part_floats};
+  return gv::cnn::Ctx{(cudaStream_t)stream, err, sms, part, part_floats, err + 1};
 }
 
 }  // namespace
@@ -967,6 +1181,7 @@ gv_status gv_unet_set_params(gv_unet* n, const float* d_in) {
   GV_CUDA(cudaMemsetAsync(n->net.m, 0, sizeof(float) * n->net.nparams, n->net.stream));
   GV_CUDA(cudaMemsetAsync(n->net.v, 0, sizeof(float) * n->net.nparams, n->net.stream));
   n->net.step = 0;
+  GV_TRY(n->net.pack());
   GV_CUDA(cudaStreamSynchronize(n->net.stream));
   return GV_OK;
 }
@@ -993,9 +1208,11 @@ gv_status gv_unet_loss_grad(gv_unet* n, const float* d_in, const float* d_target
   GV_TRY(check_batch(n, batch));
   if (!d_in || !d_target) return GV_ERR_INVALID;
   GV_TRY(n->net.forward(d_in, batch));
-  GV_TRY(n->net.loss(d_target, batch, true, loss));
+  GV_TRY(n->net.loss_launch(d_target, batch));
   GV_TRY(n->net.backward(batch));
-  return n->net.check();
+  GV_TRY(n->net.check());
+  if (loss) *loss = n->net.loss_value(batch);
+  return GV_OK;
 }
 
 gv_status gv_unet_train_step(gv_unet* n, const float* d_in, const float* d_target, int32_t batch,
@@ -1003,10 +1220,12 @@ gv_status gv_unet_train_step(gv_unet* n, const float* d_in, const float* d_targe
   GV_TRY(check_batch(n, batch));
   if (!d_in || !d_target) return GV_ERR_INVALID;
   GV_TRY(n->net.forward(d_in, batch));
-  GV_TRY(n->net.loss(d_target, batch, true, loss));
+  GV_TRY(n->net.loss_launch(d_target, batch));
   GV_TRY(n->net.backward(batch));
   GV_TRY(n->net.adam(lr));
-  return n->net.check();
+  GV_TRY(n->net.check());
+  if (loss) *loss = n->net.loss_value(batch);
+  return GV_OK;
 }
 
 gv_status gv_conv2d_forward(const float* x, const float* w, const float* bias, float* y,
@@ -1018,10 +1237,10 @@ gv_status gv_conv2d_forward(const float* x, const float* w, const float* bias, f
     return GV_ERR_INVALID;
   }
   uint32_t* err = nullptr;
-  GV_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
-  GV_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), (cudaStream_t)stream));
+  GV_CUDA(cudaMalloc(&err, 2 * sizeof(uint32_t)));
+  GV_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(uint32_t), (cudaStream_t)stream));
   const gv::cnn::Ctx c = standalone_ctx(stream, err, nullptr, 0);
-  gv_status s = gv::cnn::conv_forward(c, gv::cnn::View{(float*)x, Cin, 0}, w, bias,
+  gv_status s = gv::cnn::conv_forward(c, gv::cnn::View{(float*)x, Cin, 0}, w, nullptr, bias,
                                       gv::cnn::View{y, Cout, 0}, B, Cin, Cout, H, W, ks, relu);
   uint32_t e = 0;
   cudaMemcpyAsync(&e, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
@@ -1045,12 +1264,13 @@ gv_status gv_conv2d_backward(const float* x, const float* w, const float* dz, fl
   uint32_t* err = nullptr;
   float* part = nullptr;
   const size_t part_floats = (size_t)4 << 20;
-  GV_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
+  GV_CUDA(cudaMalloc(&err, 2 * sizeof(uint32_t)));
   GV_CUDA(cudaMalloc(&part, sizeof(float) * part_floats));
-  GV_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), (cudaStream_t)stream));
+  GV_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(uint32_t), (cudaStream_t)stream));
   const gv::cnn::Ctx c = standalone_ctx(stream, err, part, part_floats);
-  gv_status s = gv::cnn::conv_backward_data(c, gv::cnn::View{(float*)dz, Cout, 0}, w,
-                                            gv::cnn::View{dx, Cin, 0}, B, Cin, Cout, H, W, ks, 0);
+  gv_status s = gv::cnn::conv_backward_data(c, gv::cnn::View{(float*)dz, Cout, 0}, w, nullptr,
+                                            gv::cnn::View{dx, Cin, 0},
+                                            gv::cnn::View{nullptr, 0, 0}, B, Cin, Cout, H, W, ks);
   if (s == GV_OK)
     s = gv::cnn::conv_backward_weight(c, gv::cnn::View{(float*)x, Cin, 0},
                                       gv::cnn::View{(float*)dz, Cout, 0}, dw, db, B, Cin, Cout, H,
