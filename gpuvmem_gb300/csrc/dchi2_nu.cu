@@ -50,7 +50,7 @@ struct NuPlan {
   int pairs = 0;           // complex FFTs per channel
   int warps = 4;           // of a block of k_nu_spread
   float wmax = 0.0f;
-  int cmin = 0, ncol = 0;  // covered columns (signed)
+  int cmax = 0;            // covered columns: -cmax .. cmax
   int rmin = 0, nrow = 0;  // covered rows (signed)
   int wrap = 0;            // cells beyond +-N: the grid's period matters
   int tx0 = 0, ntx = 0, ty0 = 0, nty = 0;  // tiles in use
@@ -59,7 +59,7 @@ struct NuPlan {
   NuTask* d_tasks = nullptr;
   int* d_slot = nullptr;       // [C nty ntx] first task of each tile, or -1
   uint32_t* d_done = nullptr;  // [tasks] tasks of a tile done (at its first task)
-  float2* d_slots = nullptr;   // per task: [pair][plane][225] sums
+  float4* d_slots = nullptr;   // per task: [pair][225] sums {h+, h-}
   float2* d_H = nullptr;       // [channel of the group][pair][nrow][N]
   float2* d_twiddle = nullptr; // fft16_twiddles(log2 2N)
   float* d_corr = nullptr;     // [N] 1 / kernel transform
@@ -90,7 +90,7 @@ struct SpreadArgs {
   const NuTask* __restrict__ tasks;  // of the group
   int ntasks, t0;                    // t0: the group's first task
   uint32_t* __restrict__ done;
-  float2* slots;
+  float4* slots;
   int mode;        // of the DChi2 engines: 0/1 residuals, 2 Vo, 3 weights, 4 conjugated residuals
   int sh;          // fraction bits of a fixed-point position on the doubled grid
   float frac;      // 2^-sh
@@ -275,19 +275,18 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   if (cur >= 0) flush();
   __syncthreads();
   const int nw = (task.count + share - 1) / share;
-  float2* out = a.slots + (size_t)blockIdx.x * (NP * 2 * kTilePts);
-  for (int k = threadIdx.x; k < NP * kTilePts; k += 32 * kSpreadWarps) {
+  constexpr size_t kSlot = NP * kTilePts;
+  float4* out = a.slots + blockIdx.x * kSlot;
+  for (int k = threadIdx.x; k < (int)kSlot; k += 32 * kSpreadWarps) {
     float4 t = smem_f4[k];
     for (int w = 1; w < nw; w++) {
-      const float4 u = smem_f4[w * (NP * kTilePts) + k];
+      const float4 u = smem_f4[w * kSlot + k];
       t.x += u.x;
       t.y += u.y;
       t.z += u.z;
       t.w += u.w;
     }
-    const int q = k / kTilePts, o = k - q * kTilePts;
-    out[(2 * q) * kTilePts + o] = make_float2(t.x, t.y);
-    out[(2 * q + 1) * kTilePts + o] = make_float2(t.z, t.w);
+    out[k] = t;
   }
   if (task.pieces == 1) return;
   __shared__ int last_block;
@@ -300,35 +299,36 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   __syncthreads();
   if (!last_block) return;
   __threadfence();
-  constexpr size_t kSlot = NP * 2 * kTilePts;
-  float2* sum = a.slots + (size_t)(task.first - a.t0) * kSlot;
+  float4* sum = a.slots + (size_t)(task.first - a.t0) * kSlot;
   for (int k = threadIdx.x; k < (int)kSlot; k += 32 * kSpreadWarps) {
-    float2 t = __ldcg(sum + k);
+    float4 t = __ldcg(sum + k);
 #pragma unroll 8
     for (int w = 1; w < task.pieces; w++) {
-      const float2 u = __ldcg(sum + w * kSlot + k);
+      const float4 u = __ldcg(sum + w * kSlot + k);
       t.x += u.x;
       t.y += u.y;
+      t.z += u.z;
+      t.w += u.w;
     }
     sum[k] = t;
   }
 }
 
 struct RowArgs {
-  const float2* __restrict__ slots;
+  const float4* __restrict__ slots;
   const int* __restrict__ slot;
   const float2* __restrict__ tw;
   float2* __restrict__ H;
   int N, pairs, c0, t0;  // first channel and first task of the group
-  int lines;
-  int cmin, ncol, rmin, nrow, wrap;
+  int couples;           // (channel, pair, rows r and -r)
+  int cmax, rmin, nrow, wrap;
   int tx0, ntx, ty0, nty;
 };
 
 // The tiles over a row of the grid (two at most) and the row's place in them.
 struct RowTiles {
   const int* slot[2];
-  int at[2];  // first cell of the row in the tile's plane, or -1
+  int at[2];  // first cell of the row in the tile, or -1
 };
 
 __device__ __forceinline__ RowTiles row_tiles(const RowArgs& a, int ch, int r) {
@@ -344,60 +344,51 @@ __device__ __forceinline__ RowTiles row_tiles(const RowArgs& a, int ch, int r) {
   return t;
 }
 
-// Sum of a plane at column c of a row over the tiles that hold it, in order.
-__device__ __forceinline__ float2 plane_at(const RowArgs& a, const RowTiles& t, int plane, int c) {
-  float2 s = make_float2(0.0f, 0.0f);
+// The sums {h+, h-} of pair q at column c of a row over the tiles that hold
+// it, in order.
+__device__ __forceinline__ float4 cell_at(const RowArgs& a, const RowTiles& t, int q, int c) {
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const int cc = c + 3;
-  const float2* p[4];
+  const float4* p[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int tx = (cc >> 3) - (k & 1) - a.tx0, lx = (cc & 7) + 8 * (k & 1);
     int id = -1;
     if (cc >= 0 && lx < kTileSide && t.at[k >> 1] >= 0 && (unsigned)tx < (unsigned)a.ntx)
       id = __ldg(t.slot[k >> 1] + tx);
-    p[k] = id >= 0 ? a.slots + ((size_t)(id - a.t0) * a.pairs * 2 + plane) * kTilePts +
-                         t.at[k >> 1] + lx
+    p[k] = id >= 0 ? a.slots + ((size_t)(id - a.t0) * a.pairs + q) * kTilePts + t.at[k >> 1] + lx
                    : nullptr;
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     if (p[k]) {
-      const float2 v = __ldg(p[k]);
+      const float4 v = __ldg(p[k]);
       s.x += v.x;
       s.y += v.y;
+      s.z += v.z;
+      s.w += v.w;
     }
   }
   return s;
 }
 
-// The grid's value at (c, r): (h+ (c, r) + conj(h- (-c, -r))) / 2 with h+- the
-// sums of the even plus / minus the odd term, which is the Hermitian part of
-// the even term's grid plus the anti-Hermitian part of the odd one's.  The
-// sums lie in u >= 0, so away from u = 0 only one of the two is there.
-__device__ __forceinline__ float2 grid_at(const RowArgs& a, const RowTiles& up,
-                                          const RowTiles& down, int q, int c) {
-  float2 g = make_float2(0.0f, 0.0f);
-  if (c >= -3) {
-    const float2 p = plane_at(a, up, 2 * q, c);
-    g = make_float2(0.5f * p.x, 0.5f * p.y);
-  }
-  if (c <= 3) {
-    const float2 m = plane_at(a, down, 2 * q + 1, -c);
-    g.x = fmaf(0.5f, m.x, g.x);
-    g.y = fmaf(-0.5f, m.y, g.y);
-  }
-  return g;
-}
-
-// Rows of the doubled grid put together from the tiles and transformed over
-// its 2N cells, of which the N outputs about the
-// middle are kept: output x = j + r N / 8 of thread j is pixel x + N/2 for
-// r < 4 and x - 2N + N/2 for r >= 12, so pixel j + s N / 8 is r = s - 4 or
-// s + 12.  kLines rows per block.
+// Rows r and -r of the doubled grid put together from the tiles and
+// transformed over its 2N cells, of which the N outputs about the middle are
+// kept: output x = j + r N / 8 of thread j is pixel x + N/2 for r < 4 and
+// x - 2N + N/2 for r >= 12, so pixel j + s N / 8 is r = s - 4 or s + 12.
+//
+// The grid at (c, r) is (h+ (c, r) + conj(h- (-c, -r))) / 2, the Hermitian
+// part of the even term's grid plus the anti-Hermitian part of the odd one's;
+// the sums lie in u >= 0, so one cell of a tile feeds the two rows at c and
+// -c.  Taking the rows together looks every cell up and reads it once.
+// kPairs couples of rows per block.
 template <int LG>
 struct RowShape {
   static constexpr int kThreads = (1 << LG) / 16;  // per line
-  static constexpr int kLines = kThreads >= 128 ? 1 : 128 / kThreads;
+  static constexpr int kPairs = kThreads >= 64 ? 1 : 64 / kThreads;
+  static constexpr int kBlock = 2 * kPairs * kThreads;
+  static constexpr int kStride = span16(1 << LG);
+  static constexpr size_t kSmem = sizeof(float2) * (2 * kPairs * kStride + kPairs * 14);
 };
 
 __device__ __forceinline__ constexpr int kept_output(int s) {
@@ -405,24 +396,61 @@ __device__ __forceinline__ constexpr int kept_output(int s) {
 }
 
 template <int LG>
-__global__ void __launch_bounds__(RowShape<LG>::kThreads * RowShape<LG>::kLines)
+__global__ void __launch_bounds__(RowShape<LG>::kBlock, 1024 / RowShape<LG>::kBlock)
     k_nu_rows(RowArgs a) {
-  constexpr int n = 1 << LG, N = n / 2, T = RowShape<LG>::kThreads, L = RowShape<LG>::kLines;
+  using S = RowShape<LG>;
+  constexpr int n = 1 << LG, N = n / 2, T = S::kThreads;
   extern __shared__ float2 smem_f2[];
-  const int j = threadIdx.x % T, l = threadIdx.x / T;
-  const int line = blockIdx.x * L + l;
-  const bool in = line < a.lines;
-  const int plane = in ? line / a.nrow : 0, r = a.rmin + (in ? line - plane * a.nrow : 0);
+  const int j = threadIdx.x % T, l = threadIdx.x / T;  // this thread's line: l & 1 of couple l / 2
+  float2* buf = smem_f2 + l * S::kStride;
+  const int couple = blockIdx.x * S::kPairs + (l >> 1);
+  const bool in = couple < a.couples;
+  // couple k of a plane: rows k and -k; 0 alone, or with -N where all rows are there
+  const int per = a.wrap ? N : a.nrow / 2 + 1;
+  const int plane = in ? couple / per : 0, k = in ? couple - plane * per : 0;
   const int ch = a.c0 + plane / a.pairs, q = plane % a.pairs;
+  const int r = (l & 1) ? (k ? -k : -N) : k;
+  const bool mine = in && (k > 0 || !(l & 1) || a.wrap);
   float2 v[16];
   if (!a.wrap) {
-    const RowTiles up = row_tiles(a, ch, r), down = row_tiles(a, ch, -r);
-#pragma unroll
-    for (int e = 0; e < 16; e++) {
-      const int c = e < 8 ? j + e * T : j + e * T - n;
-      v[e] = in && (unsigned)(c - a.cmin) < (unsigned)a.ncol ? grid_at(a, up, down, q, c)
-                                                            : make_float2(0.0f, 0.0f);
+    // both lines' covered columns in the couple's two buffers (position c of
+    // the transform), and h- of columns -3 .. 3, which meet h+ there
+    float2* line0 = smem_f2 + (l & ~1) * S::kStride;
+    float2* line1 = line0 + S::kStride;
+    float2* near = smem_f2 + 2 * S::kPairs * S::kStride + (l >> 1) * 14;
+    const int t = threadIdx.x % (2 * T);
+    for (int p = t; p < n; p += 2 * T) line0[p] = line1[p] = make_float2(0.0f, 0.0f);
+    __syncthreads();
+    if (in) {
+      const int count = a.cmax + 4;  // columns -3 .. cmax of rows k, then of rows -k
+#pragma unroll 1
+      for (int side = 0; side < (k ? 2 : 1); side++) {
+        const RowTiles tiles = row_tiles(a, ch, side ? -k : k);
+        float2* to = side ? line1 : line0;       // h+ at (c, r)
+        float2* mirror = k ? (side ? line0 : line1) : line0;  // h- at (-c, -r)
+        for (int i = t; i < count; i += 2 * T) {
+          const int c = i - 3;
+          const float4 g = cell_at(a, tiles, q, c);
+          to[c & (n - 1)] = make_float2(0.5f * g.x, 0.5f * g.y);
+          const float2 m = make_float2(0.5f * g.z, -0.5f * g.w);
+          if (c > 3) mirror[-c & (n - 1)] = m;
+          else near[side * 7 + i] = m;
+        }
+      }
     }
+    __syncthreads();
+    for (int i = t; in && i < (k ? 14 : 7); i += 2 * T) {
+      const int side = i / 7, c = 3 - i % 7;  // h- of column -c
+      float2* to = k ? (side ? line0 : line1) : line0;
+      float2 g = to[c & (n - 1)];
+      g.x += near[i].x;
+      g.y += near[i].y;
+      to[c & (n - 1)] = g;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; e++) v[e] = buf[j + e * T];
+    __syncthreads();
   } else {
     // footprints that reach over the grid's edge come back at the other side
 #pragma unroll
@@ -434,17 +462,24 @@ __global__ void __launch_bounds__(RowShape<LG>::kThreads * RowShape<LG>::kLines)
 #pragma unroll
           for (int e = 0; e < 16; e++) {
             const int c = (e < 8 ? j + e * T : j + e * T - n) + wx * n;
-            const float2 g = grid_at(a, up, down, q, c);
-            v[e].x += g.x;
-            v[e].y += g.y;
+            if (c >= -3) {
+              const float4 g = cell_at(a, up, q, c);
+              v[e].x = fmaf(0.5f, g.x, v[e].x);
+              v[e].y = fmaf(0.5f, g.y, v[e].y);
+            }
+            if (c <= 3) {
+              const float4 g = cell_at(a, down, q, -c);
+              v[e].x = fmaf(0.5f, g.z, v[e].x);
+              v[e].y = fmaf(-0.5f, g.w, v[e].y);
+            }
           }
         }
       }
     }
   }
-  fft16<LG>(v, smem_f2 + l * span16(n), j, a.tw);
-  if (!in) return;
-  float2* h = a.H + (size_t)line * N;
+  fft16<LG>(v, buf, j, a.tw);
+  if (!mine) return;
+  float2* h = a.H + ((size_t)plane * a.nrow + r - a.rmin) * N;
 #pragma unroll
   for (int s = 0; s < 8; s++) h[j + s * T] = v[kept_output(s)];
 }
@@ -767,12 +802,11 @@ gv_status spread(const SpreadArgs& a, int warps, cudaStream_t st) {
 
 template <int LG>
 gv_status transforms(Problem& P, const RowArgs& ra, const ColArgs& ca) {
-  constexpr int L = RowShape<LG>::kLines;
-  const size_t smem = sizeof(float2) * L * span16(1 << LG);
-  if (smem > 48 * 1024)
+  using R = RowShape<LG>;
+  if (R::kSmem > 48 * 1024)
     GV_CUDA(cudaFuncSetAttribute(k_nu_rows<LG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  k_nu_rows<LG><<<(ra.lines + L - 1) / L, RowShape<LG>::kThreads * L, smem, P.stream>>>(ra);
+                                 (int)R::kSmem));
+  k_nu_rows<LG><<<(ra.couples + R::kPairs - 1) / R::kPairs, R::kBlock, R::kSmem, P.stream>>>(ra);
   GV_LAUNCH("k_nu_rows");
   GV_TRY(side_joined(P));  // the priors' gradient is where the sums are added
   using S = ColShape<LG>;
@@ -914,8 +948,7 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   const int cmax = 8 * txb + 11, rlo = 8 * tya - N - 3, rhi = 8 * tyb - N + 11;
   const int rmax = std::max(rhi, -rlo);
   n->wrap = cmax > N - 1 || rmax > N - 1;
-  n->cmin = n->wrap ? -N : -cmax;
-  n->ncol = n->wrap ? 2 * N : 2 * cmax + 1;
+  n->cmax = cmax;
   n->rmin = n->wrap ? -N : -rmax;
   n->nrow = n->wrap ? 2 * N : 2 * rmax + 1;
   // ---- tasks ------------------------------------------------------------------
@@ -947,7 +980,7 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   }
   for (int c = 0; c < C; c++) n->task_off[c + 1] += n->task_off[c];
   // ---- channel groups whose workspace stays bounded ------------------------------
-  const size_t slot_b = sizeof(float2) * 2 * kTilePts * pairs;
+  const size_t slot_b = sizeof(float4) * kTilePts * pairs;
   const size_t h_b = sizeof(float2) * (size_t)pairs * n->nrow * N;
   const size_t fac_b = sizeof(float) * (size_t)N * N;
   n->groups.push_back(0);
@@ -1030,8 +1063,7 @@ gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result
   ra.H = n.d_H;
   ra.N = N;
   ra.pairs = np;
-  ra.cmin = n.cmin;
-  ra.ncol = n.ncol;
+  ra.cmax = n.cmax;
   ra.rmin = n.rmin;
   ra.nrow = n.nrow;
   ra.wrap = n.wrap;
@@ -1073,7 +1105,7 @@ gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result
     }
     ra.c0 = c0;
     ra.t0 = t0;
-    ra.lines = nch * np * n.nrow;
+    ra.couples = nch * np * (n.wrap ? N : n.nrow / 2 + 1);
     ca.nchan = nch;
     ca.fac = mode <= 1 ? n.d_fac + c0 * MN : nullptr;
     ca.chfreq = P.d_chfreq + c0;

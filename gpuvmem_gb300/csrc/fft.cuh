@@ -273,27 +273,37 @@ __device__ __forceinline__ void fft16(float2 (&v)[16], float2* buf, int j,
       for (int r = 0; r < R0; r++) v[m + r * M0] = u[r];
     }
   }
-  // y[R0 (j + m T) + r] of item m
+  // y[R0 (j + m T) + r] of item m.  Written as one padded position and
+  // constants (r < R0 never carries into the padding's multiple of 16), here
+  // and below: the compiler does not see through the shift
+  constexpr bool kWide = (R0 * T) % 16 == 0;
+  {
+    float2* y = buf + pad16(R0 * j);
 #pragma unroll
-  for (int m = 0; m < M0; m++)
+    for (int m = 0; m < M0; m++)
 #pragma unroll
-    for (int r = 0; r < R0; r++)
-      buf[pad16(R0 * (j + m * T) + r)] = v[m + brev_c<L0>(r) * M0];
+      for (int r = 0; r < R0; r++) {
+        const float2 x = v[m + brev_c<L0>(r) * M0];
+        if constexpr (kWide) y[m * span16(R0 * T) + r] = x;
+        else buf[pad16(R0 * (j + m * T) + r)] = x;
+      }
+  }
 #pragma unroll
   for (int l = L0; l < LG; l += 4) {
     const int k = j & ((1 << l) - 1);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 16; r++) v[r] = buf[pad16(j + r * T)];
+    for (int r = 0; r < 16; r++)
+      v[r] = T % 16 == 0 ? buf[pad16(j) + r * span16(T)] : buf[pad16(j + r * T)];
 #pragma unroll
     for (int r = 1; r < 16; r++) v[r] = cmul(v[r], __ldg(tw + ((r - 1) << l) + k));
     tw += 15 << l;
     dft16(v);
     if (l + 4 < LG) {
       __syncthreads();
-      const int base = ((j >> l) << (l + 4)) + k;
+      float2* y = buf + pad16(((j >> l) << (l + 4)) + k);
 #pragma unroll
-      for (int r = 0; r < 16; r++) buf[pad16(base + (r << l))] = v[brev_c<4>(r)];
+      for (int r = 0; r < 16; r++) y[(r << l) + ((r << l) >> 4)] = v[brev_c<4>(r)];
     }
   }
 }
