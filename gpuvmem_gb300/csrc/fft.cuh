@@ -161,13 +161,25 @@ template <int LG, int L>
 __device__ __forceinline__ void fft8_passes(float2 (&v)[8], float2* buf, int j,
                                             const float2* __restrict__ tw) {
   constexpr int T = (1 << LG) / 8, LR = fft8_radix(LG, L), R = 1 << LR, M = 8 / R;
-  // the last pass' results: element ((j >> L - 3) << L) + k + r 2^(L - 3)
+  // the last pass' results: element ((j >> L - 3) << L) + k + r 2^(L - 3),
+  // then elements j + e T of the next.  Each exchange has the padding that
+  // puts the writes of a half warp into distinct banks and leaves the reads of
+  // 16 neighbours together: one position in 16 after the first pass (writes 8
+  // apart), 8 in 64 after the second (runs of 8, 64 apart), none after that.
+  // (One in 8 throughout made every read a bank conflict; the row pass runs
+  // its data pipe at three quarters of its rate.)
   const int kw = j & ((1 << (L - 3)) - 1), base = ((j >> (L - 3)) << L) + kw;
+  auto place = [](int e) { return L == 3 ? e + (e >> 4) : (L == 6 ? e + 8 * (e >> 6) : e); };
+  constexpr int kStep = 1 << (L - 3);
+  // base + r kStep stays in base's group of the padding
+  float2* y = buf + place(base);
 #pragma unroll
-  for (int r = 0; r < 8; r++) buf[fpad(base + (r << (L - 3)))] = v[brev_c<3>(r)];
+  for (int r = 0; r < 8; r++) y[r * kStep] = v[brev_c<3>(r)];
   __syncthreads();
+  constexpr int kGroup = L == 3 ? 16 : (L == 6 ? 64 : 1);
 #pragma unroll
-  for (int e = 0; e < 8; e++) v[e] = buf[fpad(j + e * T)];
+  for (int e = 0; e < 8; e++)
+    v[e] = T % kGroup == 0 ? buf[place(j) + e * place(T)] : buf[place(j + e * T)];
   if constexpr (LR == 3) {
     const int k = j & ((1 << L) - 1);
 #pragma unroll
