@@ -12,7 +12,7 @@
 // The operand tiles are staged by the CTA's threads straight from the FP32
 // NCHW activations (im2col on the fly, rounded to BF16) into 128-byte
 // swizzled MN-major shared-memory tiles; one thread issues the MMAs; two
-// stages alternate.  The epilogue (bias, ReLU, layout) is applied on the way
+// stages alternate, the next chunk's loads under way.  The epilogue (bias, ReLU, layout) is applied on the way
 // out of TMEM.  Pooling, upsampling, the loss and Adam are plain
 // bandwidth-bound kernels.
 //
@@ -38,7 +38,8 @@ namespace cnn {
 using namespace gv::tc;
 
 // ---------------------------------------------------------------- GEMM core
-constexpr int kBM = 128, kBK = 64, kGemmThreads = 256;
+// 11 warps: with 3 x 3 taps the eight-pixel groups of an A tile are 352 loads
+constexpr int kBM = 128, kBK = 64, kGemmThreads = 352;
 
 __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
@@ -66,64 +67,169 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
                     bf16x2(v[6], v[7]));
 }
 
-// Eight neighbours of an image row, columns x + dx .. x + dx + 7 (|dx| <= 1,
-// zero outside the row of W): `p` points at column x, 16-byte aligned, x and
-// W multiples of 8.  Two 16-byte loads and at most one more, where eight
-// loads one by one set the pace of the GEMMs' staging.
-__device__ __forceinline__ void row8(const float* __restrict__ p, int x, int dx, int W,
-                                     float (&v)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-  const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  if (dx == 0) {
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else if (dx > 0) {
-    v[0] = a.y; v[1] = a.z; v[2] = a.w; v[3] = b.x;
-    v[4] = b.y; v[5] = b.z; v[6] = b.w;
-    v[7] = x + 8 < W ? __ldg(p + 8) : 0.0f;
-  } else {
-    v[0] = x > 0 ? __ldg(p - 1) : 0.0f;
-    v[1] = a.x; v[2] = a.y; v[3] = a.z; v[4] = a.w;
-    v[5] = b.x; v[6] = b.y; v[7] = b.z;
+// Eight pixels of an image row (16-byte aligned) and the ones beside them.
+struct Row {
+  float4 a, b;
+  float l, r;  // zero outside the row
+  __device__ __forceinline__ void clear() {
+    a = b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    l = r = 0.0f;
   }
-}
+  template <bool kEnds>
+  __device__ __forceinline__ void load(const float* __restrict__ p, int x, int W) {
+    a = __ldg(reinterpret_cast<const float4*>(p));
+    b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    if (kEnds) {
+      l = x > 0 ? __ldg(p - 1) : 0.0f;
+      r = x + 8 < W ? __ldg(p + 8) : 0.0f;
+    }
+  }
+  __device__ __forceinline__ uint4 centre() const {
+    return make_uint4(bf16x2(a.x, a.y), bf16x2(a.z, a.w), bf16x2(b.x, b.y), bf16x2(b.z, b.w));
+  }
+  // the row one to the left, as it is and one to the right
+  __device__ __forceinline__ void shifted(uint4 (&v)[3]) const {
+    const uint32_t w1 = bf16x2(a.y, a.z), w2 = bf16x2(a.w, b.x), w3 = bf16x2(b.y, b.z);
+    v[0] = make_uint4(bf16x2(l, a.x), w1, w2, w3);
+    v[1] = centre();
+    v[2] = make_uint4(w1, w2, w3, bf16x2(b.w, r));
+  }
+};
 
 // D[m][n] = sum_k A[m][k] B[k][n] over this CTA's K range; op.a(m,k),
-// op.b(k,n) fetch FP32 operands, op.store(m, n, v, split) writes a result.
-// How the tiles are staged (op.fast: aligned tensors whose rows are multiples
-// of eight pixels; otherwise, and at ragged edges, element by element):
-//   Op::kPixelRows  the rows of A are pixels (forward, data gradient): a
-//                   thread keeps its eight pixels and takes the taps' offsets
-//                   from a table made once per chunk; B is the weights, which
-//                   op.packed holds as ready BF16 tile images;
-//   otherwise       the columns of A and B are pixels (weight gradient): both
-//                   tiles K-major, so that eight neighbours of a row are one
-//                   16-byte store; a thread keeps its row's channel and tap.
-template <class Op, int BN>
-__global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int K, int klen,
-                                                       uint32_t* err) {
+// op.b(k,n) fetch FP32 operands, op.store(row, n, count, v, split) writes up to
+// eight columns of a result.
+//
+// KS (3 or 1: the taps of a row; tensors aligned, rows multiples of eight
+// pixels) stages the tiles in groups of eight pixels; KS = 0 element by
+// element.  What bounds the network's GEMMs is the way from one chunk of 64 k
+// to the next (few chunks or few CTAs each, MMAs of well under a microsecond),
+// so a chunk's loads are issued before the last one's MMAs, into registers,
+// and cost little:
+//   A  a row of the tile is a channel and a tap.  The three taps of an image
+//      row are one load of the group and its two neighbours, rounded once and
+//      stored three times: 22 such units x 16 groups where the rows are k
+//      (Op::kPixelRows: forward, data gradient; MN-major), 44 x 8 where they
+//      are m (weight gradient; K-major), one a thread.  Neighbouring threads
+//      take neighbouring groups: with a row a thread, as this was first, each
+//      load of the weight gradient touched 32 lines.
+//   B  the weights as ready BF16 tile images (op.packed), or the gradient.
+// Bound by the instructions (two thirds of the issue slots at
+// the shallow levels).  The network of 256^2, 16 channels, 5 levels, with this
+// staging, the epilogue's eight columns and the narrower tiles: a training step
+// of batch 8 5310 -> 2670 us, a forward pass of one sky 342 -> 224.  One CTA
+// for several row tiles, with the next one's loads under the last one's
+// epilogue, gave nothing (236 -> 244).
+template <class Op, int BN, int KS>
+__global__ void __launch_bounds__(kGemmThreads, Op::kPixelRows && BN == 64 ? 3 : (BN < 256 ? 2 : 1))
+    k_gemm(Op op, int M, int N, int K, int klen, uint32_t* err) {
   using L = GemmLayout<BN>;
+  constexpr int T = kGemmThreads;
+  constexpr bool kRows = Op::kPixelRows;
+  constexpr bool kmajor = !kRows && KS > 0;
+  constexpr int kGroups = kRows ? kBM / 8 : kBK / 8;  // of eight pixels
+  constexpr int kRowsA = kRows ? kBK : kBM;
+  constexpr int kUnits = KS == 3 ? (kRowsA + 4) / 3 : kRowsA;
+  constexpr int kLoadsA = KS > 0 ? (kUnits * kGroups + T - 1) / T : 1;
+  constexpr int kLoadsB = KS == 0 ? 1 : kRows ? ((int)(L::kTileB / 16) + T - 1) / T
+                                              : (BN * kGroups + T - 1) / T;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   __shared__ uint64_t bar[2];
   __shared__ uint32_t tslot;
   __shared__ int s_abort;
-  __shared__ int4 tab[2][kBK];  // the chunk's taps, or its groups of eight pixels
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
   const int kbeg = blockIdx.z * klen;
   const int kend = min(K, kbeg + klen);
   const int nch = kend > kbeg ? (kend - kbeg + kBK - 1) / kBK : 0;
-  const bool fast = op.fast;
-  auto make_table = [&](int c) {
+
+  const int grp = tid % kGroups;  // T is a multiple of both
+  int4 at = make_int4(0, 0, 0, 0);  // the group's {offset, y, x, batch}
+  const int mg = m0 + grp * 8;
+  if (KS > 0 && kRows && mg < M) at = op.pixel(mg);  // M is a multiple of eight
+  // the first unit that touches the tile's rows from row0 on
+  auto unit = [&](int row0, int i) {
+    return (KS == 3 ? row0 / 3 : row0) + (tid + i * T) / kGroups;
+  };
+  // B's tile images: 64 columns each, the 8-row atoms of a wider tile side by side
+  constexpr int kAtoms = BN / 64, kImage = kBK * 64 / 8;  // uint4 of an image
+  auto image = [&](int c, int e) {
+    const int atom = e >> 6;
+    return op.packed + ((size_t)(blockIdx.y * kAtoms + atom % kAtoms) * ((K + kBK - 1) / kBK) +
+                        (kbeg / kBK + c)) * kImage + (atom / kAtoms) * 64 + (e & 63);
+  };
+  Row ra[kLoadsA];
+  Row rb[kmajor ? kLoadsB : 1];
+  uint4 rw[kRows ? kLoadsB : 1];
+  auto load = [&](int c) {
     const int k0 = kbeg + c * kBK;
-    if (Op::kPixelRows) {
-      if (tid < kBK) tab[c & 1][tid] = k0 + tid < kend ? op.tap(k0 + tid) : make_int4(0, 2, 0, 0);
-    } else {
-      if (tid < kBK / 8) tab[c & 1][tid] = op.pixel(k0 + 8 * tid);
+    const int rows = kRows ? K : M;
+    const bool in = kRows ? mg < M : k0 + 8 * grp < kend;
+    if (!kRows && in) at = op.pixel(k0 + 8 * grp);
+#pragma unroll
+    for (int i = 0; i < kLoadsA; i++) {
+      ra[i].clear();
+      const int u = unit(kRows ? k0 : m0, i), ch = KS == 3 ? u / 3 : u;
+      int dy = KS == 3 ? u - 3 * ch - 1 : 0;
+      if (Op::kFlip) dy = -dy;
+      if (in && tid + i * T < kUnits * kGroups && u * max(KS, 1) < rows &&
+          (unsigned)(at.y + dy) < (unsigned)op.H)
+        ra[i].template load<KS == 3>(op.src() + at.x + ch * op.H * op.W + dy * op.W, at.z, op.W);
+    }
+    if constexpr (kmajor) {
+#pragma unroll
+      for (int i = 0; i < kLoadsB; i++) {
+        rb[i].clear();
+        const int r = (tid + i * T) / kGroups;
+        if (in && r < BN && n0 + r < N)
+          rb[i].template load<false>(op.grad_row(n0 + r, at), at.z, op.W);
+      }
+    } else if (kRows) {
+      if (op.packed) {
+#pragma unroll
+        for (int i = 0; i < kLoadsB; i++)
+          if (tid + i * T < (int)(L::kTileB / 16)) rw[i] = __ldg(image(c, tid + i * T));
+      }
     }
   };
+  auto put = [&](int c, uint8_t* sa, uint8_t* sb) {
+    const int row0 = kRows ? kbeg + c * kBK : m0;
+#pragma unroll
+    for (int i = 0; i < kLoadsA; i++) {
+      if (tid + i * T >= kUnits * kGroups) break;
+      uint4 v[3];
+      if (KS == 3) ra[i].shifted(v);
+      else v[0] = ra[i].centre();
+      const int r0 = unit(row0, i) * KS - row0;
+#pragma unroll
+      for (int j = 0; j < KS; j++) {
+        const int r = r0 + j;
+        if (r < 0 || r >= kRowsA) continue;
+        const uint32_t off = kRows ? tile_off(grp >> 3, grp & 7, r, L::kSboA) : kmajor_off(r, grp);
+        *reinterpret_cast<uint4*>(sa + off) = v[Op::kFlip && KS == 3 ? 2 - j : j];
+      }
+    }
+    if constexpr (kmajor) {
+#pragma unroll
+      for (int i = 0; i < kLoadsB; i++) {
+        const int r = (tid + i * T) / kGroups;
+        // beyond the last column: zeros, once in each stage
+        if (r < BN && (n0 + r < N || c < 2))
+          *reinterpret_cast<uint4*>(sb + kmajor_off(r, grp)) = rb[i].centre();
+      }
+    } else if (kRows) {
+      if (op.packed) {
+#pragma unroll
+        for (int i = 0; i < kLoadsB; i++)
+          if (tid + i * T < (int)(L::kTileB / 16))
+            reinterpret_cast<uint4*>(sb)[tid + i * T] = rw[i];
+      }
+    }
+  };
+  if (KS > 0 && nch > 0) load(0);
+
   if (warp == 0) {
     tmem_alloc<false>(&tslot, BN);
     tmem_relinquish<false>();
@@ -134,61 +240,25 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (fast && nch > 0) make_table(0);
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tacc = tslot;
-  // this thread's pixels (rows m0 + 8 (tid & 15) ...) or row
-  const int mg = m0 + (tid & 15) * 8;
-  const bool mine = Op::kPixelRows ? mg + 7 < M : m0 + (tid & 127) < M;
-  const int4 at = !fast || !mine ? make_int4(0, 0, 0, 0)
-                  : Op::kPixelRows ? op.pixel(mg)
-                                   : op.tap(m0 + (tid & 127));
-  const bool kmajor = !Op::kPixelRows && fast;
   const uint32_t idesc = kmajor ? make_idesc_bf16(kBM, BN) & ~((1u << 15) | (1u << 16))
                                 : make_idesc_bf16(kBM, BN);
   bool ok = true;
   for (int c = 0; c < nch; c++) {
     const int st = c & 1;
-    // the MMAs that read this stage two chunks ago are done
-    if (c >= 2) ok = warp_wait(&bar[st], ((c >> 1) - 1) & 1, &s_abort, err, 11u);
-    if (!__syncthreads_and(ok ? 1 : 0)) {
-      ok = false;
-      break;
-    }
     uint8_t* sa = base + st * L::kStage;
     uint8_t* sb = sa + L::kTileA;
     const int k0 = kbeg + c * kBK;
-    if (Op::kPixelRows && fast) {
-#pragma unroll
-      for (int i = 0; i < kBK / 16; i++) {
-        const int kk = (tid >> 4) + 16 * i;
-        const int4 t = tab[st][kk];
-        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (mine) {
-          if (t.y != 2 && (unsigned)(at.y + t.y) < (unsigned)op.H)
-            row8(op.src() + at.x + t.x, at.z, t.z, op.W, v);
-        } else if (k0 + kk < kend) {
-#pragma unroll
-          for (int j = 0; j < 8; j++)
-            if (mg + j < M) v[j] = op.a(mg + j, k0 + kk);
-        }
-        *reinterpret_cast<uint4*>(sa + tile_off((tid & 15) >> 3, tid & 7, kk, L::kSboA)) = pack8(v);
-      }
-    } else if (kmajor) {
-      const int r = tid & 127;
-#pragma unroll
-      for (int i = 0; i < kBK / 16; i++) {
-        const int g = (tid >> 7) + 2 * i;
-        const int4 p = tab[st][g];  // {offset of the pixels in a plane set, y, x, batch}
-        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (mine && k0 + 8 * g < kend && (unsigned)(p.y + at.y) < (unsigned)op.H)
-          row8(op.src() + p.x + at.x, p.z, at.z, op.W, v);
-        *reinterpret_cast<uint4*>(sa + kmajor_off(r, g)) = pack8(v);
-      }
+    // the MMAs that read this stage two chunks ago are done
+    if (c >= 2) ok = warp_wait(&bar[st], ((c >> 1) - 1) & 1, &s_abort, err, 11u);
+    if constexpr (KS > 0) {
+      put(c, sa, sb);
+      if (c + 1 < nch) load(c + 1);
     } else {
-      for (int idx = tid; idx < (kBM / 8) * kBK; idx += kGemmThreads) {
+      for (int idx = tid; idx < (kBM / 8) * kBK; idx += T) {
         const int og = idx & (kBM / 8 - 1), kk = idx / (kBM / 8);
         const int k = k0 + kk;
         float v[8];
@@ -200,24 +270,11 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
         *reinterpret_cast<uint4*>(sa + tile_off(og >> 3, og & 7, kk, L::kSboA)) = pack8(v);
       }
     }
-    if (Op::kPixelRows && op.packed) {
-      // the tile image as it lies in shared memory
-      const uint4* src = op.packed + ((size_t)blockIdx.y * ((K + kBK - 1) / kBK) + k0 / kBK) *
-                                         (L::kTileB / 16);
-#pragma unroll
-      for (int i = 0; i < (int)(L::kTileB / 16) / kGemmThreads; i++)
-        reinterpret_cast<uint4*>(sb)[tid + i * kGemmThreads] = __ldg(src + tid + i * kGemmThreads);
-    } else if (kmajor) {
-#pragma unroll
-      for (int i = 0; i < (BN / 8) * kBK / kGemmThreads; i++) {
-        const int r = tid % BN, g = tid / BN + (kGemmThreads / BN) * i;
-        const int4 p = tab[st][g];
-        float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        if (n0 + r < N && k0 + 8 * g < kend) row8(op.grad_row(n0 + r, p), p.z, 0, op.W, v);
-        *reinterpret_cast<uint4*>(sb + kmajor_off(r, g)) = pack8(v);
-      }
-    } else {
-      for (int idx = tid; idx < (BN / 8) * kBK; idx += kGemmThreads) {
+    if (KS == 0 && op.packed) {
+      for (int i = tid; i < (int)(L::kTileB / 16); i += T)
+        reinterpret_cast<uint4*>(sb)[i] = __ldg(image(c, i));
+    } else if (!kmajor && !op.packed) {
+      for (int idx = tid; idx < (BN / 8) * kBK; idx += T) {
         const int og = idx % (BN / 8), kk = idx / (BN / 8);
         const int k = k0 + kk;
         float v[8];
@@ -229,9 +286,11 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
         *reinterpret_cast<uint4*>(sb + tile_off(og >> 3, og & 7, kk, L::kSboB)) = pack8(v);
       }
     }
-    if (fast && c + 1 < nch) make_table(c + 1);
     fence_proxy_async();
-    __syncthreads();
+    if (!__syncthreads_and(ok ? 1 : 0)) {
+      ok = false;
+      break;
+    }
     if (tid == 0) {
       fence_after();
       const uint32_t aa = smem_u32(sa), ba = smem_u32(sb);
@@ -250,27 +309,19 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(Op op, int M, int N, int 
     const int c = nch - 1;
     ok = warp_wait(&bar[c & 1], (c >> 1) & 1, &s_abort, err, 12u);
   }
-  if (__syncthreads_and(ok ? 1 : 0)) {
+  if (__syncthreads_and(ok ? 1 : 0) && warp < 8) {
     fence_after();
     const int q = warp & 3, h = warp >> 2;
     const int m = m0 + 32 * q + lane;
+    // eight columns at a time, the two halves of the warps in turn: all of them
+    // have work at 16 columns, and what a column needs is loaded before the
+    // stores, which the loads could not pass
+    const int cols = min(BN, N - n0);
 #pragma unroll 1
-    for (int cb = h * (BN / 2); cb < (h + 1) * (BN / 2) && n0 + cb < N; cb += 32) {
-      float v[32];
-      if (nch > 0) {
-        tmem_ld32(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)cb, v);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = 0.0f;
-      }
-      if (m < M) {
-        const auto at_m = op.row(m);
-#pragma unroll 4
-        for (int j = 0; j < 32; j++) {
-          const int n = n0 + cb + j;
-          if (n < N) op.store(at_m, n, v[j], (int)blockIdx.z);
-        }
-      }
+    for (int cb = 8 * h; cb < cols; cb += 16) {
+      float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      if (nch > 0) tmem_ld8(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)cb, v);
+      if (m < M) op.store(op.row(m), n0 + cb, min(8, cols - cb), v, (int)blockIdx.z);
     }
   }
   fence_before();
@@ -295,6 +346,7 @@ __device__ __host__ inline bool rows_of_eight(const float* p, int W) {
 // the splits, the bias and the activation
 struct ConvFwdOp {
   static constexpr bool kPixelRows = true;
+  static constexpr bool kFlip = false;
   const float* x;
   int xC, xc0;
   const float* w;
@@ -313,12 +365,6 @@ struct ConvFwdOp {
     const int b = m / HW, r = m - b * HW, y0 = r / W;
     return make_int4((b * xC + xc0) * HW + r, y0, r - y0 * W, 0);
   }
-  // a row of the weights: {offset of its channel and row, dy, dx}
-  __device__ int4 tap(int k) const {
-    const int kk = ks * ks, cin = k / kk, t = k - cin * kk;
-    const int dy = t / ks - ks / 2, dx = t % ks - ks / 2;
-    return make_int4(cin * H * W + dy * W, dy, dx, 0);
-  }
   __device__ float a(int m, int k) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW, y0 = r / W, x0 = r - y0 * W;
@@ -335,14 +381,20 @@ struct ConvFwdOp {
     const int b = m / HW, r = m - b * HW;
     return make_int2(m, (b * yC + yc0) * HW + r);
   }
-  __device__ void store(const int2& at, int n, float v, int split) const {
-    if (part) {
-      part[((size_t)split * Cout + n) * M + at.x] = v;
-      return;
+  __device__ void store(const int2& at, int n, int cnt, float (&v)[8], int split) const {
+    float* out = part ? part + ((size_t)split * Cout + n) * M + at.x
+                      : y + (size_t)at.y + (size_t)n * H * W;
+    const size_t step = part ? (size_t)M : (size_t)H * W;
+    if (!part) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        if (j < cnt) v[j] += __ldg(bias + n + j);
+        if (relu) v[j] = fmaxf(v[j], 0.0f);
+      }
     }
-    v += bias[n];
-    if (relu) v = fmaxf(v, 0.0f);
-    y[(size_t)at.y + (size_t)n * H * W] = v;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (j < cnt) out[j * step] = v[j];
   }
 };
 
@@ -365,6 +417,7 @@ __global__ void k_conv_fwd_finish(int M, int N, int nsplit, const float* __restr
 // activation whose gradient dx is) masked by its ReLU
 struct ConvBwdDataOp {
   static constexpr bool kPixelRows = true;
+  static constexpr bool kFlip = true;  // the taps run backwards
   const float* dz;
   int zC, zc0;
   const float* w;
@@ -380,11 +433,6 @@ struct ConvBwdDataOp {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW, y0 = r / W;
     return make_int4((b * zC + zc0) * HW + r, y0, r - y0 * W, 0);
-  }
-  __device__ int4 tap(int k) const {
-    const int kk = ks * ks, co = k / kk, t = k - co * kk;
-    const int dy = ks / 2 - t / ks, dx = ks / 2 - t % ks;
-    return make_int4(co * H * W + dy * W, dy, dx, 0);
   }
   __device__ float a(int m, int k) const {
     const int HW = H * W;
@@ -404,10 +452,18 @@ struct ConvBwdDataOp {
     const int b = m / HW;
     return make_int2(b, m - b * HW);
   }
-  __device__ void store(const int2& at, int n, float v, int) const {
+  __device__ void store(const int2& at, int n, int cnt, float (&v)[8], int) const {
     const int HW = H * W;
-    if (act && !(act[(size_t)(at.x * aC + ac0 + n) * HW + at.y] > 0.0f)) v = 0.0f;
-    dx[(size_t)(at.x * xC + xc0 + n) * HW + at.y] = v;
+    if (act) {
+      const float* a = act + (size_t)(at.x * aC + ac0 + n) * HW + at.y;
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        if (j < cnt && !(__ldg(a + (size_t)j * HW) > 0.0f)) v[j] = 0.0f;
+    }
+    float* out = dx + (size_t)(at.x * xC + xc0 + n) * HW + at.y;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (j < cnt) out[(size_t)j * HW] = v[j];
   }
 };
 
@@ -415,6 +471,7 @@ struct ConvBwdDataOp {
 // pixels of dz * x (shifted)
 struct ConvBwdWeightOp {
   static constexpr bool kPixelRows = false;
+  static constexpr bool kFlip = false;
   const float* x;
   int xC, xc0;
   const float* dz;
@@ -429,11 +486,6 @@ struct ConvBwdWeightOp {
     const int HW = H * W;
     const int b = k / HW, r = k - b * HW, y0 = r / W;
     return make_int4((b * xC + xc0) * HW + r, y0, r - y0 * W, b);
-  }
-  __device__ int4 tap(int m) const {
-    const int kk = ks * ks, cin = m / kk, t = m - cin * kk;
-    const int dy = t / ks - ks / 2, dx = t % ks - ks / 2;
-    return make_int4(cin * H * W + dy * W, dy, dx, 0);
   }
   __device__ float a(int m, int k) const {
     const int kk = ks * ks, cin = m / kk, t = m - cin * kk;
@@ -452,9 +504,12 @@ struct ConvBwdWeightOp {
     return dz + (size_t)(p.w * zC + zc0 + n) * H * W + p.y * W + p.z;
   }
   __device__ int row(int m) const { return m; }
-  __device__ void store(int m, int n, float v, int split) const {
-    const size_t wn = (size_t)Cout * Cin * ks * ks;
-    partial[split * wn + (size_t)n * Cin * ks * ks + m] = v;
+  __device__ void store(int m, int n, int cnt, float (&v)[8], int split) const {
+    const size_t row = (size_t)Cin * ks * ks;
+    float* out = partial + split * Cout * row + n * row + m;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (j < cnt) out[j * row] = v[j];
   }
 };
 
@@ -465,7 +520,15 @@ __global__ void k_sum_splits(size_t n, int nsplit, const float* __restrict__ par
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.0f;
-  for (int k = 0; k < nsplit; k++) s += part[k * n + i];
+  // 16 loads in flight: hundreds of splits of a few hundred weights
+  for (int k0 = 0; k0 < nsplit; k0 += 16) {
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[k] = k0 + k < nsplit ? __ldg(part + (k0 + k) * n + i) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+      if (k0 + k < nsplit) s += v[k];
+  }
   out[i] = s;
 }
 
@@ -664,9 +727,11 @@ struct Ctx {
   uint32_t* done = nullptr;  // block counter of k_bias_grad
 };
 
-template <class Op, int BN>
-gv_status launch_gemm_bn(const Ctx& c, const Op& op, int M, int N, int K, int nsplit) {
-  auto kern = k_gemm<Op, BN>;
+inline int tile_columns(int N) { return N <= 64 ? 64 : (N <= 128 ? 128 : 256); }
+
+template <class Op, int BN, int KS>
+gv_status launch_gemm_tiled(const Ctx& c, const Op& op, int M, int N, int K, int nsplit) {
+  auto kern = k_gemm<Op, BN, KS>;
   const int smem = (int)GemmLayout<BN>::kSmem;
   GV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int klen = ((K + nsplit - 1) / nsplit + kBK - 1) / kBK * kBK;
@@ -677,19 +742,31 @@ gv_status launch_gemm_bn(const Ctx& c, const Op& op, int M, int N, int K, int ns
   return GV_OK;
 }
 
+template <class Op, int BN>
+gv_status launch_gemm_bn(const Ctx& c, const Op& op, int M, int N, int K, int nsplit) {
+  if (op.fast && op.ks == 3) return launch_gemm_tiled<Op, BN, 3>(c, op, M, N, K, nsplit);
+  if (op.fast && op.ks == 1) return launch_gemm_tiled<Op, BN, 1>(c, op, M, N, K, nsplit);
+  return launch_gemm_tiled<Op, BN, 0>(c, op, M, N, K, nsplit);
+}
+
+// Column tiles of up to 256, narrower ones where the SMs would not all have a
+// CTA: what a chunk costs is its latency and A's staging, hardly its columns
+// (the
+// data gradient of the 16^2 level, 16 row tiles of 256 columns and 36 chunks:
+// 101 us in 16 CTAs, 53 in 64).
 template <class Op>
 gv_status launch_gemm(const Ctx& c, const Op& op, int M, int N, int K, int nsplit = 1) {
-  if (N <= 64) return launch_gemm_bn<Op, 64>(c, op, M, N, K, nsplit);
-  if (N <= 128) return launch_gemm_bn<Op, 128>(c, op, M, N, K, nsplit);
-  return launch_gemm_bn<Op, 256>(c, op, M, N, K, nsplit);  // column tiles of 256
+  int bn = tile_columns(N);
+  while (bn > 64 && ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn) * nsplit < c.num_sms) bn /= 2;
+  if (bn == 64) return launch_gemm_bn<Op, 64>(c, op, M, N, K, nsplit);
+  if (bn == 128) return launch_gemm_bn<Op, 128>(c, op, M, N, K, nsplit);
+  return launch_gemm_bn<Op, 256>(c, op, M, N, K, nsplit);
 }
 
 // grid of the per-channel kernels: n pixels a channel, `planes` of them
 inline dim3 plane_grid(int n, int planes) {
   return dim3((unsigned)std::min((n + 255) / 256, 64), (unsigned)planes);
 }
-
-inline int tile_columns(int N) { return N <= 64 ? 64 : (N <= 128 ? 128 : 256); }
 
 inline int ew_blocks(size_t n, const Ctx& c) {
   return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, (size_t)8 * c.num_sms));
@@ -899,7 +976,9 @@ struct UNet {
     for (const Layer& ly : layers)
       for (int back = 0; back < 2; back++) {
         const int N = back ? ly.cin : ly.cout, K = (back ? ly.cout : ly.cin) * ly.ks * ly.ks;
-        const int bn = tile_columns(N), tiles = (N + bn - 1) / bn, chunks = (K + kBK - 1) / kBK;
+        // whole tiles of whatever width the launch takes
+        const int bn = 64, chunks = (K + kBK - 1) / kBK;
+        const int tiles = (N + tile_columns(N) - 1) / tile_columns(N) * (tile_columns(N) / bn);
         entries.push_back({ly.w, ly.cin, ly.cout, ly.ks, back, bn, tiles, chunks, images});
         images += (size_t)tiles * chunks * (bn / 8) * kBK;
       }
