@@ -60,7 +60,7 @@ struct NuPlan {
   int* d_slot = nullptr;       // [C nty ntx] first task of each tile, or -1
   uint32_t* d_done = nullptr;  // [tasks] tasks of a tile done (at its first task)
   float4* d_slots = nullptr;   // per task: [pair][225] sums {h+, h-}
-  float2* d_H = nullptr;       // [channel of the group][pair][nrow][N]
+  float2* d_H = nullptr;       // [channel of the group][pair][N / 4][nrow][4]
   float2* d_twiddle = nullptr; // fft16_twiddles(log2 2N)
   float* d_corr = nullptr;     // [N] 1 / kernel transform
   float2* d_coef = nullptr;    // [pair][MN] w-term coefficients (k_nu_coefficients)
@@ -479,9 +479,14 @@ __global__ void __launch_bounds__(RowShape<LG>::kBlock, 1024 / RowShape<LG>::kBl
   }
   fft16<LG>(v, buf, j, a.tw);
   if (!mine) return;
-  float2* h = a.H + ((size_t)plane * a.nrow + r - a.rmin) * N;
+  // four columns are a sector, and the rows' sectors of these columns lie
+  // together: the column pass reads whole lines
+  float2* h = a.H + ((size_t)plane * (N / 4) * a.nrow + r - a.rmin) * 4;
 #pragma unroll
-  for (int s = 0; s < 8; s++) h[j + s * T] = v[kept_output(s)];
+  for (int s = 0; s < 8; s++) {
+    const int col = j + s * T;
+    h[(size_t)(col >> 2) * a.nrow * 4 + (col & 3)] = v[kept_output(s)];
+  }
 }
 
 // Per pixel and channel (blockIdx.y) the factor of the sum that does not
@@ -636,12 +641,13 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
     float2 v[16];
     {
       // rows below 0 first in memory: row r of the plane at r - rmin
-      const float2* h = a.H + ((int64_t)p * a.nrow - a.rmin + j) * N + col;
+      const float2* h =
+          a.H + (((int64_t)p * (N / 4) + (col >> 2)) * a.nrow - a.rmin + j) * 4 + (col & 3);
       const unsigned lo = (unsigned)(j - a.rmin);
 #pragma unroll
       for (int e = 0; e < 16; e++) {
         const int o = e < 8 ? e * T : e * T - n;
-        v[e] = in && lo + (unsigned)o < (unsigned)a.nrow ? h[(int64_t)o * N]
+        v[e] = in && lo + (unsigned)o < (unsigned)a.nrow ? h[4 * o]
                                                          : make_float2(0.0f, 0.0f);
       }
     }
