@@ -58,13 +58,16 @@ struct NuPlan {
   std::vector<int> groups;     // channel group boundaries
   NuTask* d_tasks = nullptr;
   int* d_slot = nullptr;       // [C nty ntx] first task of each tile, or -1
-  uint32_t* d_done = nullptr;  // [tasks] tasks of a tile done (at its first task)
+  // [tasks] tasks of a tile done (at its first task), [N] pieces of a column block done
+  uint32_t* d_done = nullptr;
+  int tasks = 0;
   float4* d_slots = nullptr;   // per task: [pair][225] sums {h+, h-}
   float2* d_H = nullptr;       // [channel of the group][pair][N / 4][nrow][4]
   float2* d_twiddle = nullptr; // fft16_twiddles(log2 2N)
   float* d_corr = nullptr;     // [N] 1 / kernel transform
   float2* d_coef = nullptr;    // [pair][MN] w-term coefficients (k_nu_coefficients)
   float* d_fac = nullptr;      // [C][MN] image-independent factors (k_nu_factors)
+  float* d_part = nullptr;     // sums of shared column blocks, N >= 1024
   float coef[4][12];           // the taps' polynomials (tap_polynomials)
 };
 
@@ -145,6 +148,11 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
 // left.  The warps' 15 x 15 tiles are added in order and go out once, to the
 // task's own slot; where a tile has several tasks, the last of their blocks
 // to finish adds the slots up, in order, into the first.
+//
+// Bound by issue slots and shared-memory wavefronts, 65 % of each: 47 warp
+// instructions a visibility.  8.9 M visibilities in 8 channels, two pairs:
+// 565 us (34 us of memory traffic); 47 us for 0.84 M over 1024^2.  Lanes four
+// to a column, which writes a column back in fewer wavefronts: 584.
 template <int NP, int kSpreadWarps>
 __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   extern __shared__ float4 smem_f4[];
@@ -382,6 +390,11 @@ __device__ __forceinline__ float4 cell_at(const RowArgs& a, const RowTiles& t, i
 // the sums lie in u >= 0, so one cell of a tile feeds the two rows at c and
 // -c.  Taking the rows together looks every cell up and reads it once.
 // kPairs couples of rows per block.
+//
+// Bound by the waits between its phases (looking cells up, three exchanges)
+// at two blocks an SM, about half of the issue slots: 16 planes of 2048^2 with
+// 1223 covered rows, 380 us where its traffic takes 100; a row by itself, each
+// cell looked up twice, 460.
 template <int LG>
 struct RowShape {
   static constexpr int kThreads = (1 << LG) / 16;  // per line
@@ -568,6 +581,8 @@ struct ColArgs {
   const uint8_t* __restrict__ mask;   // pixels written (kMaskIn), or null: all
   const float* __restrict__ img;      // the image's planes (chain rule), or null
   float* __restrict__ out;
+  float* part;                        // [block][2][8][kBlock] sums of shared column blocks
+  uint32_t* done;                     // [N / kCols] their pieces done
 };
 
 // Column FFTs over the covered rows of 2N, the N outputs about the middle
@@ -577,12 +592,26 @@ struct ColArgs {
 // kCols adjacent columns per block; kGroups sets of threads take the
 // (channel, pair) planes in turn and are added up at the end, so a small
 // image's few planes run side by side.
+//
+// Bound by waits on loads: two blocks an SM is what 64 registers a thread
+// allow, and a plane's loads, passes and coefficients follow one another.  16
+// planes of 2048^2: 615 us where the traffic takes 86.  With the grid laid out
+// row by row, 16 bytes of each for a block's two columns, 695.  Taken back:
+// the next plane's rows by cp.async (870), coefficients computed instead of
+// read (723), the twiddle factors in shared memory between two sets of
+// columns in one block (640).
 template <int LG>
 struct ColShape {
   static constexpr int kThreads = (1 << LG) / 16;  // per line
   static constexpr int kCols = LG >= 13 ? 1 : (LG == 12 ? 2 : (LG == 11 ? 4 : 2));
   static constexpr int kGroups = LG >= 11 ? 1 : 2;
+  // Large sides: the (column block, plane) units in equal runs over two blocks
+  // an SM.  1024^2 has 256 column blocks, too few for the 304 places (8
+  // channels in two pairs: 187 us with a block each, 178 so); at 2048^2, with
+  // 3.4 waves, either takes 615 us.
+  static constexpr bool kShared = kGroups == 1;
   static constexpr int kBlock = kThreads * kCols * kGroups;
+  static_assert(!kShared || kBlock == 512, "size of the shared sums");
   // columns are this far apart: 16 / kCols more than a multiple of 16, so the
   // lanes of a half warp, kCols columns wide, fall in distinct banks
   static constexpr int kStride = (span16(1 << LG) + 15) / 16 * 16 + 16 / kCols;
@@ -596,6 +625,46 @@ __device__ __noinline__ float power(float nudiv, float al) {
   return al == 0.0f ? 1.0f : powf(nudiv, al);
 }
 
+// The planes of a column block that is shared out between blocks: each leaves
+// its sums, and the last to finish adds them up in the planes' order, into
+// acc, and goes on with them (true).
+template <int kBlock>
+__device__ __forceinline__ bool pieces_done(const ColArgs& a, int cblk, int first, int planes,
+                                         int cblks, float (&acc)[8]) {
+  // a block's piece that starts a column block lies in its second slot
+  float* mine = a.part + ((size_t)blockIdx.x * 2 + (first == 0)) * 8 * kBlock + threadIdx.x;
+#pragma unroll
+  for (int s = 0; s < 8; s++) __stcg(mine + s * kBlock, acc[s]);
+  // the blocks that hold the column block's first and last unit
+  const int64_t total = (int64_t)cblks * planes;
+  auto holder = [&](int64_t u) {
+    int b = (int)(u * gridDim.x / total);
+    while ((b + 1) * total / gridDim.x <= u) b++;
+    return b;
+  };
+  const int b0 = holder((int64_t)cblk * planes), b1 = holder((int64_t)(cblk + 1) * planes - 1);
+  __shared__ int is_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    is_last = atomicAdd(a.done + cblk, 1u) == (uint32_t)(b1 - b0);
+    if (is_last) a.done[cblk] = 0u;
+  }
+  __syncthreads();
+  const bool mine_to_finish = is_last != 0;
+  __syncthreads();  // is_last is read before the next piece sets it
+  if (!mine_to_finish) return false;
+  __threadfence();
+#pragma unroll
+  for (int s = 0; s < 8; s++) acc[s] = 0.0f;
+  for (int b = b0; b <= b1; b++) {
+    const float* p = a.part + ((size_t)b * 2 + (b == b0)) * 8 * kBlock + threadIdx.x;
+#pragma unroll
+    for (int s = 0; s < 8; s++) acc[s] += __ldcg(p + s * kBlock);
+  }
+  return true;
+}
+
 template <int LG>
 __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 512 ? 2 : 1)
     k_nu_cols(ColArgs a) {
@@ -604,117 +673,134 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
   extern __shared__ float2 smem_f2[];
   const int cc = threadIdx.x % CB, j = (threadIdx.x / CB) % T, g = threadIdx.x / (CB * T);
   float2* buf = smem_f2 + (g * CB + cc) * S::kStride;
-  const int col = blockIdx.x * CB + cc;
   constexpr int64_t MN = (int64_t)N * N;
-  // the thread's pixels of the image's alpha plane, kept for all planes
   float* al = reinterpret_cast<float*>(smem_f2 + G * CB * S::kStride) + threadIdx.x;
-  bool flat = true;
-  if (a.img) {
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-      const float v = __ldg(a.img + MN + (int64_t)N * (j + s * T) + col);
-      al[s * S::kBlock] = v;
-      flat = flat && v == 0.0f;
-    }
-  }
-  // small sides, whose blocks run once through a plane or two: everything the
-  // end needs is on its way before the first transform
-  constexpr bool kAhead = LG <= 10;
-  float old[kAhead ? 8 : 1];
-  bool write[kAhead ? 8 : 1];
-  if constexpr (kAhead) {
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-      const int64_t px = (int64_t)N * (j + s * T) + col;
-      write[s] = !a.mask || (a.mask[px] & kMaskIn);
-      old[s] = a.out[px];
-    }
-  }
-  float acc[8];
-#pragma unroll
-  for (int s = 0; s < 8; s++) acc[s] = 0.0f;
   const int planes = a.nchan * a.np;
-  for (int p0 = 0; p0 < planes; p0 += G) {
-    const int p = p0 + g;
-    const bool in = p < planes;
-    const int c = p / a.np, q = p - c * a.np;
-    float2 v[16];
-    {
-      // rows below 0 first in memory: row r of the plane at r - rmin
-      const float2* h =
-          a.H + (((int64_t)p * (N / 4) + (col >> 2)) * a.nrow - a.rmin + j) * 4 + (col & 3);
-      const unsigned lo = (unsigned)(j - a.rmin);
+  // this block's units (columns, then planes), see kShared
+  int unit = blockIdx.x * planes, end = unit + planes;
+  if constexpr (S::kShared) {
+    const int64_t total = (int64_t)(N / CB) * planes;
+    unit = (int)(blockIdx.x * total / gridDim.x);
+    end = (int)((blockIdx.x + 1) * total / gridDim.x);
+  }
+#pragma unroll 1
+  while (unit < end) {
+    const int cblk = unit / planes, first = unit - cblk * planes;
+    const int last = min(planes, first + end - unit);
+    unit += last - first;
+    const int col = cblk * CB + cc;
+    // the thread's pixels of the image's alpha plane, kept for all planes
+    bool flat = true;
+    if (a.img) {
 #pragma unroll
-      for (int e = 0; e < 16; e++) {
-        const int o = e < 8 ? e * T : e * T - n;
-        v[e] = in && lo + (unsigned)o < (unsigned)a.nrow ? h[4 * o]
-                                                         : make_float2(0.0f, 0.0f);
+      for (int s = 0; s < 8; s++) {
+        const float v = __ldg(a.img + MN + (int64_t)N * (j + s * T) + col);
+        al[s * S::kBlock] = v;
+        flat = flat && v == 0.0f;
       }
     }
-    const float2* kq = a.coef + q * MN + (int64_t)N * col + j;
-    const float* fc = a.fac ? a.fac + c * MN + (int64_t)N * col + j : nullptr;
-    float2 kk[kAhead ? 8 : 1];
-    float ff[kAhead ? 8 : 1];
+    // small sides, whose blocks run once through a plane or two: everything the
+    // end needs is on its way before the first transform
+    constexpr bool kAhead = LG <= 10;
+    float old[kAhead ? 8 : 1];
+    bool write[kAhead ? 8 : 1];
     if constexpr (kAhead) {
 #pragma unroll
       for (int s = 0; s < 8; s++) {
-        kk[s] = in ? __ldg(kq + s * T) : make_float2(0.0f, 0.0f);
-        ff[s] = in && fc ? __ldg(fc + s * T) : 1.0f;
+        const int64_t px = (int64_t)N * (j + s * T) + col;
+        write[s] = !a.mask || (a.mask[px] & kMaskIn);
+        old[s] = a.out[px];
       }
     }
-    __syncthreads();  // the last line has been read
-    fft16<LG>(v, buf, j, a.tw);
-    if (!in) continue;
-    const float nudiv = a.img ? a.chfreq[c] / a.nu_0 : 1.0f;
-    const float lg = a.alpha ? logf(nudiv) : 1.0f;
+    float acc[8];
 #pragma unroll
-    for (int s = 0; s < 8; s++) {
-      const float2 x = v[kept_output(s)];
-      float t;
-      if (a.wterm) {
-        const float2 k = kAhead ? kk[kAhead ? s : 0] : __ldg(kq + s * T);
-        t = fmaf(k.x, x.x, k.y * x.y);
-      } else {
-        t = q == 0 ? x.x * (__ldg(a.corr + j + s * T) * __ldg(a.corr + col)) : 0.0f;
-      }
-      float f = kAhead ? ff[kAhead ? s : 0] : (fc ? __ldg(fc + s * T) : 1.0f);
-      f *= lg;
-      if (!flat) {
-        const float av = al[s * S::kBlock];
-        if constexpr (kAhead) {
-          f *= power(nudiv, av);
-        } else if (av != 0.0f) {
-          f *= powf(nudiv, av);
+    for (int s = 0; s < 8; s++) acc[s] = 0.0f;
+    for (int p0 = first; p0 < last; p0 += G) {
+      const int p = p0 + g;
+      const bool in = p < last;
+      const int c = p / a.np, q = p - c * a.np;
+      float2 v[16];
+      {
+        // rows below 0 first in memory: row r of the plane at r - rmin
+        const float2* h =
+            a.H + (((int64_t)p * (N / 4) + (col >> 2)) * a.nrow - a.rmin + j) * 4 + (col & 3);
+        const unsigned lo = (unsigned)(j - a.rmin);
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+          const int o = e < 8 ? e * T : e * T - n;
+          v[e] = in && lo + (unsigned)o < (unsigned)a.nrow ? h[4 * o] : make_float2(0.0f, 0.0f);
         }
       }
-      acc[s] = fmaf(f, t, acc[s]);
-    }
-  }
-  if constexpr (G > 1) {
-    // the groups' sums, in order
-    float* part = reinterpret_cast<float*>(smem_f2);
-    __syncthreads();
-    if (g > 0) {
+      const float2* kq = a.coef + q * MN + (int64_t)N * col + j;
+      const float* fc = a.fac ? a.fac + c * MN + (int64_t)N * col + j : nullptr;
+      float2 kk[kAhead ? 8 : 1];
+      float ff[kAhead ? 8 : 1];
+      if constexpr (kAhead) {
 #pragma unroll
-      for (int s = 0; s < 8; s++) part[((g - 1) * 8 + s) * T * CB + threadIdx.x % (T * CB)] = acc[s];
-    }
-    __syncthreads();
-    if (g > 0) return;
-    for (int o = 0; o < G - 1; o++)
+        for (int s = 0; s < 8; s++) {
+          kk[s] = in ? __ldg(kq + s * T) : make_float2(0.0f, 0.0f);
+          ff[s] = in && fc ? __ldg(fc + s * T) : 1.0f;
+        }
+      }
+      __syncthreads();  // the last line has been read
+      fft16<LG>(v, buf, j, a.tw);
+      if (!in) continue;
+      const float nudiv = a.img ? a.chfreq[c] / a.nu_0 : 1.0f;
+      const float lg = a.alpha ? logf(nudiv) : 1.0f;
 #pragma unroll
-      for (int s = 0; s < 8; s++) acc[s] += part[(o * 8 + s) * T * CB + threadIdx.x];
-  }
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    const int64_t px = (int64_t)N * (j + s * T) + col;
-    if (!(kAhead ? write[kAhead ? s : 0] : !a.mask || (a.mask[px] & kMaskIn))) continue;
-    float t = acc[s];
-    if (a.alpha) {
-      const float i0 = a.img[px];
-      if (!(i0 > a.threshold)) continue;
-      t *= i0 * a.fg_scale;
+      for (int s = 0; s < 8; s++) {
+        const float2 x = v[kept_output(s)];
+        float t;
+        if (a.wterm) {
+          const float2 k = kAhead ? kk[kAhead ? s : 0] : __ldg(kq + s * T);
+          t = fmaf(k.x, x.x, k.y * x.y);
+        } else {
+          t = q == 0 ? x.x * (__ldg(a.corr + j + s * T) * __ldg(a.corr + col)) : 0.0f;
+        }
+        float f = kAhead ? ff[kAhead ? s : 0] : (fc ? __ldg(fc + s * T) : 1.0f);
+        f *= lg;
+        if (!flat) {
+          const float av = al[s * S::kBlock];
+          if constexpr (kAhead) {
+            f *= power(nudiv, av);
+          } else if (av != 0.0f) {
+            f *= powf(nudiv, av);
+          }
+        }
+        acc[s] = fmaf(f, t, acc[s]);
+      }
     }
-    a.out[px] = (kAhead ? old[kAhead ? s : 0] : a.out[px]) + t;
+    if constexpr (G > 1) {
+      // the groups' sums, in order
+      float* part = reinterpret_cast<float*>(smem_f2);
+      __syncthreads();
+      if (g > 0) {
+#pragma unroll
+        for (int s = 0; s < 8; s++)
+          part[((g - 1) * 8 + s) * T * CB + threadIdx.x % (T * CB)] = acc[s];
+      }
+      __syncthreads();
+      if (g > 0) return;
+      for (int o = 0; o < G - 1; o++)
+#pragma unroll
+        for (int s = 0; s < 8; s++) acc[s] += part[(o * 8 + s) * T * CB + threadIdx.x];
+    }
+    if constexpr (S::kShared) {
+      if (last - first < planes && !pieces_done<S::kBlock>(a, cblk, first, planes, N / CB, acc))
+        continue;
+    }
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      const int64_t px = (int64_t)N * (j + s * T) + col;
+      if (!(kAhead ? write[kAhead ? s : 0] : !a.mask || (a.mask[px] & kMaskIn))) continue;
+      float t = acc[s];
+      if (a.alpha) {
+        const float i0 = a.img[px];
+        if (!(i0 > a.threshold)) continue;
+        t *= i0 * a.fg_scale;
+      }
+      a.out[px] = (kAhead ? old[kAhead ? s : 0] : a.out[px]) + t;
+    }
   }
 }
 
@@ -806,6 +892,9 @@ gv_status spread(const SpreadArgs& a, int warps, cudaStream_t st) {
   return warps == 8 ? spread_warps<NP, 8>(a, st) : spread_warps<NP, 1>(a, st);
 }
 
+// blocks of k_nu_cols that share the column blocks out: two an SM
+int shared_blocks(const Problem& P) { return 2 * P.num_sms; }
+
 template <int LG>
 gv_status transforms(Problem& P, const RowArgs& ra, const ColArgs& ca) {
   using R = RowShape<LG>;
@@ -819,7 +908,9 @@ gv_status transforms(Problem& P, const RowArgs& ra, const ColArgs& ca) {
   if (S::kSmem > 48 * 1024)
     GV_CUDA(cudaFuncSetAttribute(k_nu_cols<LG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)S::kSmem));
-  k_nu_cols<LG><<<P.N / S::kCols, S::kBlock, S::kSmem, P.stream>>>(ca);
+  int blocks = P.N / S::kCols;
+  if (S::kShared) blocks = std::min(blocks * ca.nchan * ca.np, shared_blocks(P));
+  k_nu_cols<LG><<<blocks, S::kBlock, S::kSmem, P.stream>>>(ca);
   GV_LAUNCH("k_nu_cols");
   return GV_OK;
 }
@@ -848,6 +939,7 @@ void nu_free(Problem& P) {
   cudaFree(n->d_corr);
   cudaFree(n->d_coef);
   cudaFree(n->d_fac);
+  cudaFree(n->d_part);
   delete n;
   P.nu = nullptr;
 }
@@ -1017,13 +1109,15 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   auto upload = [&]() -> cudaError_t {
     cudaError_t e = cudaMalloc(&n->d_tasks, sizeof(NuTask) * tasks.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_slot, sizeof(int) * slot.size());
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_done, sizeof(uint32_t) * tasks.size());
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_done, sizeof(uint32_t) * (tasks.size() + N));
     if (e == cudaSuccess) e = cudaMalloc(&n->d_slots, slot_b * max_slots);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_H, h_b * max_ch);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_twiddle, sizeof(float2) * tw.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_corr, sizeof(float) * N);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_coef, sizeof(float2) * (size_t)pairs * N * N);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_fac, fac_b * C);
+    if (e == cudaSuccess && N >= 1024)
+      e = cudaMalloc(&n->d_part, sizeof(float) * shared_blocks(P) * 2 * 8 * ColShape<11>::kBlock);
     return e;
   };
   const cudaError_t e = upload();
@@ -1037,7 +1131,8 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   GV_CUDA(cudaMemcpy(n->d_tasks, tasks.data(), sizeof(NuTask) * tasks.size(),
                      cudaMemcpyHostToDevice));
   GV_CUDA(cudaMemcpy(n->d_slot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice));
-  GV_CUDA(cudaMemset(n->d_done, 0, sizeof(uint32_t) * tasks.size()));
+  GV_CUDA(cudaMemset(n->d_done, 0, sizeof(uint32_t) * (tasks.size() + N)));
+  n->tasks = (int)tasks.size();
   GV_CUDA(cudaMemcpy(n->d_twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   GV_CUDA(cudaMemcpy(n->d_corr, corr.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
   return GV_OK;
@@ -1079,6 +1174,8 @@ gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result
   ra.nty = n.nty;
   const int64_t MN = (int64_t)P.M * N;
   ColArgs ca;
+  ca.part = n.d_part;
+  ca.done = n.d_done + n.tasks;
   ca.np = np;
   ca.nrow = n.nrow;
   ca.rmin = n.rmin;

@@ -140,3 +140,20 @@ def test_repeats_bit_for_bit():
     g = pa.dchi2(ia)
     for _ in range(3):
         assert torch.equal(pa.dchi2(ia), g)
+
+
+@pytest.mark.parametrize("nchan,wscale", [(1, 0.0), (1, 1.0), (3, 1.0), (5, 2.0)])
+def test_columns_shared_out(nchan, wscale):
+    """Sides from 1024 up share the columns' planes out between blocks: one
+    plane a column (nothing shared, fewer units than blocks), two (a column in
+    two pieces at most) and more than a block's run."""
+    import torch
+    pa, pb = _pair(1024, nchan=nchan, seed=21, wscale=wscale)
+    ia, ib = _image(pa, 9, True), _image(pb, 9, True)
+    pa.chi2(ia)
+    pb.chi2(ib)
+    # one channel is at the reference frequency: its alpha gradient is zero
+    for flag in (0, 1) if nchan > 1 else (0,):
+        ga, gb = pa.dchi2(ia, flag_opt=flag), pb.dchi2(ib, flag_opt=flag)
+        _close(ga[flag], gb[flag])
+        assert torch.equal(ga, pa.dchi2(ia, flag_opt=flag))
