@@ -11,10 +11,10 @@
 //                splits summed in a fixed order)
 // The operand tiles are staged by the CTA's threads straight from the FP32
 // NCHW activations (im2col on the fly, rounded to BF16) into 128-byte
-// swizzled MN-major shared-memory tiles; one thread issues the MMAs; two
-// stages alternate, the next chunk's loads under way.  The epilogue (bias, ReLU, layout) is applied on the way
-// out of TMEM.  Pooling, upsampling, the loss and Adam are plain
-// bandwidth-bound kernels.
+// swizzled shared-memory tiles; one thread issues the MMAs; two stages
+// alternate, the next chunk's loads under way.  The epilogue (bias, ReLU,
+// layout) is applied on the way out of TMEM.  Pooling, upsampling, the loss
+// and Adam are plain bandwidth-bound kernels.
 //
 // Layout of the network (levels l = 0..L-1, C_l = c0 * 2^l channels, side
 // H / 2^l):  enc_l = relu(conv(relu(conv(in_l)))), in_{l+1} = avgpool2(enc_l);
@@ -751,9 +751,8 @@ gv_status launch_gemm_bn(const Ctx& c, const Op& op, int M, int N, int K, int ns
 
 // Column tiles of up to 256, narrower ones where the SMs would not all have a
 // CTA: what a chunk costs is its latency and A's staging, hardly its columns
-// (the
-// data gradient of the 16^2 level, 16 row tiles of 256 columns and 36 chunks:
-// 101 us in 16 CTAs, 53 in 64).
+// (the data gradient of the 16^2 level, 16 row tiles of 256 columns and 36
+// chunks: 101 us in 16 CTAs, 53 in 64).
 template <class Op>
 gv_status launch_gemm(const Ctx& c, const Op& op, int M, int N, int K, int nsplit = 1) {
   int bn = tile_columns(N);

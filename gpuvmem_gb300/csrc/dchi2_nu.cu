@@ -595,7 +595,7 @@ struct ColArgs {
 //
 // Bound by waits on loads: two blocks an SM is what 64 registers a thread
 // allow, and a plane's loads, passes and coefficients follow one another.  16
-// planes of 2048^2: 615 us where the traffic takes 86.  With the grid laid out
+// planes of 2048^2: 585 us where the traffic takes 86.  With the grid laid out
 // row by row, 16 bytes of each for a block's two columns, 695.  Taken back:
 // the next plane's rows by cp.async (870), coefficients computed instead of
 // read (723), the twiddle factors in shared memory between two sets of
@@ -607,9 +607,13 @@ struct ColShape {
   static constexpr int kGroups = LG >= 11 ? 1 : 2;
   // Large sides: the (column block, plane) units in equal runs over two blocks
   // an SM.  1024^2 has 256 column blocks, too few for the 304 places (8
-  // channels in two pairs: 187 us with a block each, 178 so); at 2048^2, with
-  // 3.4 waves, either takes 615 us.
+  // channels in two pairs: 187 us with a block each, 178 so); 2048^2 would
+  // have 3.4 waves (614 us, 585 so).
+  // Blocks whose columns share sectors of the grid take the same run: with one
+  // run after the other over single blocks each sector came from HBM twice
+  // (2048^2: 1.1 GB, 615 us).
   static constexpr bool kShared = kGroups == 1;
+  static constexpr int kTeam = kShared ? 4 / kCols : 1;
   static constexpr int kBlock = kThreads * kCols * kGroups;
   static_assert(!kShared || kBlock == 512, "size of the shared sums");
   // columns are this far apart: 16 / kCols more than a multiple of 16, so the
@@ -628,21 +632,22 @@ __device__ __noinline__ float power(float nudiv, float al) {
 // The planes of a column block that is shared out between blocks: each leaves
 // its sums, and the last to finish adds them up in the planes' order, into
 // acc, and goes on with them (true).
-template <int kBlock>
+template <int kBlock, int kTeam>
 __device__ __forceinline__ bool pieces_done(const ColArgs& a, int cblk, int first, int planes,
-                                         int cblks, float (&acc)[8]) {
+                                            int cblks, float (&acc)[8]) {
   // a block's piece that starts a column block lies in its second slot
   float* mine = a.part + ((size_t)blockIdx.x * 2 + (first == 0)) * 8 * kBlock + threadIdx.x;
 #pragma unroll
   for (int s = 0; s < 8; s++) __stcg(mine + s * kBlock, acc[s]);
-  // the blocks that hold the column block's first and last unit
-  const int64_t total = (int64_t)cblks * planes;
+  // the runs that hold the column block's first and last unit
+  const int64_t total = (int64_t)(cblks / kTeam) * planes;
+  const int runs = gridDim.x / kTeam, quad = cblk / kTeam;
   auto holder = [&](int64_t u) {
-    int b = (int)(u * gridDim.x / total);
-    while ((b + 1) * total / gridDim.x <= u) b++;
+    int b = (int)(u * runs / total);
+    while ((b + 1) * total / runs <= u) b++;
     return b;
   };
-  const int b0 = holder((int64_t)cblk * planes), b1 = holder((int64_t)(cblk + 1) * planes - 1);
+  const int b0 = holder((int64_t)quad * planes), b1 = holder((int64_t)(quad + 1) * planes - 1);
   __shared__ int is_last;
   __threadfence();
   __syncthreads();
@@ -658,7 +663,9 @@ __device__ __forceinline__ bool pieces_done(const ColArgs& a, int cblk, int firs
 #pragma unroll
   for (int s = 0; s < 8; s++) acc[s] = 0.0f;
   for (int b = b0; b <= b1; b++) {
-    const float* p = a.part + ((size_t)b * 2 + (b == b0)) * 8 * kBlock + threadIdx.x;
+    const float* p = a.part +
+                     ((size_t)(b * kTeam + cblk % kTeam) * 2 + (b == b0)) * 8 * kBlock +
+                     threadIdx.x;
 #pragma unroll
     for (int s = 0; s < 8; s++) acc[s] += __ldcg(p + s * kBlock);
   }
@@ -679,13 +686,15 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
   // this block's units (columns, then planes), see kShared
   int unit = blockIdx.x * planes, end = unit + planes;
   if constexpr (S::kShared) {
-    const int64_t total = (int64_t)(N / CB) * planes;
-    unit = (int)(blockIdx.x * total / gridDim.x);
-    end = (int)((blockIdx.x + 1) * total / gridDim.x);
+    const int64_t total = (int64_t)(N / CB / S::kTeam) * planes;
+    const int run = blockIdx.x / S::kTeam, runs = gridDim.x / S::kTeam;
+    unit = (int)(run * total / runs);
+    end = (int)((run + 1) * total / runs);
   }
 #pragma unroll 1
   while (unit < end) {
-    const int cblk = unit / planes, first = unit - cblk * planes;
+    const int at = unit / planes, first = unit - at * planes;
+    const int cblk = S::kShared ? at * S::kTeam + (int)(blockIdx.x % S::kTeam) : at;
     const int last = min(planes, first + end - unit);
     unit += last - first;
     const int col = cblk * CB + cc;
@@ -786,7 +795,8 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
         for (int s = 0; s < 8; s++) acc[s] += part[(o * 8 + s) * T * CB + threadIdx.x];
     }
     if constexpr (S::kShared) {
-      if (last - first < planes && !pieces_done<S::kBlock>(a, cblk, first, planes, N / CB, acc))
+      if (last - first < planes &&
+          !pieces_done<S::kBlock, S::kTeam>(a, cblk, first, planes, N / CB, acc))
         continue;
     }
 #pragma unroll
@@ -909,7 +919,9 @@ gv_status transforms(Problem& P, const RowArgs& ra, const ColArgs& ca) {
     GV_CUDA(cudaFuncSetAttribute(k_nu_cols<LG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)S::kSmem));
   int blocks = P.N / S::kCols;
-  if (S::kShared) blocks = std::min(blocks * ca.nchan * ca.np, shared_blocks(P));
+  if (S::kShared)
+    blocks = S::kTeam * std::max(1, std::min(blocks / S::kTeam * ca.nchan * ca.np,
+                                             shared_blocks(P) / S::kTeam));
   k_nu_cols<LG><<<blocks, S::kBlock, S::kSmem, P.stream>>>(ca);
   GV_LAUNCH("k_nu_cols");
   return GV_OK;
