@@ -1,7 +1,7 @@
 """Benchmark: objective + gradient evaluations per second on one GB300.
 
 A step is one ObjectiveFunction::calcFunction + calcGradient pair (chi2 with
-entropy and TSV priors active, DChi2 direct-sum gradient) over the whole
+entropy and TSV priors active, DChi2 gradient) over the whole
 synthetic data set, i.e. one "chi2+grad evaluation" of the headline metric.
 Default workload: 2048 x 2048 image, 8 channels 225-235 GHz, 50 antennas in a
 2 km disk, 4 h at 4 s, Briggs robust 0 (35.28M visibilities), seeded
@@ -11,11 +11,13 @@ synthetic data.
   e2e     the same through the public API (gpuvmem_gb300.Problem), the image
           copied in from pinned host memory and the gradient and objective
           read back every step;
-  roofline  the dominant kernel (tcgen05 DChi2, timed inside the timed
-          loop as the gradient call) as TFLOP/s against the measured
-          sustained dense BF16 peak / 3 (three FP16 products per
-          algorithmic multiply-add; the gradient runs about a second per
-          launch inside a long loop);
+  roofline  the gradient call (DChi2 and the priors' gradients, timed inside
+          the timed loop): the bytes that it cannot do without against the
+          measured HBM copy bandwidth, since the default engine's work, a
+          local spreading per visibility and two FFTs per channel, is far
+          below the arithmetic peaks.  With --engine 2 (the direct sum as
+          a tcgen05 GEMM) TFLOP/s against the measured sustained dense BF16
+          peak / 3 (three FP16 products per algorithmic multiply-add);
   reference_cuda  the reference's own CUDA kernels (compiled from its
           sources, launched with its launch shapes and host sequence by the
           harness in oracle/ref_harness) timed on the same GPU: chi2() in
@@ -155,13 +157,54 @@ def measured_peaks():
 
 # DRAM bytes per visibility of one DChi2 launch (dram__bytes_read.sum +
 # dram__bytes_write.sum of k_dchi2_tc in an ncu capture of the one-channel
-# 2048^2 case, `bench.py --case dchi2_2048_1ch`, divided by its
+# 2048^2 case, `bench.py --case dchi2_2048_1ch --engine 2`, divided by its
 # visibilities).  The traffic of the full launch is this times its
 # visibilities: the operands are generated on chip, so the traffic is the
 # visibility constants re-read per output tile plus the partial images.
 DCHI2_DRAM_BYTES_PER_VIS = 168.48
 DCHI2_TRAFFIC_SOURCE = ("ncu capture of k_dchi2_tc, one channel of 2048^2 (bench.py --case "
                         "dchi2_2048_1ch), scaled by the visibility count")
+
+
+# DRAM bytes of one DChi2 by the default engine at 2048^2 and eight channels
+# (two pairs of w-terms): the grids between its passes and the tiles' sums, from
+# an ncu capture at 8.82M visibilities, besides the 24 B per visibility
+DCHI2_NU_GRID_BYTES_2048_8CH = 1.74e9
+DCHI2_NU_TRAFFIC_SOURCE = ("ncu capture of k_nu_spread, k_nu_rows and k_nu_cols at 2048^2, 8 "
+                           "channels and 8.82M visibilities, plus 24 B for every further one")
+
+
+def dchi2_roofline(engine, n, channels, vis, t, peaks, src):
+    """The gradient call's roofline: see the top of this file."""
+    if engine != 0:
+        peak = peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"]) / 3.0
+        flops = 4.0 * n * n * vis
+        achieved = flops / t / 1e12
+        tc = engine == 2
+        return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak,
+                "traffic": DCHI2_DRAM_BYTES_PER_VIS * vis if tc else None,
+                "traffic_source": DCHI2_TRAFFIC_SOURCE if tc else None,
+                "kernel": ("k_dchi2_tc + k_reduce_partials" if tc else "k_dchi2_direct") +
+                          " (+ prior gradients): the gradient call, timed inside the timed loop",
+                "peak_source": f"{src} dense bf16 sustained "
+                               f"{peaks.get('bf16_tflops_sustained')} TFLOP/s / 3",
+                "frac_of_burst": achieved / (peaks["bf16_tflops"] / 3.0),
+                "algorithmic_flop": flops}
+    nbytes = 24.0 * vis + 12.0 * n * n
+    achieved = nbytes / t / 1e9
+    at = (n, channels) == (2048, 8)
+    return {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+            "frac": achieved / peaks["hbm_gbs"],
+            "traffic": DCHI2_NU_GRID_BYTES_2048_8CH + 24.0 * vis if at else None,
+            "traffic_source": DCHI2_NU_TRAFFIC_SOURCE if at else None,
+            "kernel": "k_nu_spread + k_nu_rows + k_nu_cols (+ prior gradients): the gradient "
+                      "call, timed inside the timed loop",
+            "peak_source": f"{src} copy bandwidth", "algorithmic_bytes": nbytes,
+            "note": "position and residual of every visibility (24 B) and three image planes, "
+                    "once; issue slots, shared memory and the waits between the FFTs' phases "
+                    "bound the kernels",
+            "direct_sum_tflops": 4.0 * n * n * vis / t / 1e12}
 
 
 def cpu_baseline(data, terms, sample_s, impl_kind="port"):
@@ -460,14 +503,10 @@ def run_ours(args):
             dist.destroy_process_group()
         return
     peaks, src = measured_peaks()
-    # about a second per launch, inside a loop of several seconds: the
-    # sustained (power-capped) peak; the burst figure is reported beside it
-    peak = peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"]) / 3.0
-    peak_burst = peaks["bf16_tflops"] / 3.0
     V = info.nvis_in_grid
-    flops = 4.0 * cfg.n * cfg.n * V
-    achieved = flops / t_grad / 1e12
-    traffic = DCHI2_DRAM_BYTES_PER_VIS * V if info.dchi2_engine == 2 else None
+    roof = dchi2_roofline(args.engine, cfg.n, len(data.freqs), V, t_grad, peaks, src)
+    roof["gradient_ms"] = 1e3 * t_grad
+    roof["dchi2_alone_ms"] = 1e3 * t_dchi2
     # objective algorithmic bytes of a line-search evaluation: both image
     # planes read once (8 MN), per channel a grid written by the row FFTs and
     # read + written by the column FFTs (16 MN), 20 B per visibility in
@@ -504,20 +543,12 @@ def run_ours(args):
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": 1e3 * t / args.steps, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f32 (DChi2: fp16 hi/lo x3, fp32 acc)",
+        "scaling": "weak", "vs_baseline": None,
+        "dtype": "f32 (DChi2: fp16 hi/lo x3, fp32 acc)" if args.engine == 2 else "f32",
         "data": "synthetic (seeded; no public data set)", "config": config_desc(cfg, data),
         "e2e": {"value": e2e, "unit": METRIC, "h2d_bytes_per_step": int(img.numel() * 4),
                 "d2h_bytes_per_step": int(xi.numel() * 4 + 8 * (1 + len(terms)))},
-        "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak, "traffic": traffic,
-                     "traffic_source": DCHI2_TRAFFIC_SOURCE,
-                     "kernel": "k_dchi2_tc + k_reduce_partials (+ prior gradients): the "
-                               "gradient call, timed inside the timed loop",
-                     "peak_source": f"{src} dense bf16 sustained "
-                                    f"{peaks.get('bf16_tflops_sustained')} TFLOP/s / 3",
-                     "frac_of_burst": achieved / peak_burst,
-                     "gradient_ms": 1e3 * t_grad, "dchi2_alone_ms": 1e3 * t_dchi2,
-                     "algorithmic_flop": flops},
+        "roofline": roof,
         "objective": obj,
         "reference_cuda": refc,
         "converge": conv,
@@ -542,7 +573,7 @@ def run_batch(args):
     rank = int(os.environ.get("RANK", "0"))
     cfgs, lams = synth.config3_problems()
     probs, imgs, xis = [], [], []
-    flops, nvis = 0.0, 0
+    nvis = 0
     for c, lam in zip(cfgs, lams):
         d = synth.generate(c, device="cuda")
         p = gv.Problem(d, [gv.term("Chi2", 1.0), gv.term("Entropy", lam)])
@@ -550,7 +581,6 @@ def run_batch(args):
         img = p.initial_image()
         imgs.append(img)
         xis.append(torch.zeros_like(img))
-        flops += 4.0 * c.n * c.n * p.info.nvis_in_grid
         nvis += d.nvis
     batch = gv.Batch(probs)
     n = len(probs)
@@ -594,22 +624,24 @@ def run_batch(args):
     if rank != 0:
         return
     peaks, src = measured_peaks()
-    peak = peaks["bf16_tflops"] / 3.0
+    peak = peaks["hbm_gbs"]
+    # objective and gradient: 24 B per visibility and two image planes each
+    nbytes = 48.0 * nvis + sum(16.0 * i_.shape[-1] ** 2 for i_ in imgs)
     bytes_img = sum(i_.numel() * 4 for i_ in imgs)
     line = {
         "metric": METRIC, "value": n / t_graph, "unit": "problem " + METRIC, "n_gpus": 1,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * t_graph,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32 (DChi2: fp16 hi/lo x3, fp32 acc)", "data": "synthetic (seeded)",
+        "dtype": "f32", "data": "synthetic (seeded)",
         "config": {"workload": f"batch of {n} independent problems (sides 128/256/512, "
                                f"{nvis} visibilities in total), one graph launch per step",
                    "problems": n, "visibilities": int(nvis), "step": "objective + gradient of every problem"},
         "e2e": {"value": n / t_e2e, "unit": "problem " + METRIC,
                 "h2d_bytes_per_step": int(bytes_img), "d2h_bytes_per_step": int(bytes_img)},
-        "roofline": {"bound": "tensor", "achieved": flops / t_graph / 1e12, "peak": peak,
-                     "unit": "TFLOP/s", "frac": flops / t_graph / 1e12 / peak, "traffic": None,
-                     "kernel": "whole batch step (DChi2 FLOP over the step time)",
-                     "peak_source": f"{src} dense bf16 burst / 3"},
+        "roofline": {"bound": "hbm", "achieved": nbytes / t_graph / 1e9, "peak": peak,
+                     "unit": "GB/s", "frac": nbytes / t_graph / 1e9 / peak, "traffic": None,
+                     "kernel": "whole batch step (latency of the problems' chains of kernels)",
+                     "peak_source": f"{src} copy bandwidth"},
         "batch_ms": {"one_graph": 1e3 * t_graph, "streams_no_graph": 1e3 * t_streams,
                      "one_problem_after_another": 1e3 * t_seq},
         "clocks": clk.summary(0), "gpu_launches": int(launches),
@@ -630,7 +662,7 @@ def weighting_inputs(cfg):
     return uvw, w, freqs, off
 
 
-def run_case(name, reps):
+def run_case(name, reps, engine=0):
     """Small fixed workloads for profiling one kernel (used by the commands
     recorded in profiles/): `dchi2_2048_1ch` (configuration 1 reduced to one
     channel at 230 GHz, natural weights, 16 s integrations), `cfg0`, and
@@ -712,7 +744,7 @@ def run_case(name, reps):
     else:
         raise SystemExit(f"unknown case {name}")
     data = synth.generate(cfg, device="cuda")
-    prob = gv.Problem(data, [gv.term("Chi2", 1.0), gv.term("Entropy", 0.01)])
+    prob = gv.Problem(data, [gv.term("Chi2", 1.0), gv.term("Entropy", 0.01)], engine=engine)
     img = prob.initial_image()
     prob.chi2(img)
     xi = torch.zeros_like(img)
@@ -727,7 +759,7 @@ def run_case(name, reps):
 def main():
     args = parse()
     if args.case:
-        run_case(args.case, args.steps)
+        run_case(args.case, args.steps, args.engine)
         return
     if args.impl == "reference":
         run_reference(args)

@@ -149,10 +149,12 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
 // task's own slot; where a tile has several tasks, the last of their blocks
 // to finish adds the slots up, in order, into the first.
 //
-// Bound by issue slots and shared-memory wavefronts, 65 % of each: 47 warp
-// instructions a visibility.  8.9 M visibilities in 8 channels, two pairs:
-// 565 us (34 us of memory traffic); 47 us for 0.84 M over 1024^2.  Lanes four
-// to a column, which writes a column back in fewer wavefronts: 584.
+// Bound by issue slots, two thirds of them at the 19 warps an SM that the tiles
+// leave room for: 41 warp instructions a visibility.  8.9 M visibilities in 8
+// channels, two pairs: 495 us (34 us of memory traffic; 565 with a test for a
+// new cell at every visibility, whose loads then could not run ahead, and the
+// two y taps read one by one).  Lanes four to a column, which writes a column
+// back in fewer wavefronts: 3 % slower.
 template <int NP, int kSpreadWarps>
 __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   extern __shared__ float4 smem_f4[];
@@ -173,12 +175,13 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   for (int h = 0; h < 2; h++)
 #pragma unroll
     for (int q = 0; q < NP; q++) acc[h][q][0] = acc[h][q][1] = 0ull;
-  // this lane's place in the footprint at (bx, by): its x tap and two y taps
-  int bx = 0, by = 0, ox = tx, oy0 = ty, oy1 = ty + 4;
+  // this lane's place in the footprint at (bx, by): its x tap and two y taps,
+  // oy and oy + 4, which lie side by side in the staging
+  int bx = 0, by = 0, ox = tx, oy = ty;
   auto flush = [&]() {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int idx = (by + (h ? oy1 : oy0)) * kTileSide + bx + ox;
+      const int idx = (by + oy + 4 * h) * kTileSide + bx + ox;
 #pragma unroll
       for (int q = 0; q < NP; q++) {
         float4 t = tile[q * kTilePts + idx];
@@ -236,8 +239,8 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
       wl[0] = make_float4(w[0], w[1], w[2], w[3]);
       wl[1] = make_float4(w[4], w[5], w[6], w[7]);
       taps(a, (float)(fv & below) * a.frac, w);
-      wl[2] = make_float4(w[0], w[1], w[2], w[3]);
-      wl[3] = make_float4(w[4], w[5], w[6], w[7]);
+      wl[2] = make_float4(w[0], w[4], w[1], w[5]);
+      wl[3] = make_float4(w[2], w[6], w[3], w[7]);
       float te = 1.0f, to = s;  // T_2q, T_2q+1
 #pragma unroll
       for (int q = 0; q < NP; q++) {
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
     if (lane == 0) prev = cur;
     const uint32_t heads = __ballot_sync(0xffffffffu, base != prev);
     __syncwarp();
-    for (int i = 0; i < cnt; i++) {
+    for (int i = 0; i < cnt;) {
       if ((heads >> i) & 1u) {
         const int next = __shfl_sync(0xffffffffu, base, i);
         const int nx = next & 7, ny = next >> 3;
@@ -263,20 +266,26 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
         bx = nx;
         by = ny;
         ox = (tx - bx) & 7;
-        oy0 = (ty - by) & 7;
-        oy1 = oy0 ^ 4;
+        oy = (ty - by) & 3;
       }
-      const float kx = wts[i * 20 + ox];
-      const float w0 = kx * wts[i * 20 + 8 + oy0], w1 = kx * wts[i * 20 + 8 + oy1];
-      const f32x2 p0 = pack2(w0, w0), p1 = pack2(w1, w1);
+      // the visibilities of this cell
+      const uint32_t later = (heads >> i) & ~1u;
+      const int end = later ? min(cnt, i + __ffs(later) - 1) : cnt;
+#pragma unroll 2
+      for (; i < end; i++) {
+        const float kx = wts[i * 20 + ox];
+        const float2 ky = *reinterpret_cast<const float2*>(wts + i * 20 + 8 + 2 * oy);
+        const float w0 = kx * ky.x, w1 = kx * ky.y;
+        const f32x2 p0 = pack2(w0, w0), p1 = pack2(w1, w1);
 #pragma unroll
-      for (int q = 0; q < NP; q++) {
-        const float4 v = val[q * 32 + i];
-        const f32x2 vp = pack2(v.x, v.y), vm = pack2(v.z, v.w);
-        acc[0][q][0] = fma2(p0, vp, acc[0][q][0]);
-        acc[0][q][1] = fma2(p0, vm, acc[0][q][1]);
-        acc[1][q][0] = fma2(p1, vp, acc[1][q][0]);
-        acc[1][q][1] = fma2(p1, vm, acc[1][q][1]);
+        for (int q = 0; q < NP; q++) {
+          const float4 v = val[q * 32 + i];
+          const f32x2 vp = pack2(v.x, v.y), vm = pack2(v.z, v.w);
+          acc[0][q][0] = fma2(p0, vp, acc[0][q][0]);
+          acc[0][q][1] = fma2(p0, vm, acc[0][q][1]);
+          acc[1][q][0] = fma2(p1, vp, acc[1][q][0]);
+          acc[1][q][1] = fma2(p1, vm, acc[1][q][1]);
+        }
       }
     }
   }

@@ -417,7 +417,8 @@ gv_status gv_run_length_encode_u32(const uint32_t* d_keys, int64_t n, uint32_t* 
  * defaults (only reduction orders change).  Runs a few objective and DChi2
  * evaluations; call it before capturing graphs. */
 typedef struct gv_tune_report {
-  int32_t tc_pair;         /* 1 CTA pairs, 0 single CTAs (-1: DChi2 not on tensor cores) */
+  int32_t tc_pair;         /* 1 CTA pairs, 0 single CTAs (-1: DChi2 not on tensor cores:
+                            * the non-uniform FFT and the SIMT engine) */
   int32_t tc_nsplit;
   int32_t degrid_threads;
   int32_t degrid_blocks;   /* per channel */
