@@ -151,7 +151,7 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
 //
 // Bound by issue slots, two thirds of them at the 19 warps an SM that the tiles
 // leave room for: 41 warp instructions a visibility.  8.9 M visibilities in 8
-// channels, two pairs: 495 us (34 us of memory traffic; 565 with a test for a
+// channels, two pairs: some 470 us (34 us of memory traffic; 565 with a test for a
 // new cell at every visibility, whose loads then could not run ahead, and the
 // two y taps read one by one).  Lanes four to a column, which writes a column
 // back in fewer wavefronts: 3 % slower.
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
       // the visibilities of this cell
       const uint32_t later = (heads >> i) & ~1u;
       const int end = later ? min(cnt, i + __ffs(later) - 1) : cnt;
-#pragma unroll 2
+#pragma unroll 4
       for (; i < end; i++) {
         const float kx = wts[i * 20 + ox];
         const float2 ky = *reinterpret_cast<const float2*>(wts + i * 20 + 8 + 2 * oy);
@@ -1075,9 +1075,13 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   // tiles: the blocks run nearly at once and their longest chain decides, so
   // 8 warps share a piece of 512 (256^2, 104,400 visibilities in 290 tiles:
   // the whole evaluation 89 us, against 110 with 4 warps and pieces of 128).
-  // Otherwise one warp a piece, so that none idles in a thin tile.
+  // Otherwise one warp a piece, so that none idles in a thin tile, and the dense
+  // tiles' pieces do not outlast the rest (2048^2, 8.9 M visibilities in 8
+  // channels, an evaluation: 1754 us with pieces of 1024, 1728 of 512, 1735 of
+  // 256, which cost more slots: 35 M visibilities 365, 366 and 355 evaluations
+  // a second).
   n->warps = R <= (size_t)(16 * P.num_sms) && P.Vgrid >= 64 * (int64_t)R ? 8 : 1;
-  const int T = n->warps == 8 ? 512 : 1024;
+  const int T = 512;
   std::vector<NuTask> tasks;
   const size_t tiles = (size_t)n->nty * n->ntx;
   std::vector<int> slot((size_t)C * tiles, -1);
