@@ -239,7 +239,12 @@ gv_status gv_objective_many(gv_problem* p, const float* const* d_imgs, int32_t c
     P.h_many_cap = need;
   }
   const size_t bytes = sizeof(float) * 2 * (size_t)P.M * (size_t)P.N;
-  const int32_t batch = gv::many_at_once(P);
+  int32_t batch = gv::many_at_once(P);
+  if (batch > 1) {
+    bool room = false;
+    GV_TRY(gv::many_reserve(P, std::min(batch, count), &room));
+    if (!room) batch = 1;
+  }
   if (batch > 1) {
     for (int32_t i = 0; i < count; i += batch)
       GV_TRY(gv::objective_many_launch(P, d_imgs + i, std::min(batch, count - i), flag_opt,

@@ -378,6 +378,7 @@ gv_status side_joined(Problem& P);
 // d_many's end (many_values); GV_ERR_UNSUPPORTED where the terms or the sizes
 // want one image at a time.
 int many_at_once(const Problem& P);
+gv_status many_reserve(Problem& P, int count, bool* ok);
 gv_status objective_many_launch(Problem& P, const float* const* d_imgs, int count, int flag_opt,
                                 double* h_values);
 // Batches: the objectives of several problems (store_res on) in one

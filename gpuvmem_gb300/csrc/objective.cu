@@ -1455,22 +1455,37 @@ int many_at_once(const Problem& P) {
   return (int)std::min<int64_t>(kMaxImages, (int64_t(1) << 27) / grid);
 }
 
+// Room for count images a launch; *ok is false where the memory does not have
+// it (they then go one after another).
+gv_status many_reserve(Problem& P, int count, bool* ok) {
+  *ok = true;
+  if (P.many_cap >= count) return GV_OK;
+  const size_t C = P.chans.size();
+  const size_t each = sizeof(float2) * (size_t)P.M * P.N * C +
+                      sizeof(double) * ((size_t)P.part_stride * (C + kMaxTerms) + kMaxTerms) +
+                      2 * sizeof(uint32_t);
+  GV_CUDA(cudaStreamSynchronize(P.stream));
+  cudaFree(P.d_many);
+  P.d_many = nullptr;
+  P.many_cap = 0;
+  const cudaError_t e = cudaMalloc(&P.d_many, each * count);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    *ok = false;
+    return GV_OK;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "gv_objective_many");
+  P.many_cap = count;
+  GV_CUDA(cudaMemsetAsync(P.d_many, 0, each * count, P.stream));
+  return GV_OK;
+}
+
+// count images, at most as many as reserved
 gv_status objective_many_launch(Problem& P, const float* const* d_imgs, int count, int flag_opt,
                                 double* h_values) {
   const int C = (int)P.chans.size(), nt = (int)P.terms.size();
   const int64_t MN = (int64_t)P.M * P.N;
-  const size_t grid_b = sizeof(float2) * (size_t)MN * C;
   const size_t part_n = (size_t)P.part_stride * (C + kMaxTerms);
-  const size_t each = grid_b + sizeof(double) * (part_n + kMaxTerms) + 2 * sizeof(uint32_t);
-  if (P.many_cap < count) {
-    GV_CUDA(cudaStreamSynchronize(P.stream));
-    cudaFree(P.d_many);
-    P.d_many = nullptr;
-    P.many_cap = 0;
-    GV_CUDA(cudaMalloc(&P.d_many, each * count));
-    P.many_cap = count;
-    GV_CUDA(cudaMemsetAsync(P.d_many, 0, each * count, P.stream));
-  }
   const int cap = P.many_cap;
   float2* grid = static_cast<float2*>(P.d_many);
   double* part = reinterpret_cast<double*>(grid + (size_t)MN * C * cap);
