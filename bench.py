@@ -169,7 +169,7 @@ DCHI2_TRAFFIC_SOURCE = ("ncu capture of k_dchi2_tc, one channel of 2048^2 (bench
 # DRAM bytes of one DChi2 by the default engine at 2048^2 and eight channels
 # (two pairs of w-terms): the grids between its passes and the tiles' sums, from
 # an ncu capture at 8.82M visibilities, besides the 24 B per visibility
-DCHI2_NU_GRID_BYTES_2048_8CH = 1.74e9
+DCHI2_NU_GRID_BYTES_2048_8CH = 1.76e9
 DCHI2_NU_TRAFFIC_SOURCE = ("ncu capture of k_nu_spread, k_nu_rows and k_nu_cols at 2048^2, 8 "
                            "channels and 8.82M visibilities, plus 24 B for every further one")
 

@@ -150,8 +150,8 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
 // to finish adds the slots up, in order, into the first.
 //
 // Bound by issue slots, two thirds of them at the 19 warps an SM that the tiles
-// leave room for: 41 warp instructions a visibility.  8.9 M visibilities in 8
-// channels, two pairs: some 470 us (34 us of memory traffic; 565 with a test for a
+// leave room for: 40 warp instructions a visibility.  8.8 M visibilities in 8
+// channels, two pairs: 453 us (87 us of memory traffic; 563 with a test for a
 // new cell at every visibility, whose loads then could not run ahead, and the
 // two y taps read one by one).  Lanes four to a column, which writes a column
 // back in fewer wavefronts: 3 % slower.
