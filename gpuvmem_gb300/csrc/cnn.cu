@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kGemmThreads, Op::kPixelRows && BN == 64 ? 3 :
   const int nch = kend > kbeg ? (kend - kbeg + kBK - 1) / kBK : 0;
 
   const int grp = tid % kGroups;  // T is a multiple of both
-  int4 at = make_int4(0, 0, 0, 0);  // the group's {offset, y, x, batch}
+  Pixel at{0, 0, 0, 0};             // the group's first
   const int mg = m0 + grp * 8;
   if (KS > 0 && kRows && mg < M) at = op.pixel(mg);  // M is a multiple of eight
   // the first unit that touches the tile's rows from row0 on
@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(kGemmThreads, Op::kPixelRows && BN == 64 ? 3 :
       if (Op::kFlip) dy = -dy;
       if (in && tid + i * T < kUnits * kGroups && u * max(KS, 1) < rows &&
           (unsigned)(at.y + dy) < (unsigned)op.H)
-        ra[i].template load<KS == 3>(op.src() + at.x + ch * op.H * op.W + dy * op.W, at.z, op.W);
+        ra[i].template load<KS == 3>(op.src() + at.off + (int64_t)ch * (op.H * op.W) + dy * op.W,
+                                     at.x, op.W);
     }
     if constexpr (kmajor) {
 #pragma unroll
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(kGemmThreads, Op::kPixelRows && BN == 64 ? 3 :
         rb[i].clear();
         const int r = (tid + i * T) / kGroups;
         if (in && r < BN && n0 + r < N)
-          rb[i].template load<false>(op.grad_row(n0 + r, at), at.z, op.W);
+          rb[i].template load<false>(op.grad_row(n0 + r, at), at.x, op.W);
       }
     } else if (kRows) {
       if (op.packed) {

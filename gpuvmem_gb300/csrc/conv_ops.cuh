@@ -1,5 +1,7 @@
 // Operands of the convolution GEMMs (k_gemm, cnn.cu): where the elements of the
-// three products lie in the tensors.
+// three products lie in the tensors.  A tensor may hold 2^31 elements and more
+// (the 48-channel concatenation of a 2048^2 network at batch 11), so offsets
+// are 64 bits wide; a batch's pixels and a side's stay in 32.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,6 +21,17 @@ __device__ __host__ inline bool rows_of_eight(const float* p, int W) {
   return W % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
 }
 
+// A pixel of an operand: its offset in the first channel, row, column, batch.
+struct Pixel {
+  int64_t off;
+  int y, x, b;
+};
+// A row of a result: its number and the offset of its pixel in channel 0.
+struct OutRow {
+  int m;
+  int64_t off;
+};
+
 // forward: y = act(conv(x) + bias); with split-K (part set) each split
 // stores its partial sum to part[split][n][m] and k_conv_fwd_finish adds
 // the splits, the bias and the activation
@@ -37,11 +50,10 @@ struct ConvFwdOp {
   int M;
   bool fast;
   __device__ const float* src() const { return x; }
-  // a pixel: {offset of its plane set's first channel and itself, y, x}
-  __device__ int4 pixel(int m) const {
+  __host__ __device__ Pixel pixel(int m) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW, y0 = r / W;
-    return make_int4((b * xC + xc0) * HW + r, y0, r - y0 * W, 0);
+    return {(int64_t)(b * xC + xc0) * HW + r, y0, r - y0 * W, b};
   }
   __device__ float a(int m, int k) const {
     const int HW = H * W;
@@ -52,16 +64,15 @@ struct ConvFwdOp {
     return x[((size_t)(b * xC + xc0 + cin) * H + yy) * W + xx];
   }
   __device__ float b(int k, int n) const { return w[(size_t)n * Cin * ks * ks + k]; }
-  __device__ const float* grad_row(int, const int4&) const { return nullptr; }
-  // where row m of the result goes: {m, offset of its pixel in y}
-  __device__ int2 row(int m) const {
+  __device__ const float* grad_row(int, const Pixel&) const { return nullptr; }
+  __host__ __device__ OutRow row(int m) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW;
-    return make_int2(m, (b * yC + yc0) * HW + r);
+    return {m, (int64_t)(b * yC + yc0) * HW + r};
   }
-  __device__ void store(const int2& at, int n, int cnt, float (&v)[8], int split) const {
-    float* out = part ? part + ((size_t)split * Cout + n) * M + at.x
-                      : y + (size_t)at.y + (size_t)n * H * W;
+  __device__ void store(const OutRow& at, int n, int cnt, float (&v)[8], int split) const {
+    float* out = part ? part + ((size_t)split * Cout + n) * M + at.m
+                      : y + at.off + (size_t)n * H * W;
     const size_t step = part ? (size_t)M : (size_t)H * W;
     if (!part) {
 #pragma unroll
@@ -92,10 +103,10 @@ struct ConvBwdDataOp {
   int Cin, Cout, H, W, ks;
   bool fast;
   __device__ const float* src() const { return dz; }
-  __device__ int4 pixel(int m) const {
+  __host__ __device__ Pixel pixel(int m) const {
     const int HW = H * W;
     const int b = m / HW, r = m - b * HW, y0 = r / W;
-    return make_int4((b * zC + zc0) * HW + r, y0, r - y0 * W, 0);
+    return {(int64_t)(b * zC + zc0) * HW + r, y0, r - y0 * W, b};
   }
   __device__ float a(int m, int k) const {
     const int HW = H * W;
@@ -109,7 +120,7 @@ struct ConvBwdDataOp {
     const int kk = ks * ks, co = k / kk, t = k - co * kk;
     return w[((size_t)co * Cin + n) * kk + t];
   }
-  __device__ const float* grad_row(int, const int4&) const { return nullptr; }
+  __device__ const float* grad_row(int, const Pixel&) const { return nullptr; }
   __device__ int2 row(int m) const {
     const int HW = H * W;
     const int b = m / HW;
@@ -144,11 +155,10 @@ struct ConvBwdWeightOp {
   bool fast;
   static constexpr const uint4* packed = nullptr;
   __device__ const float* src() const { return x; }
-  // eight pixels: {their offset in x's first channel, y, x, batch}
-  __device__ int4 pixel(int k) const {
+  __host__ __device__ Pixel pixel(int k) const {
     const int HW = H * W;
     const int b = k / HW, r = k - b * HW, y0 = r / W;
-    return make_int4((b * xC + xc0) * HW + r, y0, r - y0 * W, b);
+    return {(int64_t)(b * xC + xc0) * HW + r, y0, r - y0 * W, b};
   }
   __device__ float a(int m, int k) const {
     const int kk = ks * ks, cin = m / kk, t = m - cin * kk;
@@ -163,8 +173,8 @@ struct ConvBwdWeightOp {
     const int b = k / HW, r = k - b * HW;
     return dz[(size_t)(b * zC + zc0 + n) * HW + r];
   }
-  __device__ const float* grad_row(int n, const int4& p) const {
-    return dz + (size_t)(p.w * zC + zc0 + n) * H * W + p.y * W + p.z;
+  __device__ const float* grad_row(int n, const Pixel& p) const {
+    return dz + (size_t)(p.b * zC + zc0 + n) * H * W + p.y * W + p.x;
   }
   __device__ int row(int m) const { return m; }
   __device__ void store(int m, int n, int cnt, float (&v)[8], int split) const {
