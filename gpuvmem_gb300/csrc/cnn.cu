@@ -369,7 +369,7 @@ __global__ void k_sum_splits(size_t n, int nsplit, const float* __restrict__ par
 // db[c] = sum over pixels of dz, as 256 threads striding over each plane of
 // the batch add it: thread t takes pixels t, t + 256, ..., then a butterfly
 // within each warp and one over the warps.  A block stands for one of those
-// 8 warps (blockIdx.x), so that a channel's sum is not one block's: all its
+// 8 warps (blockIdx.x % 8), so that a channel's sum is not one block's: all its
 // threads bring the next 128 steps of the warp's 32 running sums into shared
 // memory while the first warp adds the last ones.  16 channels of 256^2,
 // batch 8, in one block each: some 600 us; so: 30 us.
@@ -378,9 +378,9 @@ __global__ void __launch_bounds__(256) k_bias_grad(int B, int HW, View dz, float
                                                    uint32_t* __restrict__ done,
                                                    float* __restrict__ db) {
   __shared__ float stage[2][kBiasSteps][32];
-  const int c = blockIdx.y, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int c = blockIdx.x / 8, lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const int S = (HW + 255) / 256, total = B * S;  // steps a plane, of the batch
-  const int t0 = blockIdx.x * 32 + lane;           // the thread stood for
+  const int t0 = blockIdx.x % 8 * 32 + lane;       // the thread stood for
   float next[kBiasSteps / 8];
   auto fetch = [&](int s0) {
 #pragma unroll
@@ -404,10 +404,10 @@ __global__ void __launch_bounds__(256) k_bias_grad(int B, int HW, View dz, float
   }
   if (row == 0) {
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) part[c * 8 + blockIdx.x] = sum;
+    if (lane == 0) part[blockIdx.x] = sum;
   }
-  if (!last_block_done(done, gridDim.x * gridDim.y)) return;
-  for (int k = threadIdx.x; k < (int)gridDim.y; k += blockDim.x) {
+  if (!last_block_done(done, gridDim.x)) return;
+  for (int k = threadIdx.x; k < (int)gridDim.x / 8; k += blockDim.x) {
     float w[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) w[i] = __ldcg(part + k * 8 + i);
@@ -415,10 +415,11 @@ __global__ void __launch_bounds__(256) k_bias_grad(int B, int HW, View dz, float
   }
 }
 
-// The resampling kernels: blockIdx.y = batch and channel, a thread per pixel
-// of the smaller side.  y = 2x2 average of x (x is H x W, y is H/2 x W/2)
-__global__ void __launch_bounds__(256) k_pool2(int C, int H, int W, View x, View y) {
-  const int c = blockIdx.y % C, b = blockIdx.y / C, Ho = H / 2, Wo = W / 2;
+// The resampling kernels: p0 + blockIdx.y = batch and channel (by_planes), a
+// thread per pixel of the smaller side.  y = 2x2 average of x (x is H x W, y is
+// H/2 x W/2)
+__global__ void __launch_bounds__(256) k_pool2(int p0, int C, int H, int W, View x, View y) {
+  const int plane = p0 + blockIdx.y, c = plane % C, b = plane / C, Ho = H / 2, Wo = W / 2;
   const float* xp = x.p + (size_t)(b * x.C + x.c0 + c) * H * W;
   float* yp = y.p + (size_t)(b * y.C + y.c0 + c) * Ho * Wo;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Ho * Wo; i += gridDim.x * blockDim.x) {
@@ -431,9 +432,9 @@ __global__ void __launch_bounds__(256) k_pool2(int C, int H, int W, View x, View
 
 // dx += dy / 4 broadcast over each 2x2 block, then masked by the ReLU of act
 // (dx's activation)
-__global__ void __launch_bounds__(256) k_pool2_bwd(int C, int H, int W, View dy, View dx,
-                                                   View act) {
-  const int c = blockIdx.y % C, b = blockIdx.y / C, Ho = H / 2, Wo = W / 2;
+__global__ void __launch_bounds__(256) k_pool2_bwd(int p0, int C, int H, int W, View dy,
+                                                   View dx, View act) {
+  const int plane = p0 + blockIdx.y, c = plane % C, b = plane / C, Ho = H / 2, Wo = W / 2;
   const float* gp = dy.p + (size_t)(b * dy.C + dy.c0 + c) * Ho * Wo;
   float* xp = dx.p + (size_t)(b * dx.C + dx.c0 + c) * H * W;
   const float* ap = act.p + (size_t)(b * act.C + act.c0 + c) * H * W;
@@ -452,8 +453,8 @@ __global__ void __launch_bounds__(256) k_pool2_bwd(int C, int H, int W, View dy,
 }
 
 // y = nearest 2x upsample of x (x is H x W)
-__global__ void __launch_bounds__(256) k_up2(int C, int H, int W, View x, View y) {
-  const int c = blockIdx.y % C, b = blockIdx.y / C, Wo = 2 * W;
+__global__ void __launch_bounds__(256) k_up2(int p0, int C, int H, int W, View x, View y) {
+  const int plane = p0 + blockIdx.y, c = plane % C, b = plane / C, Wo = 2 * W;
   const float* xp = x.p + (size_t)(b * x.C + x.c0 + c) * H * W;
   float* yp = y.p + (size_t)(b * y.C + y.c0 + c) * 4 * H * W;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H * W; i += gridDim.x * blockDim.x) {
@@ -465,8 +466,9 @@ __global__ void __launch_bounds__(256) k_up2(int C, int H, int W, View x, View y
 }
 
 // dx = sum of dy over each 2x2 block (dx is H x W), masked by the ReLU of act
-__global__ void __launch_bounds__(256) k_up2_bwd(int C, int H, int W, View dy, View dx, View act) {
-  const int c = blockIdx.y % C, b = blockIdx.y / C, Wo = 2 * W;
+__global__ void __launch_bounds__(256) k_up2_bwd(int p0, int C, int H, int W, View dy, View dx,
+                                                 View act) {
+  const int plane = p0 + blockIdx.y, c = plane % C, b = plane / C, Wo = 2 * W;
   const float* gp = dy.p + (size_t)(b * dy.C + dy.c0 + c) * 4 * H * W;
   float* xp = dx.p + (size_t)(b * dx.C + dx.c0 + c) * H * W;
   const float* ap = act.p + (size_t)(b * act.C + act.c0 + c) * H * W;
@@ -596,9 +598,17 @@ gv_status launch_gemm(const Ctx& c, const Op& op, int M, int N, int K, int nspli
   return launch_gemm_bn<Op, 256>(c, op, M, N, K, nsplit);
 }
 
-// grid of the per-channel kernels: n pixels a channel, `planes` of them
-inline dim3 plane_grid(int n, int planes) {
-  return dim3((unsigned)std::min((n + 255) / 256, 64), (unsigned)planes);
+// launch(grid, first plane) of a resampling kernel: n pixels a plane, as many
+// planes at once as a grid's second dimension takes
+template <class F>
+gv_status by_planes(const char* name, int n, int planes, F&& launch) {
+  constexpr int kMost = 65535;
+  for (int p0 = 0; p0 < planes; p0 += kMost) {
+    launch(dim3((unsigned)std::min((n + 255) / 256, 64), (unsigned)std::min(planes - p0, kMost)),
+           p0);
+    GV_LAUNCH(name);
+  }
+  return GV_OK;
 }
 
 inline int ew_blocks(size_t n, const Ctx& c) {
@@ -655,7 +665,7 @@ gv_status conv_backward_weight(const Ctx& c, View x, View dz, float* dw, float* 
   k_sum_splits<<<(unsigned)((wn + 255) / 256), 256, 0, c.stream>>>(wn, nz, c.part, dw);
   GV_LAUNCH("k_sum_splits");
   // the splits' scratch is free again
-  k_bias_grad<<<dim3(8, Cout), 256, 0, c.stream>>>(B, H * W, dz, c.part, c.done, db);
+  k_bias_grad<<<8 * Cout, 256, 0, c.stream>>>(B, H * W, dz, c.part, c.done, db);
   GV_LAUNCH("k_bias_grad");
   return GV_OK;
 }
@@ -901,16 +911,17 @@ struct UNet {
       GV_TRY(layer_forward(c, enc_layer(l, 0), View{in[l], ci, 0}, View{a[l], C(l), 0}, B, s));
       GV_TRY(layer_forward(c, enc_layer(l, 1), View{a[l], C(l), 0}, enc_view(l), B, s));
       if (l + 1 < L) {
-        k_pool2<<<plane_grid(s * s / 4, B * C(l)), 256, 0, stream>>>(C(l), s, s, enc_view(l),
-                                                                     View{in[l + 1], C(l), 0});
-        GV_LAUNCH("k_pool2");
+        GV_TRY(by_planes("k_pool2", s * s / 4, B * C(l), [&](dim3 grid, int p0) {
+          k_pool2<<<grid, 256, 0, stream>>>(p0, C(l), s, s, enc_view(l), View{in[l + 1], C(l), 0});
+        }));
       }
     }
     for (int l = L - 2; l >= 0; l--) {
       const int s = S(l), cc = C(l + 1) + C(l);
-      k_up2<<<plane_grid(s * s / 4, B * C(l + 1)), 256, 0, stream>>>(
-          C(l + 1), s / 2, s / 2, dec_view(l + 1), View{cat[l], cc, 0});
-      GV_LAUNCH("k_up2");
+      GV_TRY(by_planes("k_up2", s * s / 4, B * C(l + 1), [&](dim3 grid, int p0) {
+        k_up2<<<grid, 256, 0, stream>>>(p0, C(l + 1), s / 2, s / 2, dec_view(l + 1),
+                                        View{cat[l], cc, 0});
+      }));
       GV_TRY(layer_forward(c, dec_layer(l, 0), View{cat[l], cc, 0}, View{b[l], C(l), 0}, B, s));
       GV_TRY(layer_forward(c, dec_layer(l, 1), View{b[l], C(l), 0}, dec_view(l), B, s));
     }
@@ -963,17 +974,19 @@ struct UNet {
       GV_TRY(layer_backward(c, dec_layer(l, 1), bv, ddec_view(l), dbv, bv, B, s));
       GV_TRY(layer_backward(c, dec_layer(l, 0), View{cat[l], cc, 0}, dbv, dcatv, none, B, s));
       // the upsampled part of the concat feeds dec_{l+1}
-      k_up2_bwd<<<plane_grid(s * s / 4, B * C(l + 1)), 256, 0, stream>>>(
-          C(l + 1), s / 2, s / 2, dcatv, ddec_view(l + 1), dec_view(l + 1));
-      GV_LAUNCH("k_up2_bwd");
+      GV_TRY(by_planes("k_up2_bwd", s * s / 4, B * C(l + 1), [&](dim3 grid, int p0) {
+        k_up2_bwd<<<grid, 256, 0, stream>>>(p0, C(l + 1), s / 2, s / 2, dcatv, ddec_view(l + 1),
+                                            dec_view(l + 1));
+      }));
     }
     for (int l = L - 1; l >= 0; l--) {
       const int s = S(l), ci = l == 0 ? cin : C(l - 1);
       if (l + 1 < L) {
         // enc_l also feeds the pool of level l+1: add that gradient
-        k_pool2_bwd<<<plane_grid(s * s / 4, B * C(l)), 256, 0, stream>>>(
-            C(l), s, s, View{din[l + 1], C(l), 0}, denc_view(l), enc_view(l));
-        GV_LAUNCH("k_pool2_bwd");
+        GV_TRY(by_planes("k_pool2_bwd", s * s / 4, B * C(l), [&](dim3 grid, int p0) {
+          k_pool2_bwd<<<grid, 256, 0, stream>>>(p0, C(l), s, s, View{din[l + 1], C(l), 0},
+                                                denc_view(l), enc_view(l));
+        }));
       }
       const View av{a[l], C(l), 0}, dav{da[l], C(l), 0};
       GV_TRY(layer_backward(c, enc_layer(l, 1), av, denc_view(l), dav, av, B, s));
