@@ -648,6 +648,12 @@ gv_status conv_backward_data(const Ctx& c, View dz, const float* w, const uint4*
   return launch_gemm(c, op, B * H * W, Cin, Cout * ks * ks);
 }
 
+// FP32 scratch of a weight gradient: a whole split's partial sums, or the bias
+// gradient's 8 a channel
+inline size_t weight_scratch(int Cin, int Cout, int ks) {
+  return (size_t)Cout * std::max<size_t>((size_t)Cin * ks * ks, 8);
+}
+
 gv_status conv_backward_weight(const Ctx& c, View x, View dz, float* dw, float* db, int B,
                                int Cin, int Cout, int H, int W, int ks) {
   const int M = Cin * ks * ks, N = Cout, K = B * H * W;
@@ -814,6 +820,8 @@ struct UNet {
     GV_TRY(alloc(&out, B * (size_t)H * W));
     GV_TRY(alloc(&dout, B * (size_t)H * W));
     part_floats = (size_t)4 << 20;  // 16 MB of split-K partials
+    for (const Layer& ly : layers)
+      part_floats = std::max(part_floats, weight_scratch(ly.cin, ly.cout, ly.ks));
     GV_TRY(alloc(&part, part_floats));
     GV_CUDA(cudaMalloc(&loss_part, sizeof(double) * 1024));
     allocs.push_back(loss_part);
@@ -1213,7 +1221,8 @@ gv_status gv_conv2d_backward(const float* x, const float* w, const float* dz, fl
   }
   uint32_t* err = nullptr;
   float* part = nullptr;
-  const size_t part_floats = (size_t)4 << 20;
+  const size_t part_floats =
+      std::max((size_t)4 << 20, gv::cnn::weight_scratch(Cin, Cout, ks));
   GV_CUDA(cudaMalloc(&err, 2 * sizeof(uint32_t)));
   GV_CUDA(cudaMalloc(&part, sizeof(float) * part_floats));
   GV_CUDA(cudaMemsetAsync(err, 0, 2 * sizeof(uint32_t), (cudaStream_t)stream));

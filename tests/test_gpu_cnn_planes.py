@@ -61,3 +61,21 @@ def test_bias_gradient_of_65536_channels():
     assert torch.equal(db, dz.sum((0, 2, 3)))
     assert torch.equal(dw.view(-1), (dz * x).sum((0, 2, 3)))
     assert torch.equal(dx, dz.sum(1, keepdim=True))
+
+
+def test_weight_gradient_of_more_weights_than_the_splits_scratch():
+    """512 x 1024 channels: 4.7M weights, beyond the 4M floats that the splits
+    otherwise share.  Operands -1, 0 and 1: exact sums."""
+    import torch
+    from gpuvmem_gb300 import unet
+    g = torch.Generator().manual_seed(4)
+    x = torch.randint(-1, 2, (1, 512, 8, 8), generator=g).float().cuda()
+    dz = torch.randint(-1, 2, (1, 1024, 8, 8), generator=g).float().cuda()
+    w = torch.randint(-1, 2, (1024, 512, 3, 3), generator=g).float().cuda()
+    dx, dw, db = unet.conv2d_backward(x, w, dz, 3)
+    ref = torch.nn.functional.conv2d(x.double().transpose(0, 1), dz.double().transpose(0, 1),
+                                     padding=1).transpose(0, 1)
+    assert torch.equal(dw.double(), ref)
+    assert torch.equal(db, dz.sum((0, 2, 3)))
+    assert torch.equal(dx.double(), torch.nn.functional.conv_transpose2d(dz.double(), w.double(),
+                                                                         padding=1))
