@@ -140,7 +140,9 @@ __global__ void k_prepare_vis(int64_t n, int64_t off, int chan, float freq,
   const float GV = (float)(w * dy * dy * 0.5);
   ph_u[g] = make_uint4(FU, FV, __float_as_uint(GU), __float_as_uint(GV));
   wl_u[g] = (float)w;
-  atomicMax(maxw, __float_as_uint(fabsf((float)w)));
+  // not a NaN, whose bits are above all others (a flagged visibility's, say)
+  const float aw = fabsf((float)w);
+  if (aw >= 0.0f) atomicMax(maxw, __float_as_uint(aw));
   // sort key: the visibility's cell, or (tile_sh >= 0: the non-uniform FFT's
   // order) its 8 x 8 tile of the doubled grid folded into u >= 0, then its
   // cell in the tile; the model grid's cells of a tile lie together either way
