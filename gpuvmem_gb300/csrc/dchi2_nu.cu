@@ -513,7 +513,8 @@ __global__ void __launch_bounds__(RowShape<LG>::kBlock, 1024 / RowShape<LG>::kBl
 
 // Per pixel and channel (blockIdx.y) the factor of the sum that does not
 // depend on the image: - fg_scale, beam, GCF and 1/V as the direct engines
-// apply them, 0 outside the mask.  Like the coefficients below it is fixed by
+// apply them, 0 outside the mask and for a channel without visibilities
+// (whose 1/V times its empty sum would be a NaN).  Like the coefficients below it is fixed by
 // the problem, made once and laid out column by column ([j][i]), as the
 // column pass reads it.
 struct FactorArgs {
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(256) k_nu_factors(FactorArgs a) {
   const int j = (int)(q / a.N), i = (int)(q - (int64_t)j * a.N);
   const int64_t px = (int64_t)a.N * i + j;
   float f = 0.0f;
-  if (a.mask[px] & kMaskIn) {
+  if ((a.mask[px] & kMaskIn) && a.chnvis[c] > 0) {
     f = -(a.fg_scale * attenuation_xy(a.beam_x[j], a.beam_y[i], a.chfreq[c], a.D, a.pbf, a.pbcut,
                                       a.pb));
     if (a.gcf) f *= a.gcf[px];

@@ -38,3 +38,21 @@ def test_flagged_visibility_without_a_w(n):
     uvw[17, 2] = np.nan
     got = _gradient(dataclasses.replace(data, weight=w, uvw_m=uvw))
     assert ref.any() and torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("empty", [0, 1, 2])
+def test_channel_without_visibilities(empty):
+    """It adds nothing to a normalised gradient (1/V is not taken), as in the
+    GEMM engine; the other channels' sums agree with it to the GEMM's accuracy."""
+    data = _data(128, nchan=3)
+    off = data.chan_off
+    keep = np.ones(data.weight.size, bool)
+    keep[off[empty]:off[empty + 1]] = False
+    sizes = np.diff(off)
+    sizes[empty] = 0
+    data = dataclasses.replace(data, uvw_m=data.uvw_m[keep], vo=data.vo[keep],
+                               weight=data.weight[keep],
+                               chan_off=np.concatenate([[0], np.cumsum(sizes)]).astype(off.dtype))
+    got, ref = (_gradient(data, engine=e, normalize=True)[0] for e in (0, 2))
+    assert ref.abs().max() > 0
+    assert (got - ref).abs().max() <= 1e-5 * ref.abs().max()
