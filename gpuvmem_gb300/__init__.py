@@ -103,7 +103,8 @@ EXPORTS = ["gv_problem_create", "gv_problem_destroy", "gv_problem_info_get",
            "gv_problem_set_stream", "gv_noise_image", "gv_initial_image", "gv_chi2", "gv_dchi2",
            "gv_dchi2_channel", "gv_prior_value", "gv_prior_gradient", "gv_objective",
            "gv_gradient", "gv_optimize", "gv_dirty_image", "gv_residuals", "gv_last_error",
-           "gv_version", "gv_launch_count"]
+           "gv_version", "gv_launch_count",
+           "gv_problem_dchi2_pairs"]
 
 
 def lib():
@@ -121,6 +122,7 @@ def lib():
         "gv_problem_create": [C.POINTER(ProblemDesc), C.POINTER(vp)],
         "gv_problem_destroy": [vp],
         "gv_problem_info_get": [vp, C.POINTER(ProblemInfo)],
+        "gv_problem_dchi2_pairs": [vp, C.POINTER(i32)],
         "gv_problem_set_stream": [vp, vp],
         "gv_noise_image": [vp, vp],
         "gv_initial_image": [vp, vp],
@@ -275,6 +277,14 @@ class Problem:
         inf = ProblemInfo()
         check(lib().gv_problem_info_get(self.h, C.byref(inf)))
         return inf
+
+    @property
+    def dchi2_pairs(self) -> int:
+        """Complex FFTs per channel of the non-uniform FFT that DChi2 runs as;
+        0 where the direct sums of info.dchi2_engine run."""
+        v = C.c_int32()
+        check(lib().gv_problem_dchi2_pairs(self.h, C.byref(v)))
+        return v.value
 
     def _img(self):
         import torch

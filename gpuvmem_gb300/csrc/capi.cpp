@@ -109,6 +109,16 @@ gv_status gv_problem_info_get(const gv_problem* p, gv_problem_info* info) {
   return GV_OK;
 }
 
+gv_status gv_problem_dchi2_pairs(const gv_problem* p, int32_t* pairs) {
+  GV_CHECK_PROBLEM(p);
+  if (!pairs) {
+    gv::set_error("null pairs");
+    return GV_ERR_INVALID;
+  }
+  *pairs = gv::nu_pairs(p->P);
+  return GV_OK;
+}
+
 gv_status gv_problem_set_stream(gv_problem* p, void* stream) {
   GV_CHECK_PROBLEM(p);
   p->P.stream = (cudaStream_t)stream;

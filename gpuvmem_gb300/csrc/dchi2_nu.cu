@@ -983,6 +983,8 @@ gv_status nu_finish(Problem& P) {
   return GV_OK;
 }
 
+int nu_pairs(const Problem& P) { return P.nu ? P.nu->pairs : 0; }
+
 uint32_t nu_tiles_x(int N) { return (uint32_t)(N / 8 + 1); }
 
 // Builds the plan of P (P.nu stays null where the direct sums are to run):

@@ -437,6 +437,7 @@ gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result
 gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw);
 gv_status nu_finish(Problem& P);
 void nu_free(Problem& P);
+int nu_pairs(const Problem& P);  // of its w series; 0: direct sums
 uint32_t nu_tiles_x(int N);  // tiles per row of the doubled grid's half plane
 // the engine P runs DChi2 with
 gv_status dchi2_run(Problem& P, const float* d_img, int flag_opt, float* d_result,

@@ -147,13 +147,16 @@ typedef struct gv_problem_info {
   int64_t mask_pixels;   /* pixels with noise < noise_cut */
   int32_t dchi2_engine;  /* direct-sum engine of the problem (1 SIMT, 2 GEMM);
                             created with 0, it runs where the non-uniform
-                            FFT does not */
+                            FFT does not (gv_problem_dchi2_pairs) */
   int32_t nterms;        /* terms kept (lambda != 0) */
 } gv_problem_info;
 
 gv_status gv_problem_create(const gv_problem_desc* desc, gv_problem** out);
 gv_status gv_problem_destroy(gv_problem* p);
 gv_status gv_problem_info_get(const gv_problem* p, gv_problem_info* info);
+/* Complex FFTs per channel (pairs of w-terms, 1 to 4) of the non-uniform FFT
+ * that DChi2 runs as, or 0 where the direct sums of info.dchi2_engine run. */
+gv_status gv_problem_dchi2_pairs(const gv_problem* p, int32_t* pairs);
 /* cudaStream_t passed as void*; NULL = the legacy default stream */
 gv_status gv_problem_set_stream(gv_problem* p, void* stream);
 /* Copies the noise image (M*N floats) to a device buffer. */

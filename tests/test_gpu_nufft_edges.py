@@ -56,3 +56,43 @@ def test_channel_without_visibilities(empty):
     got, ref = (_gradient(data, engine=e, normalize=True)[0] for e in (0, 2))
     assert ref.abs().max() > 0
     assert (got - ref).abs().max() <= 1e-5 * ref.abs().max()
+
+
+def _pairs_of_the_series(data):
+    """Pairs of terms after which the w series leaves no more than 3e-7
+    (2 (A/2)^2p / (2p)! with A the largest phase), or 0 beyond 4."""
+    lam = np.repeat(299792458.0 / np.asarray(data.freqs, np.float64), np.diff(data.chan_off))
+    w = np.abs(data.uvw_m[:, 2] / lam).max()
+    half = [max(x, data.N - 1 - x) * abs(d) * np.pi / 180.0
+            for x, d in ((int(data.xobs), data.DELTAX), (int(data.yobs), data.DELTAY))]
+    r2 = half[0] ** 2 + half[1] ** 2
+    a = 2.0 * np.pi * w * r2 / (1.0 + np.sqrt(1.0 - r2))
+    for p in range(1, 5):
+        if 2.0 * np.prod([0.5 * a / k for k in range(1, 2 * p + 1)]) <= 3e-7:
+            return p
+    return 0
+
+
+def test_engine_that_runs():
+    """The pairs reported are the series' own, from 1 to 4, and 0 where more are
+    needed or a direct engine is asked for."""
+    import gpuvmem_gb300 as gv
+    seen = set()
+    for wscale in (0.0, 1.0, 30.0, 300.0, 1500.0, 2600.0, 1e5):
+        data = _data(128, seed=5)
+        data = dataclasses.replace(data, uvw_m=data.uvw_m * np.array([1.0, 1.0, wscale]))
+        want = _pairs_of_the_series(data)
+        prob = gv.Problem(data, [gv.term("Chi2", 1.0)])
+        assert prob.dchi2_pairs == want
+        seen.add(want)
+        prob.close()
+    assert seen == {0, 1, 2, 3, 4}
+    for engine in (1, 2):
+        assert gv.Problem(_data(128), [gv.term("Chi2", 1.0)], engine=engine).dchi2_pairs == 0
+
+
+@pytest.mark.parametrize("n", [16, 64, 256, 1024])
+def test_default_engine(n):
+    import gpuvmem_gb300 as gv
+    prob = gv.Problem(_data(n, nchan=2), [gv.term("Chi2", 1.0)])
+    assert 1 <= prob.dchi2_pairs <= 4
