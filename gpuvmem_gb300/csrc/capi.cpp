@@ -32,6 +32,7 @@ void add_launches(int64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed
 void set_error(const std::string& msg) { g_last_error = msg; }
 
 gv_status cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next call's launches start without it
   g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
   if (e == cudaErrorMemoryAllocation) return GV_ERR_NOMEM;
   return GV_ERR_CUDA;
