@@ -69,6 +69,10 @@ struct NuPlan {
   float* d_fac = nullptr;      // [C][MN] image-independent factors (k_nu_factors)
   float* d_part = nullptr;     // sums of shared column blocks, N >= 1024
   float coef[4][12];           // the taps' polynomials (tap_polynomials)
+  // from nu_plan to nu_build
+  std::vector<NuTask> h_tasks;
+  std::vector<int> h_slot;
+  size_t max_slots = 0, max_ch = 0;  // tasks and channels of the largest group
 };
 
 namespace {
@@ -947,6 +951,12 @@ double max_depth(const Problem& P) {
   return r2 < 1.0 ? r2 / (1.0 + std::sqrt(1.0 - r2)) : 1.0;
 }
 
+// a task's slot, and a channel's grid
+size_t slot_bytes(const NuPlan& n) { return sizeof(float4) * kTilePts * n.pairs; }
+size_t plane_bytes(const Problem& P) {
+  return sizeof(float2) * (size_t)P.nu->pairs * P.nu->nrow * P.N;
+}
+
 }  // namespace
 
 void nu_free(Problem& P) {
@@ -966,31 +976,16 @@ void nu_free(Problem& P) {
   P.nu = nullptr;
 }
 
-// The pixels' w-term coefficients and factors, once the beam tables (the
-// pixels' offsets), the mask and the channels' tables are in place.
-gv_status nu_finish(Problem& P) {
-  if (!P.nu) return GV_OK;
-  const NuPlan& n = *P.nu;
-  const int64_t MN = (int64_t)P.N * P.N;
-  k_nu_coefficients<<<(unsigned)((MN + 255) / 256), 256, 0, P.stream>>>(
-      P.N, n.pairs, (float)(2.0 * kPiD * n.wmax), P.d_beam_x, P.d_beam_y, n.d_corr, n.d_coef);
-  GV_LAUNCH("k_nu_coefficients");
-  const FactorArgs fa{P.N, P.normalize, P.pb, P.D, P.pbf, P.pbcut, P.fg_scale, P.d_beam_x,
-                      P.d_beam_y, P.d_chfreq, P.d_chnvis, P.d_mask, P.d_gcf, n.d_fac};
-  k_nu_factors<<<dim3((unsigned)((MN + 255) / 256), (unsigned)P.chans.size()), 256, 0,
-                 P.stream>>>(fa);
-  GV_LAUNCH("k_nu_factors");
-  return GV_OK;
-}
-
 int nu_pairs(const Problem& P) { return P.nu ? P.nu->pairs : 0; }
 
 uint32_t nu_tiles_x(int N) { return (uint32_t)(N / 8 + 1); }
 
-// Builds the plan of P (P.nu stays null where the direct sums are to run):
+// The plan of P on the host (P.nu stays null where the direct sums are to run):
 // keys are the sorted (channel << 32 | tile << 6 | cell in tile) of all
-// visibilities, all ones in the low word for those left out.
-gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
+// visibilities, all ones in the low word for those left out.  Its device
+// buffers come last of a problem's (nu_build): the direct sums, which need less
+// memory, run where there is no room for them, nor for the scratch here.
+gv_status nu_plan(Problem& P, const unsigned long long* d_keys, double maxw) {
   const int C = (int)P.chans.size(), N = P.N;
   if (P.Vgrid <= 0 || P.V >= (int64_t(1) << 31)) return GV_OK;
   const double A = 2.0 * kPiD * maxw * max_depth(P);
@@ -1013,10 +1008,16 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     unsigned long long* dk = nullptr;
     uint32_t* ds = nullptr;
     const size_t tb = scan_scratch(V);
+    bool room = true;
+    auto take = [&](void* p, size_t bytes) -> gv_status {
+      const cudaError_t e = cudaMalloc(static_cast<void**>(p), bytes);
+      room = e != cudaErrorMemoryAllocation;
+      return e == cudaSuccess ? GV_OK : cuda_fail(e, "nu_plan");
+    };
     auto work = [&]() -> gv_status {
-      GV_CUDA(cudaMalloc(&head, sizeof(int) * V));
-      GV_CUDA(cudaMalloc(&pos, sizeof(int) * V));
-      GV_CUDA(cudaMalloc(&tmp, tb));
+      GV_TRY(take(&head, sizeof(int) * V));
+      GV_TRY(take(&pos, sizeof(int) * V));
+      GV_TRY(take(&tmp, tb));
       const unsigned gb = (unsigned)((V + 255) / 256);
       k_tile_heads<<<gb, 256, 0, st>>>(V, d_keys, head);
       GV_LAUNCH("k_tile_heads");
@@ -1028,8 +1029,8 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
       const size_t R = (size_t)last[0] + last[1];
       rkey.resize(R);
       rstart.resize(R);
-      GV_CUDA(cudaMalloc(&dk, sizeof(*dk) * R));
-      GV_CUDA(cudaMalloc(&ds, sizeof(*ds) * R));
+      GV_TRY(take(&dk, sizeof(*dk) * R));
+      GV_TRY(take(&ds, sizeof(*ds) * R));
       k_tile_runs<<<gb, 256, 0, st>>>(V, d_keys, head, pos, dk, ds);
       GV_LAUNCH("k_tile_runs");
       GV_CUDA(cudaMemcpyAsync(rkey.data(), dk, sizeof(*dk) * R, cudaMemcpyDeviceToHost, st));
@@ -1043,6 +1044,10 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     cudaFree(tmp);
     cudaFree(dk);
     cudaFree(ds);
+    if (!room) {
+      cudaGetLastError();
+      return GV_OK;
+    }
     if (s != GV_OK) return s;
   }
   const size_t R = rkey.size();
@@ -1085,9 +1090,10 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   // a second).
   n->warps = R <= (size_t)(16 * P.num_sms) && P.Vgrid >= 64 * (int64_t)R ? 8 : 1;
   const int T = 512;
-  std::vector<NuTask> tasks;
+  std::vector<NuTask>& tasks = n->h_tasks;
   const size_t tiles = (size_t)n->nty * n->ntx;
-  std::vector<int> slot((size_t)C * tiles, -1);
+  std::vector<int>& slot = n->h_slot;
+  slot.assign((size_t)C * tiles, -1);
   n->task_off.assign(C + 1, 0);
   for (size_t r = 0; r < R; r++) {
     const uint32_t t = (uint32_t)(rkey[r] & 0x3FFFFFFu);
@@ -1106,11 +1112,8 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   }
   for (int c = 0; c < C; c++) n->task_off[c + 1] += n->task_off[c];
   // ---- channel groups whose workspace stays bounded ------------------------------
-  const size_t slot_b = sizeof(float4) * kTilePts * pairs;
-  const size_t h_b = sizeof(float2) * (size_t)pairs * n->nrow * N;
-  const size_t fac_b = sizeof(float) * (size_t)N * N;
+  const size_t slot_b = slot_bytes(*n), h_b = plane_bytes(P);
   n->groups.push_back(0);
-  size_t max_slots = 0, max_ch = 0;
   for (int c = 0; c < C;) {
     size_t used = 0;
     const int c0 = c;
@@ -1121,9 +1124,23 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
       c++;
     }
     n->groups.push_back(c);
-    max_ch = std::max<size_t>(max_ch, c - c0);
-    max_slots = std::max<size_t>(max_slots, n->task_off[c] - n->task_off[c0]);
+    n->max_ch = std::max<size_t>(n->max_ch, c - c0);
+    n->max_slots = std::max<size_t>(n->max_slots, n->task_off[c] - n->task_off[c0]);
   }
+  return GV_OK;
+}
+
+// The plan's device buffers, and the pixels' w-term coefficients and factors:
+// once the beam tables (the pixels' offsets), the mask and the channels' tables
+// are in place.
+gv_status nu_build(Problem& P) {
+  if (!P.nu) return GV_OK;
+  NuPlan* n = P.nu;
+  const int C = (int)P.chans.size(), N = P.N, pairs = n->pairs;
+  const std::vector<NuTask>& tasks = n->h_tasks;
+  const std::vector<int>& slot = n->h_slot;
+  const size_t slot_b = slot_bytes(*n), h_b = plane_bytes(P);
+  const size_t fac_b = sizeof(float) * (size_t)N * N;
   const int lg = P.log2n + 1;
   std::vector<float2> tw;
   for (int l = fft16_first(lg); l < lg; l += 4)
@@ -1138,8 +1155,8 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     cudaError_t e = cudaMalloc(&n->d_tasks, sizeof(NuTask) * tasks.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_slot, sizeof(int) * slot.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_done, sizeof(uint32_t) * (tasks.size() + N));
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_slots, slot_b * max_slots);
-    if (e == cudaSuccess) e = cudaMalloc(&n->d_H, h_b * max_ch);
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_slots, slot_b * n->max_slots);
+    if (e == cudaSuccess) e = cudaMalloc(&n->d_H, h_b * n->max_ch);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_twiddle, sizeof(float2) * tw.size());
     if (e == cudaSuccess) e = cudaMalloc(&n->d_corr, sizeof(float) * N);
     if (e == cudaSuccess) e = cudaMalloc(&n->d_coef, sizeof(float2) * (size_t)pairs * N * N);
@@ -1149,13 +1166,14 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
     return e;
   };
   const cudaError_t e = upload();
-  if (e == cudaErrorMemoryAllocation) {
+  const size_t large = slot_b * n->max_slots + h_b * n->max_ch + fac_b * C;
+  if (e == cudaErrorMemoryAllocation || (e == cudaSuccess && !room_left(large))) {
     // no room for the grids: the direct sums need less
     cudaGetLastError();
     nu_free(P);
     return GV_OK;
   }
-  if (e != cudaSuccess) return cuda_fail(e, "nu_setup");
+  if (e != cudaSuccess) return cuda_fail(e, "nu_build");
   GV_CUDA(cudaMemcpy(n->d_tasks, tasks.data(), sizeof(NuTask) * tasks.size(),
                      cudaMemcpyHostToDevice));
   GV_CUDA(cudaMemcpy(n->d_slot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice));
@@ -1163,6 +1181,16 @@ gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw) {
   n->tasks = (int)tasks.size();
   GV_CUDA(cudaMemcpy(n->d_twiddle, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   GV_CUDA(cudaMemcpy(n->d_corr, corr.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
+  n->h_tasks = {};
+  n->h_slot = {};
+  const int64_t MN = (int64_t)N * N;
+  k_nu_coefficients<<<(unsigned)((MN + 255) / 256), 256, 0, P.stream>>>(
+      N, pairs, (float)(2.0 * kPiD * n->wmax), P.d_beam_x, P.d_beam_y, n->d_corr, n->d_coef);
+  GV_LAUNCH("k_nu_coefficients");
+  const FactorArgs fa{N, P.normalize, P.pb, P.D, P.pbf, P.pbcut, P.fg_scale, P.d_beam_x,
+                      P.d_beam_y, P.d_chfreq, P.d_chnvis, P.d_mask, P.d_gcf, n->d_fac};
+  k_nu_factors<<<dim3((unsigned)((MN + 255) / 256), (unsigned)C), 256, 0, P.stream>>>(fa);
+  GV_LAUNCH("k_nu_factors");
   return GV_OK;
 }
 

@@ -115,7 +115,7 @@ struct Problem {
   float2* d_grid = nullptr;      // [C][MN] model grids
   float2* d_twiddle = nullptr;   // [n] e^{+2 pi i m/n} (objective.cu smem_fft)
   float2* d_tw8 = nullptr;       // fft8_twiddles(log2n): twiddles pass by pass (fft8)
-  float* d_atten = nullptr;      // [C][MN] beam of every pixel and channel
+  float* d_atten = nullptr;      // [C][MN] beam of every pixel and channel, or null: no room
   uint8_t* d_need = nullptr;     // [N + N] columns, then rows, of the grids that are read
   int* d_col_blocks = nullptr;   // the column pass' blocks with a needed column
   int col_blocks = 0;
@@ -359,6 +359,7 @@ struct XtSource {
   int positivity;
 };
 gv_status objective_setup(Problem& P);
+gv_status beam_table(Problem& P);
 gv_status chi2_launch(Problem& P, float* d_img, int flag_opt, bool store_res,
                       const XtSource* xs = nullptr, double* term_out = nullptr,
                       uint32_t zero_terms = 0u);
@@ -434,8 +435,11 @@ gv_status dchi2_tc(Problem& P, const float* d_img, int flag_opt, float* d_result
 // non-uniform FFT (dchi2_nu.cu), where P.nu is set
 gv_status dchi2_nu(Problem& P, const float* d_img, int flag_opt, float* d_result,
                    int only_channel, int mode);
-gv_status nu_setup(Problem& P, const unsigned long long* d_keys, double maxw);
-gv_status nu_finish(Problem& P);
+gv_status nu_plan(Problem& P, const unsigned long long* d_keys, double maxw);
+gv_status nu_build(Problem& P);
+// Whether buffers of `bytes` that a problem can do without, just allocated,
+// leave the memory that its calls may still ask for (setup.cu).
+bool room_left(size_t bytes);
 void nu_free(Problem& P);
 int nu_pairs(const Problem& P);  // of its w series; 0: direct sums
 uint32_t nu_tiles_x(int N);  // tiles per row of the doubled grid's half plane

@@ -177,7 +177,9 @@ struct RowPass {
   static constexpr int kBlock = kThreads * kLines;
 };
 
-template <int LG>
+// kTable: the beams come from atten; otherwise, where the memory had no room for
+// it, they are formed here, by the same operations.
+template <int LG, bool kTable>
 __global__ void __launch_bounds__(RowPass<LG>::kBlock,
                                   RowPass<LG>::kBlock > 384 ? 1 : 768 / RowPass<LG>::kBlock)
     k_rows_fft(StageParams sp, const float* __restrict__ chfreq, int C, Images imgs,
@@ -229,10 +231,17 @@ __global__ void __launch_bounds__(RowPass<LG>::kBlock,
   const float floor_inu = -1.0f * sp.eta * sp.minpix;
   for (int c = 0; c < C; c++) {
     const float nudiv = chfreq[c] / sp.nu_0;
-    const float* at = atten + c * MN + q0;
     float2 v[8];
+    if constexpr (kTable) {
+      const float* at = atten + c * MN + q0;
 #pragma unroll
-    for (int e = 0; e < 8; e++) v[e].x = __ldg(at + e * T);
+      for (int e = 0; e < 8; e++) v[e].x = __ldg(at + e * T);
+    } else {
+      const BeamAt beam = beam_at(chfreq[c], sp.D, sp.pbf, sp.pbcut, sp.pb);
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        v[e].x = attenuation_at(beam_arc(__ldg(sp.beam_x + j + e * T), __ldg(sp.beam_y + i)), beam);
+    }
 #pragma unroll
     for (int e = 0; e < 8; e++) {
       // calculateInu, apply_beam2I, fg_scale, apply_GCF as in stage_value
@@ -999,7 +1008,8 @@ static gv_status pass_of_side(Problem& P, int pass, const StageParams& sp, const
   using R = RowPass<LG>;
   using K = ColPass<LG>;
   if (pass == 1) {
-    k_rows_fft<LG><<<dim3(P.N / R::kLines, count), R::kBlock, 0, P.stream>>>(
+    const auto rows = P.d_atten ? k_rows_fft<LG, true> : k_rows_fft<LG, false>;
+    rows<<<dim3(P.N / R::kLines, count), R::kBlock, 0, P.stream>>>(
         sp, P.d_chfreq, C, imgs, P.d_mask, P.d_atten, P.d_need, P.d_tw8, grid);
     GV_LAUNCH("k_rows_fft");
   } else if (P.col_blocks > 0) {  // else no visibility lies on the grid
@@ -1099,8 +1109,6 @@ static int prior_blocks(const Problem& P) {
   return (int)std::min<int64_t>((MN + 255) / 256, P.part_stride);
 }
 
-// Tables of the row and column passes: the channels' beams, the columns and
-// rows of the model grid that the visibilities read, the twiddles by pass.
 __global__ void __launch_bounds__(256) k_attenuation(int N, const float* __restrict__ chfreq,
                                                      const float* __restrict__ beam_x,
                                                      const float* __restrict__ beam_y, float D,
@@ -1127,13 +1135,30 @@ __global__ void __launch_bounds__(256) k_needed(int N, const ChanRange* __restri
   }
 }
 
-gv_status objective_setup(Problem& P) {
+// The channels' beams, where the memory has room for them: the row pass forms
+// them as it goes where it has not.
+gv_status beam_table(Problem& P) {
   const int N = P.N, C = (int)P.chans.size();
   const int64_t MN = (int64_t)N * N;
-  GV_CUDA(cudaMalloc(&P.d_atten, sizeof(float) * MN * C));
+  const size_t bytes = sizeof(float) * (size_t)MN * C;
+  const cudaError_t e = cudaMalloc(&P.d_atten, bytes);
+  if (e == cudaErrorMemoryAllocation || (e == cudaSuccess && !room_left(bytes))) {
+    cudaGetLastError();
+    cudaFree(P.d_atten);
+    P.d_atten = nullptr;
+    return GV_OK;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "beam_table");
   k_attenuation<<<dim3((unsigned)((MN + 255) / 256), C), 256, 0, P.stream>>>(
       N, P.d_chfreq, P.d_beam_x, P.d_beam_y, P.D, P.pbf, P.pbcut, P.pb, P.d_atten);
   GV_LAUNCH("k_attenuation");
+  return GV_OK;
+}
+
+// Tables of the row and column passes: the columns and rows of the model grid
+// that the visibilities read, the twiddles by pass.
+gv_status objective_setup(Problem& P) {
+  const int N = P.N, C = (int)P.chans.size();
   // bits of the needed columns, then rows, then the same as bytes
   const int words = 2 * N / 32;
   uint32_t* bits = nullptr;

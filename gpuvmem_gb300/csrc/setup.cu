@@ -254,6 +254,13 @@ __global__ void k_rho(int M, int N, float xobs, float yobs, double dx, double dy
 
 }  // namespace
 
+bool room_left(size_t bytes) {
+  // not asked about small buffers: the query takes longer than they do
+  constexpr size_t kSmall = size_t(256) << 20, kRoom = size_t(4) << 30;
+  size_t left = 0, total = 0;
+  return bytes < kSmall || (cudaMemGetInfo(&left, &total) == cudaSuccess && left >= kRoom);
+}
+
 void free_problem(Problem& P) {
   cudaFree(P.d_deg);
   cudaFree(P.d_vo);
@@ -410,6 +417,13 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
   cudaStream_t st = P.stream;
 
   // ---- visibilities: upload, prepare, sort by (channel, cell) -------------
+  // w in wavelengths, unsorted: of use to the direct engines alone, kept until
+  // it is known whether they run
+  struct Unsorted {
+    float* p = nullptr;
+    ~Unsorted() { cudaFree(p); }
+  } wl;
+  float*& wl_u = wl.p;
   {
     double* d_uvw = nullptr;
     float2* d_vo_in = nullptr;
@@ -421,7 +435,6 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     float4* deg_u = nullptr;
     float2* vo_u = nullptr;
     uint4* ph_u = nullptr;
-    float* wl_u = nullptr;
     uint32_t* d_maxw = nullptr;
     int64_t* d_kept = nullptr;
     unsigned long long *keys = nullptr, *keys2 = nullptr;
@@ -433,7 +446,7 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     auto cleanup = [&]() {
       cudaFree(d_uvw); cudaFree(d_vo_in); cudaFree(d_w_in); cudaFree(deg_u);
       cudaFree(d_mom); cudaFree(d_mdone); cudaFree(d_wsum); cudaFree(d_off);
-      cudaFree(vo_u); cudaFree(ph_u); cudaFree(wl_u); cudaFree(d_maxw); cudaFree(d_kept); cudaFree(keys); cudaFree(keys2);
+      cudaFree(vo_u); cudaFree(ph_u); cudaFree(d_maxw); cudaFree(d_kept); cudaFree(keys); cudaFree(keys2);
       cudaFree(idx); cudaFree(tmp);
     };
 #define GV_SETUP_CUDA(call)                         \
@@ -576,22 +589,11 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     }
     P.max_wrho = maxw * rmax;
     if (tile_sh >= 0) {
-      const gv_status s = nu_setup(P, keys2, maxw);
+      const gv_status s = nu_plan(P, keys2, maxw);
       if (s != GV_OK) {
         cleanup();
         return s;
       }
-    }
-    if (!P.nu) {
-      // the direct engines' own streams
-      GV_SETUP_CUDA(cudaMalloc(&P.d_wl, sizeof(float) * V));
-      k_gather<float><<<gb, 256, 0, st>>>(V, P.d_perm, wl_u, P.d_wl);
-      if (d.dchi2_engine != 1 && dchi2_tc_geometry(P)) {
-        GV_SETUP_CUDA(cudaMalloc(&P.d_E, sizeof(float4) * V));
-        k_phasors<<<gb, 256, 0, st>>>(V, P.d_ph, P.d_E);
-      }
-      GV_SETUP_CUDA(cudaGetLastError());
-      GV_SETUP_CUDA(cudaStreamSynchronize(st));
     }
     cleanup();
 #undef GV_SETUP_CUDA
@@ -697,7 +699,6 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     GV_CUDA(cudaMemcpy(P.d_kc_off, kc.data(), sizeof(int64_t) * (C + 1), cudaMemcpyHostToDevice));
     GV_CUDA(cudaMemcpy(P.d_kc_one, k1.data(), sizeof(int64_t) * 2 * C, cudaMemcpyHostToDevice));
   }
-  GV_TRY(nu_finish(P));
   GV_TRY(objective_setup(P));
   GV_CUDA(cudaMalloc(&P.d_scal, kScalBytes));
   P.d_flags = reinterpret_cast<uint32_t*>(P.d_scal + kNumScal);
@@ -707,6 +708,28 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     k_dirty_max<<<gb, 256, 0, st>>>(V, P.d_deg, P.d_vo, P.d_flags + kFlagDirtyMax,
                                     P.d_flags + kFlagPsfMax);
     GV_LAUNCH("k_dirty_max");
+  }
+  P.part_stride = 4 * P.num_sms;
+  const int nslots = C + kMaxTerms + 8;
+  GV_CUDA(cudaMalloc(&P.d_part, sizeof(double) * (size_t)P.part_stride * nslots));
+  GV_CUDA(cudaMallocHost(&P.h_scal, kScalBytes));
+  GV_CUDA(cudaMalloc(&P.d_tmp, sizeof(float) * 2 * MN));
+
+  // ---- DChi2: the non-uniform FFT, or the direct engines' own buffers -------
+  // After everything that a problem needs in any case, so that one which fits
+  // the memory with the direct sums is not refused for the FFT's sake.
+  GV_TRY(nu_build(P));
+  if (!P.nu) {
+    const unsigned gb = (unsigned)((V + 255) / 256);
+    GV_CUDA(cudaMalloc(&P.d_wl, sizeof(float) * V));
+    k_gather<float><<<gb, 256, 0, st>>>(V, P.d_perm, wl_u, P.d_wl);
+    GV_LAUNCH("k_gather");
+    GV_CUDA(cudaStreamSynchronize(st));
+    if (d.dchi2_engine != 1 && dchi2_tc_geometry(P)) {
+      GV_CUDA(cudaMalloc(&P.d_E, sizeof(float4) * V));
+      k_phasors<<<gb, 256, 0, st>>>(V, P.d_ph, P.d_E);
+      GV_LAUNCH("k_phasors");
+    }
   }
   // split-K partial images of the tensor-core engine: pick the split count
   // that fills whole waves of SMs (of CTA pairs in pair mode), keeping
@@ -742,11 +765,7 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
     P.use_graphs = (g && g[0] == '0') ? 0 : 1;
   }
   if (const char* e = std::getenv("GV_FUSED")) P.fused = std::atoi(e) != 0 ? 1 : 0;
-  P.part_stride = 4 * P.num_sms;
-  const int nslots = C + kMaxTerms + 8;
-  GV_CUDA(cudaMalloc(&P.d_part, sizeof(double) * (size_t)P.part_stride * nslots));
-  GV_CUDA(cudaMallocHost(&P.h_scal, kScalBytes));
-  GV_CUDA(cudaMalloc(&P.d_tmp, sizeof(float) * 2 * MN));
+  GV_TRY(beam_table(P));
   // DChi2's direct-sum engine: the tensor-core GEMM where it covers the
   // geometry, else the SIMT kernel.  With dchi2_engine 0 the non-uniform FFT
   // (P.nu) runs in its place wherever it covers the w-term: objective and

@@ -46,3 +46,65 @@ def test_call_after_a_refused_one():
             prob = _problem(small, engine if engine != 2 else 1)
             assert prob is not None
             prob.close()
+
+
+@pytest.mark.parametrize("n,nchan,n_ant,n_times,direct,most,step", [
+    (512, 8, 9, 31, 2, 260, 4),       # image-sized buffers: plan, grids, beam table
+    (64, 2, 60, 1200, 1, 768, 12),    # visibilities: the plan's scratch among set-up's copies
+])
+def test_created_wherever_the_direct_sums_are(n, nchan, n_ant, n_times, direct, most, step):
+    """From plenty of memory down to where the direct-sum engine is refused: the
+    default engine is created as long as the direct one is, as a non-uniform FFT
+    first and as direct sums then.  Those take the visibilities in another order
+    (by tile) than the engine by itself: 1e-5, as the engines agree elsewhere."""
+    import torch
+    data = synth.generate(synth.small_config(n=n, nchan=nchan, seed=3, n_ant=n_ant,
+                                             n_times=n_times))
+    ref, chi2, out = {}, {}, torch.zeros((2, n, n), device="cuda")
+    img = None
+    for engine in (direct, 0):
+        prob = _problem(data, engine)
+        if img is None:
+            img = prob.initial_image()
+            img[0] += (200.0 * torch.rand(img[0].shape, device="cuda") ** 6)
+            prob.chi2(img)  # clips it
+        chi2[engine] = prob.chi2(img)
+        ref[engine] = prob.dchi2(img).clone()
+        assert (prob.dchi2_pairs > 0) == (engine == 0)
+        prob.close()
+    assert chi2[0] == pytest.approx(chi2[direct], rel=1e-12)
+    seen = []
+    for mb in range(most, 0, -step):
+        with only(mb):
+            prob = _problem(data, direct)
+            if prob is None:
+                break
+            prob.close()
+            prob = _problem(data, 0)
+            assert prob is not None, f"{mb} MB: the direct engine was created"
+            pairs = prob.dchi2_pairs
+            f = prob.chi2(img)
+            out.zero_()
+            prob.dchi2(img, out=out)
+            prob.close()
+        seen.append(pairs)
+        assert f == pytest.approx(chi2[0], rel=1e-12)
+        if pairs:
+            assert torch.equal(out, ref[0]), mb
+        else:
+            assert (out - ref[direct]).abs().max() <= 1e-5 * ref[direct].abs().max(), mb
+    assert seen[0] > 0 and seen[-1] == 0, seen
+
+
+def test_large_plans_leave_room():
+    """A plan of 256 MB and more leaves 4 GB, which the optimisers' vectors and
+    the images of a call may need."""
+    data = synth.generate(synth.small_config(n=1024, nchan=8, seed=3, n_ant=9, n_times=31))
+    prob = _problem(data, 0)
+    assert prob.dchi2_pairs > 0
+    prob.close()
+    for mb, runs in ((6000, True), (4200, False)):
+        with only(mb):
+            prob = _problem(data, 0)
+            assert (prob.dchi2_pairs > 0) == runs
+            prob.close()
