@@ -142,6 +142,13 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
   }
 }
 
+// s += x with the rounding error in e (Knuth's two-sum)
+__device__ __forceinline__ void two_sum(float& s, float& e, float x) {
+  const float t = s + x, b = t - s;
+  e += (s - (t - b)) + (x - b);
+  s = t;
+}
+
 // One block per task, its visibilities shared out among the warps in order.
 // Each lane prepares one of 32 visibilities at a time (position, taps, the
 // pairs' values) in shared memory; then the warp takes them one by one.  Lane
@@ -151,7 +158,8 @@ __device__ __forceinline__ void taps(const SpreadArgs& a, float f, float (&w)[kT
 // by cell), so a step to the next cell writes back only the column that is
 // left.  The warps' 15 x 15 tiles are added in order and go out once, to the
 // task's own slot; where a tile has several tasks, the last of their blocks
-// to finish adds the slots up, in order, into the first.
+// to finish adds the slots up, in order and the sums of eight compensated (a
+// dense tile has thousands of them), into the first.
 //
 // Bound by issue slots, two thirds of them at the 19 warps an SM that the tiles
 // leave room for: 40 warp instructions a visibility.  8.8 M visibilities in 8
@@ -322,16 +330,25 @@ __global__ void __launch_bounds__(32 * kSpreadWarps) k_nu_spread(SpreadArgs a) {
   __threadfence();
   float4* sum = a.slots + (size_t)(task.first - a.t0) * kSlot;
   for (int k = threadIdx.x; k < (int)kSlot; k += 32 * kSpreadWarps) {
-    float4 t = __ldcg(sum + k);
-#pragma unroll 8
-    for (int w = 1; w < task.pieces; w++) {
-      const float4 u = __ldcg(sum + w * kSlot + k);
-      t.x += u.x;
-      t.y += u.y;
-      t.z += u.z;
-      t.w += u.w;
+    float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f), e = t;
+    const float4* from = sum + k;
+    for (int w = 0; w < task.pieces; w += 8, from += 8 * kSlot) {
+      float4 u = __ldcg(from);
+#pragma unroll
+      for (int i = 1; i < 8; i++) {
+        const float4 p = w + i < task.pieces ? __ldcg(from + i * kSlot)
+                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        u.x += p.x;
+        u.y += p.y;
+        u.z += p.z;
+        u.w += p.w;
+      }
+      two_sum(t.x, e.x, u.x);
+      two_sum(t.y, e.y, u.y);
+      two_sum(t.z, e.z, u.z);
+      two_sum(t.w, e.w, u.w);
     }
-    sum[k] = t;
+    sum[k] = make_float4(t.x + e.x, t.y + e.y, t.z + e.z, t.w + e.w);
   }
 }
 
