@@ -729,7 +729,9 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
     const int last = min(planes, first + end - unit);
     unit += last - first;
     const int col = cblk * CB + cc;
-    // the thread's pixels of the image's alpha plane, kept for all planes
+    // the thread's pixels of the image's alpha plane, kept for all planes; without
+    // an image the rounding errors of the planes' sum (a PSF's channels all have
+    // one sign)
     bool flat = true;
     if (a.img) {
 #pragma unroll
@@ -738,6 +740,9 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
         al[s * S::kBlock] = v;
         flat = flat && v == 0.0f;
       }
+    } else {
+#pragma unroll
+      for (int s = 0; s < 8; s++) al[s * S::kBlock] = 0.0f;
     }
     // small sides, whose blocks run once through a plane or two: everything the
     // end needs is on its way before the first transform
@@ -807,8 +812,18 @@ __global__ void __launch_bounds__(ColShape<LG>::kBlock, ColShape<LG>::kBlock == 
             f *= powf(nudiv, av);
           }
         }
-        acc[s] = fmaf(f, t, acc[s]);
+        if (a.img) {
+          acc[s] = fmaf(f, t, acc[s]);
+        } else {
+          float e = al[s * S::kBlock];
+          two_sum(acc[s], e, f * t);
+          al[s * S::kBlock] = e;
+        }
       }
+    }
+    if (!a.img) {
+#pragma unroll
+      for (int s = 0; s < 8; s++) acc[s] += al[s * S::kBlock];
     }
     if constexpr (G > 1) {
       // the groups' sums, in order

@@ -94,3 +94,9 @@ def test_sizes(n, nchan, n_ant, n_times, uvscale, wscale):
 def test_many_pieces_a_tile(n, uvscale):
     """2.1M visibilities in one channel, thousands of pieces in the densest tiles."""
     _check(n, 1, 60, 1200, uvscale, 1.0, pixels=600)
+
+
+def test_many_channels():
+    """2048 channels of 100 visibilities: the terms of a PSF have one sign, so
+    that rounding errors of a sum over channels add up."""
+    _check(32, 2048, 5, 10, 1.0, 1.0)
