@@ -3,6 +3,7 @@ gives way to what needs little, and the results stay."""
 
 import contextlib
 
+import numpy as np
 import pytest
 
 from gpuvmem_gb300 import synth
@@ -49,7 +50,7 @@ def test_call_after_a_refused_one():
 
 
 @pytest.mark.parametrize("n,nchan,n_ant,n_times,direct,most,step", [
-    (512, 8, 9, 31, 2, 260, 4),       # image-sized buffers: plan, grids, beam table
+    (512, 8, 9, 31, 2, 256, 8),       # image-sized buffers: plan, grids, beam table
     (64, 2, 60, 1200, 1, 768, 12),    # visibilities: the plan's scratch among set-up's copies
 ])
 def test_created_wherever_the_direct_sums_are(n, nchan, n_ant, n_times, direct, most, step):
@@ -108,3 +109,73 @@ def test_large_plans_leave_room():
             prob = _problem(data, 0)
             assert (prob.dchi2_pairs > 0) == runs
             prob.close()
+
+
+def _under(mb, call):
+    """call() with plenty of memory and with mb MB: the results of both, and the
+    kernels that each launched."""
+    import gpuvmem_gb300 as gv
+    call()  # loads the kernels
+    n0 = gv.launch_count()
+    plenty = call()
+    n1 = gv.launch_count()
+    with only(mb):
+        little = call()
+    return plenty, little, n1 - n0, gv.launch_count() - n1
+
+
+@pytest.mark.parametrize("scheme", ["uniform", "briggs"])
+def test_weighting_channel_by_channel(scheme):
+    """The sort of all channels (48 MB here) gives way to a sort for each."""
+    import gpuvmem_gb300 as gv
+    rng = np.random.default_rng(4)
+    C, n, M, cell = 24, 30000, 64, 0.05 / 3600.0
+    off = np.arange(C + 1, dtype=np.int64) * n
+    freqs = np.linspace(220e9, 240e9, C).astype(np.float32)
+    uvw = rng.normal(0, 150.0, (C * n, 3))  # some beyond the grid's edge
+    w = (rng.random(C * n) + 0.5).astype(np.float32)
+    w[::9] = 0.0
+    a, b, na, nb = _under(16, lambda: gv.apply_weighting(scheme, 0.5, M, M, -cell, cell, freqs,
+                                                         off, uvw, w))
+    assert nb > 2 * na
+    assert np.array_equal(a, b, equal_nan=True)
+
+
+def test_gridding_by_taps():
+    """The tiles of all channels (90 MB here) give way to a sort of each
+    channel's taps."""
+    import gpuvmem_gb300 as gv
+    rng = np.random.default_rng(5)
+    C, n, M, cell = 64, 3000, 128, 0.05 / 3600.0
+    off = np.arange(C + 1, dtype=np.int64) * n
+    freqs = np.linspace(220e9, 240e9, C).astype(np.float32)
+    uvw = rng.normal(0, 0.2 * 1.3e-3 / (cell * np.pi / 180.0), (C * n, 3))
+    vo = rng.normal(0, 1, (C * n, 2)).astype(np.float32)
+    w = rng.uniform(0.5, 2.0, C * n).astype(np.float32)
+    table = rng.uniform(-0.2, 1.0, (3, 3)).astype(np.float32)
+    a, b, na, nb = _under(24, lambda: gv.grid_visibilities(table, (1, 1), M, M, -cell, cell, freqs,
+                                                           off, uvw, vo, w))
+    assert nb > 2 * na
+    for x, y in zip(a, b):
+        assert x.tobytes() == y.tobytes()
+
+
+def test_candidates_one_after_another():
+    """The grids of all candidates at once (134 MB here) give way to one image
+    after another."""
+    import gpuvmem_gb300 as gv
+    import torch
+    data = synth.generate(synth.small_config(n=512, nchan=4, seed=3, n_ant=9, n_times=31))
+    prob = gv.Problem(data, [gv.term("Chi2", 1.0), gv.term("Entropy", 0.01, prior_value=0.001,
+                                                           eta=-1.0)])
+    prob.set_iteration(1)
+    imgs = prob.initial_image()[None].repeat(16, 1, 1, 1)
+    imgs[:, 0] += torch.rand((16, 512, 512), device="cuda") ** 6
+    with only(64):
+        little = prob.objective_many(imgs)
+        n0 = gv.launch_count()
+        assert prob.objective_many(imgs) == little
+        n1 = gv.launch_count()
+    plenty = prob.objective_many(imgs)
+    assert gv.launch_count() - n1 < (n1 - n0) / 4
+    assert plenty == little

@@ -96,3 +96,38 @@ def test_default_engine(n):
     import gpuvmem_gb300 as gv
     prob = gv.Problem(_data(n, nchan=2), [gv.term("Chi2", 1.0)])
     assert 1 <= prob.dchi2_pairs <= 4
+
+
+def _with_pairs(data, uvscale, pairs):
+    """The data with their uv scaled, and their w so that the series takes `pairs`."""
+    for wscale in 10.0 ** np.arange(-4.0, 4.0, 0.05):
+        d = dataclasses.replace(data, uvw_m=data.uvw_m * np.array([uvscale, uvscale, wscale]))
+        if _pairs_of_the_series(d) == pairs:
+            return d
+    raise AssertionError(f"no scale of w takes {pairs} pairs")
+
+
+def _against_simt(data, pairs):
+    """Tolerance as for the other comparisons with the SIMT sums."""
+    import gpuvmem_gb300 as gv
+    from test_gpu_nufft import TOL
+    prob = gv.Problem(data, [gv.term("Chi2", 1.0)])
+    assert prob.dchi2_pairs == pairs
+    prob.close()
+    got, ref = (_gradient(data, engine=e)[0] for e in (0, 1))
+    assert ref.abs().max() > 0
+    assert (got - ref).abs().max() <= TOL * ref.abs().max()
+
+
+@pytest.mark.parametrize("n,pairs,uvscale", [(1024, 1, 1.0), (1024, 4, 6.0), (2048, 2, 1.0),
+                                             (2048, 3, 6.0), (4096, 1, 1.0), (4096, 2, 0.3)])
+def test_large_sides(n, pairs, uvscale):
+    """The largest sides as a non-uniform FFT: the small arrays' own w needs more
+    pairs than there are from 2048^2 on."""
+    _against_simt(_with_pairs(_data(n, nchan=2), uvscale, pairs), pairs)
+
+
+def test_channel_groups():
+    """4096^2 with all rows of the grid and four pairs: 1.07 GB a channel, so that
+    five channels go in two groups of at most 4 GB."""
+    _against_simt(_with_pairs(_data(4096, nchan=5), 6.0, 4), 4)
