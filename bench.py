@@ -203,8 +203,7 @@ def dchi2_roofline(engine, n, channels, vis, t, peaks, src):
             "peak_source": f"{src} copy bandwidth", "algorithmic_bytes": nbytes,
             "note": "position and residual of every visibility (24 B) and three image planes, "
                     "once; issue slots, shared memory and the waits between the FFTs' phases "
-                    "bound the kernels",
-            "direct_sum_tflops": 4.0 * n * n * vis / t / 1e12}
+                    "bound the kernels"}
 
 
 def cpu_baseline(data, terms, sample_s, impl_kind="port"):
