@@ -502,18 +502,6 @@ struct GridBuffers {
 // and grid cells
 constexpr int64_t kMaxPairs = int64_t(1) << 28, kMaxCells = int64_t(1) << 28;
 
-struct Arena {
-  unsigned char* p = nullptr;
-  size_t used = 0;
-  template <class T>
-  T* take(int64_t n) {
-    T* r = p ? reinterpret_cast<T*>(p + used) : nullptr;
-    used += (sizeof(T) * (size_t)n + 255) & ~size_t(255);
-    return r;
-  }
-  ~Arena() { cudaFree(p); }
-};
-
 // Channels c0 .. c1 - 1 through the tiles; *done is false (nothing written)
 // where the scratch does not fit.
 gv_status grid_by_tiles(const gv_grid_kernel* kernel, GridGeom g, int C, const gv_channel_desc* in,

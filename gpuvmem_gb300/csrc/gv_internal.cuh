@@ -406,6 +406,20 @@ constexpr size_t kScalBytes = sizeof(double) * kNumScal + sizeof(uint32_t) * kNu
 // a device error word into a status.
 gv_status finish_graph(Problem& P);
 
+// A call's scratch in one allocation: the buffers are taken twice, without
+// memory for its size and then with it.
+struct Arena {
+  unsigned char* p = nullptr;
+  size_t used = 0;
+  template <class T>
+  T* take(int64_t n) {
+    T* r = p ? reinterpret_cast<T*>(p + used) : nullptr;
+    used += (sizeof(T) * (size_t)n + 255) & ~size_t(255);
+    return r;
+  }
+  ~Arena() { cudaFree(p); }
+};
+
 // Device-wide sort / scan / run-length primitives (sortscan.cu).  Scratch
 // sizes first, then the call; nothing is allocated inside.
 template <class K, class V>

@@ -29,6 +29,7 @@ namespace gv {
 namespace {
 
 constexpr uint32_t kNoCell = 0xFFFFFFFFu;
+// half a side at most: grids end at 4096, as images do
 constexpr int kMaxHalf = 2048;
 // bounds of the one-sort path: visibilities, and floats of the table of sums
 constexpr int64_t kOneSort = int64_t(1) << 28, kTable = int64_t(1) << 30;
@@ -264,18 +265,6 @@ cudaError_t copy_channels(int C, const int64_t* off, int width, cudaStream_t st,
   }
   return cudaSuccess;
 }
-
-struct Arena {
-  unsigned char* p = nullptr;
-  size_t used = 0;
-  template <class T>
-  T* take(int64_t n) {
-    T* r = p ? reinterpret_cast<T*>(p + used) : nullptr;
-    used += (sizeof(T) * (size_t)n + 255) & ~size_t(255);
-    return r;
-  }
-  ~Arena() { cudaFree(p); }
-};
 
 // Uniform and Briggs weights of all channels from one sort; *done is false
 // (and nothing written) where the data are beyond its bounds or do not fit.
