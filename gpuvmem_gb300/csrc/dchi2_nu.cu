@@ -495,30 +495,50 @@ __global__ void __launch_bounds__(RowShape<LG>::kBlock, 1024 / RowShape<LG>::kBl
     for (int e = 0; e < 16; e++) v[e] = buf[j + e * T];
     __syncthreads();
   } else {
-    // footprints that reach over the grid's edge come back at the other side
-#pragma unroll
-    for (int e = 0; e < 16; e++) v[e] = make_float2(0.0f, 0.0f);
-    if (in) {
-      for (int wy = -1; wy <= 1; wy++) {
-        const RowTiles up = row_tiles(a, ch, r + wy * n), down = row_tiles(a, ch, -r - wy * n);
-        for (int wx = -1; wx <= 1; wx++) {
-#pragma unroll
-          for (int e = 0; e < 16; e++) {
-            const int c = (e < 8 ? j + e * T : j + e * T - n) + wx * n;
-            if (c >= -3) {
-              const float4 g = cell_at(a, up, q, c);
-              v[e].x = fmaf(0.5f, g.x, v[e].x);
-              v[e].y = fmaf(0.5f, g.y, v[e].y);
-            }
-            if (c <= 3) {
-              const float4 g = cell_at(a, down, q, -c);
-              v[e].x = fmaf(0.5f, g.z, v[e].x);
-              v[e].y = fmaf(-0.5f, g.w, v[e].y);
-            }
-          }
-        }
+    // Footprints that reach over the grid's edge come back at the other side:
+    // rows r and r +- 2N are one line, and so are columns.  First every h+ at its
+    // column and the h- that meet no h+ at theirs, then the others (-3 .. 3, and
+    // those about the edge); a thread has the same columns, so the same
+    // positions, of all rows.
+    float2* line0 = smem_f2 + (l & ~1) * S::kStride;
+    float2* line1 = line0 + S::kStride;
+    const int t = threadIdx.x % (2 * T);
+    for (int p = t; p < n; p += 2 * T) line0[p] = line1[p] = make_float2(0.0f, 0.0f);
+    __syncthreads();
+    auto add = [&](float2* to, int c, float x, float y) {
+      const float2 g = to[c & (n - 1)];
+      to[c & (n - 1)] = make_float2(fmaf(0.5f, x, g.x), fmaf(0.5f, y, g.y));
+    };
+    auto lines = [&](auto&& take) {
+#pragma unroll 1
+      for (int s = 0; in && s < 6; s++) {
+        const int side = s & 1, row = (side ? (k ? -k : -N) : k) + (s / 2 - 1) * n;
+        const RowTiles tiles = row_tiles(a, ch, row);
+        if (tiles.at[0] < 0 && tiles.at[1] < 0) continue;
+        // rows 0 and -N are their own mirror images
+        take(tiles, side ? line1 : line0, (side != 0) == (k == 0) ? line1 : line0);
       }
-    }
+    };
+    const int edge = n - a.cmax;  // h- of column c >= edge meets an h+
+    lines([&](const RowTiles& tiles, float2* to, float2* mirror) {
+      for (int c = t - 3; c <= a.cmax; c += 2 * T) {
+        const float4 g = cell_at(a, tiles, q, c);
+        add(to, c, g.x, g.y);
+        if (c > 3 && c < edge) add(mirror, -c, g.z, -g.w);
+      }
+    });
+    __syncthreads();
+    lines([&](const RowTiles& tiles, float2*, float2* mirror) {
+      for (int i = t; i < 7 + max(0, a.cmax + 1 - edge); i += 2 * T) {
+        const int c = i < 7 ? i - 3 : edge + i - 7;
+        const float4 g = cell_at(a, tiles, q, c);
+        add(mirror, -c, g.z, -g.w);
+      }
+    });
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 16; e++) v[e] = buf[j + e * T];
+    __syncthreads();
   }
   fft16<LG>(v, buf, j, a.tw);
   if (!mine) return;
