@@ -245,20 +245,31 @@ struct Buffers {
 };
 
 // Copies of the channels' arrays that lie one after another on the host as one
-// array go as one copy (a user's channels are slices of one).
+// array go as one copy (a user's channels are slices of one); one by one where
+// they only happen to be neighbours, each pinned by itself, which a copy may not
+// span.
 template <class T, class F>
 cudaError_t copy_channels(int C, const int64_t* off, int width, cudaStream_t st, T* dev, F&& host,
                           cudaMemcpyKind kind) {
+  auto copy = [&](int c, int e) {  // channels c .. e - 1
+    auto* h = host(c);
+    T* d = dev + off[c] * width;
+    const size_t bytes = sizeof(T) * (size_t)(off[e] - off[c]) * width;
+    return kind == cudaMemcpyHostToDevice ? cudaMemcpyAsync(d, (const void*)h, bytes, kind, st)
+                                          : cudaMemcpyAsync((void*)h, d, bytes, kind, st);
+  };
   for (int c = 0; c < C;) {
     int e = c + 1;
     if (off[e] > off[c]) {
       auto* h = host(c);
       while (e < C && (off[e + 1] == off[e] || host(e) == h + (off[e] - off[c]) * width)) e++;
-      T* d = dev + off[c] * width;
-      const size_t bytes = sizeof(T) * (size_t)(off[e] - off[c]) * width;
-      const cudaError_t err = kind == cudaMemcpyHostToDevice
-                                  ? cudaMemcpyAsync(d, (const void*)h, bytes, kind, st)
-                                  : cudaMemcpyAsync((void*)h, d, bytes, kind, st);
+      cudaError_t err = copy(c, e);
+      if (err == cudaErrorInvalidValue && e > c + 1) {
+        cudaGetLastError();
+        err = cudaSuccess;
+        for (int k = c; k < e && err == cudaSuccess; k++)
+          if (off[k + 1] > off[k]) err = copy(k, k + 1);
+      }
       if (err != cudaSuccess) return err;
     }
     c = e;
