@@ -25,10 +25,15 @@
 // 2 (A/2)^(2 kPairs) / (2 kPairs)!, A = max |a|; problems whose A needs more
 // than 4 pairs keep the direct sums.
 //
-// All arithmetic is FP32 on exact 32-bit fixed-point grid positions; every
-// sum is taken in a fixed order (no atomics), so results repeat bit for bit.
-// Against 64-bit sums the gradient is 1.1 to 1.7e-7 off in the 2-norm (256^2
-// and 1024^2), where the tensor-core sum is 1.2 to 1.4e-6 off.
+// All arithmetic is FP32 on exact 32-bit fixed-point grid positions, the sums
+// over a tile's pieces and over the channels of a dirty image or PSF with their
+// rounding errors kept; every sum is taken in a fixed order (no atomics), so
+// results repeat bit for bit.  Against 64-bit sums gradients are 0.8 to 1.7e-7 off
+// in the 2-norm (64^2 to 1024^2), where the tensor-core sum is 1.2 to 1.4e-6 off
+// and the SIMT sum 0.8 to 2.7e-7; dirty images and PSFs 0.3 to 1.6e-7.  The
+// kernel's truncation and the FFTs' rounding make that up, so it does not fall
+// with the number of visibilities as the SIMT sum's error does where their terms
+// add up (2.5e-8 for 2.1M visibilities of one 64^2 channel).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -48,7 +53,7 @@ struct NuTask {
 
 struct NuPlan {
   int pairs = 0;           // complex FFTs per channel
-  int warps = 4;           // of a block of k_nu_spread
+  int warps = 1;           // of a block of k_nu_spread, or 8
   float wmax = 0.0f;
   int cmax = 0;            // covered columns: -cmax .. cmax
   int rmin = 0, nrow = 0;  // covered rows (signed)
@@ -1133,8 +1138,7 @@ gv_status nu_plan(Problem& P, const unsigned long long* d_keys, double maxw) {
   // ---- tasks ------------------------------------------------------------------
   // A tile's visibilities in pieces of T, a block each.  Few and well filled
   // tiles: the blocks run nearly at once and their longest chain decides, so
-  // 8 warps share a piece of 512 (256^2, 104,400 visibilities in 290 tiles:
-  // the whole evaluation 89 us, against 110 with 4 warps and pieces of 128).
+  // 8 warps share a piece of 512 (256^2, 104,400 visibilities in 290 tiles).
   // Otherwise one warp a piece, so that none idles in a thin tile, and the dense
   // tiles' pieces do not outlast the rest (2048^2, 8.9 M visibilities in 8
   // channels, an evaluation: 1754 us with pieces of 1024, 1728 of 512, 1735 of

@@ -75,7 +75,8 @@ struct Term {
   float* d_prior = nullptr;  // [MN] GEntropy / GL1Norm prior image (owned by the Problem)
 };
 
-// Packed per-visibility streams, sorted by grid cell within each channel.
+// Packed per-visibility streams, within each channel sorted by cell of the model
+// grid, or with dchi2_engine 0 by 8 x 8 tile of the doubled grid and cell in it.
 //   deg  : {cell (j1 << 16 | i1) as bits, du, dv, w}       16 B
 //   vo   : observed visibility                              8 B
 //   cvr  : w * (Vo - Vm), written by the chi2 pass          8 B

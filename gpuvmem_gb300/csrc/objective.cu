@@ -161,8 +161,8 @@ __device__ __noinline__ float spectral_power(float nudiv, float al) { return pow
 // arithmetic per pixel and channel as row_task; the beam comes from a table of
 // the same values (134 MB read at 2048^2 x 8 channels, where its exponentials
 // were a quarter of the pass).  n / 8 threads a row, kLines rows a block.
-// 2048^2 x 8 channels: 348 -> 129 us, bound by instruction issue and the
-// table's bytes.
+// 2048^2 x 8 channels: 348 -> 109 us, bound by the LSU's wavefronts (two thirds
+// of their peak) and instruction issue (56 %).
 // Images evaluated in one launch (blockIdx.y of the row pass): one, or the
 // candidates of gv_objective_many.
 constexpr int kMaxImages = 16;

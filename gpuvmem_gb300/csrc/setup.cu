@@ -8,7 +8,8 @@
 //    choice (src/functions.cu:2557-2609) are evaluated once per visibility
 //    (u,v,w are constant), so weights of visibilities outside the grid are
 //    zeroed here instead of on the first objective evaluation; visibilities
-//    are then sorted by grid cell so the degridding gathers hit L2 in order.
+//    are then sorted by grid cell, or by tile and cell (the non-uniform FFT's
+//    order), so the degridding gathers hit L2 in order.
 //  * total_attenuation / weight_image / noise_image, fg_scale = min(noise),
 //    noise_cut = factor * min(noise) (src/mfs.cu:849-916).
 
@@ -769,10 +770,17 @@ gv_status setup_problem(Problem& P, const gv_problem_desc& d) {
   // DChi2's direct-sum engine: the tensor-core GEMM where it covers the
   // geometry, else the SIMT kernel.  With dchi2_engine 0 the non-uniform FFT
   // (P.nu) runs in its place wherever it covers the w-term: objective and
-  // gradient at 64^2 with 1,120 visibilities 75 against 126 us, at 256^2 with
-  // 104,400 128 against 150 us, at 2048^2 x 8 channels with 8.8M 5.0 against
-  // 313 ms, and nearer the 64-bit sum (1.1 to 1.7e-7 of the 2-norm against
-  // 2e-7 for the SIMT sum, 1.2 to 1.4e-6 for the GEMM).
+  // gradient at 64^2 with 1,120 visibilities 39 against 126 us, at 256^2 with
+  // 104,400 64 against 150 us, at 2048^2 x 8 channels with 8.8M 1.71 against
+  // 313 ms.  Large images of few visibilities are the exception (its cost is the
+  // image's, theirs the product's): 1024^2 with fewer than some 2,000 a channel,
+  // 2048^2 with 6,000, 4096^2 with 10,000 to 25,000 take up to four times as long
+  // as with the GEMM (2048^2, 1,116 visibilities, the grid covered to a third:
+  // 372 against 190 us), which engine 2 still gives.  The line is not drawn there
+  // because the GEMM's error is ten times the FFT's: 1.2 to 1.4e-6 of the
+  // gradient's 2-norm against 0.8 to 1.7e-7, the SIMT sum 0.8 to 2.7e-7.  Where a
+  // dirty image's or a PSF's terms add up, the SIMT sum is nearer than the FFT
+  // (64^2, 2.1M visibilities: 2.7e-8 against 1.0e-7).
   P.engine = d.dchi2_engine;
   if (P.engine == 0) P.engine = dchi2_tc_geometry(P) ? 2 : 1;
   if (P.engine == 2 && !P.nu && !dchi2_tc_supported(P)) {
