@@ -428,8 +428,9 @@ __device__ __forceinline__ float4 cell_at(const RowArgs& a, const RowTiles& t, i
 //
 // Bound by the waits between its phases (looking cells up, three exchanges)
 // at two blocks an SM, about half of the issue slots: 16 planes of 2048^2 with
-// 1223 covered rows, 380 us where its traffic takes 100; a row by itself, each
-// cell looked up twice, 460.
+// 1223 covered rows, 372 us where its traffic takes 100 (381 with the registers
+// that the rows beyond the grid's edge spilled); a row by itself, each cell
+// looked up twice, 460.
 template <int LG>
 struct RowShape {
   static constexpr int kThreads = (1 << LG) / 16;  // per line
