@@ -1472,12 +1472,13 @@ gv_status batch_objective_launch(int np, const void* d_args, const int* d_off, i
 }
 
 // Images per launch of gv_objective_many: 16, fewer where their grids would
-// take more than 1 GB, 1 (one after another) where one image fills the GPU or
-// the terms are not Chi2 and priors of its clipped image.
+// take more than 1 GB or their channels pass a grid's second dimension (the
+// column pass), 1 (one after another) where one image fills the GPU or the terms
+// are not Chi2 and priors of its clipped image.
 int many_at_once(const Problem& P) {
   if (P.terms.empty() || P.terms[0].kind != GV_FI_CHI2 || fused_ok(P)) return 1;
-  const int64_t grid = (int64_t)P.M * P.N * (int64_t)P.chans.size();
-  return (int)std::min<int64_t>(kMaxImages, (int64_t(1) << 27) / grid);
+  const int64_t C = (int64_t)P.chans.size(), grid = (int64_t)P.M * P.N * C;
+  return (int)std::min({(int64_t)kMaxImages, (int64_t(1) << 27) / grid, 65535 / C});
 }
 
 // Room for count images a launch; *ok is false where the memory does not have
