@@ -74,15 +74,19 @@ def test_created_wherever_the_direct_sums_are(n, nchan, n_ant, n_times, direct, 
         assert (prob.dchi2_pairs > 0) == (engine == 0)
         prob.close()
     assert chi2[0] == pytest.approx(chi2[direct], rel=1e-12)
-    seen = []
+    seen, refused = [], None
     for mb in range(most, 0, -step):
         with only(mb):
             prob = _problem(data, direct)
             if prob is None:
                 break
             prob.close()
+            # one step of slack: a kernel's first launch takes memory of its own
+            assert refused is None, f"refused at {refused} MB, the direct engine not at {mb}"
             prob = _problem(data, 0)
-            assert prob is not None, f"{mb} MB: the direct engine was created"
+            if prob is None:
+                refused = mb
+                continue
             pairs = prob.dchi2_pairs
             f = prob.chi2(img)
             out.zero_()
