@@ -122,9 +122,11 @@ typedef struct gv_problem_desc {
   const gv_channel_desc* channels;
   int32_t nterms;
   const gv_fi_desc* terms;
-  /* 0 auto: DChi2 as a non-uniform FFT where it covers the w-term (nearer
-   * the 64-bit sum than the direct sums, and much faster), else the direct
-   * sum; 1 direct SIMT sum, 2 direct sum as a tensor-core GEMM */
+  /* 0 auto: DChi2 as a non-uniform FFT where it covers the w-term and the
+   * memory has room for it (about 1e-7 off the 64-bit sum), else the direct
+   * sum; 1 direct SIMT sum (nearer where many visibilities add up), 2 direct
+   * sum as a tensor-core GEMM (1.4e-6 off; faster for few visibilities on
+   * images of 1024^2 and more) */
   int32_t dchi2_engine;
   /* gridding correction function (host, M*N floats) of gridded data, or
    * NULL: with it chi2() multiplies the beam-weighted image by it before the
